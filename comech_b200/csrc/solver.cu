@@ -2318,7 +2318,8 @@ int build_dense(FebHandle* h) {
   // feb_create returns without waiting for them (FebHandle::settle joins them)
   FEB_TRY(H.pool.upload(&H.cmap, cmap.data(), cmap.size()));
   FEB_TRY(H.pool.upload(&H.klist, klist.data(), klist.size()));
-  FEB_TRY(H.pool.zeros(&H.Minv, (size_t)H.nd * H.nd));
+  const int ld = dense_ld(H.nd);
+  FEB_TRY(H.pool.zeros(&H.Minv, (size_t)ld * ld));
   int *dr = nullptr, *dc = nullptr;
   double* dv = nullptr;
   if (H.coarsest > 0 && V.sparse.size()) {
@@ -2341,17 +2342,17 @@ int build_dense(FebHandle* h) {
   cudaStream_t ds = H.dense_s;
   if (H.coarsest == 0) {
     switch (H.mode) {
-      case MAT_ISO_SRI: launch_dense_from_fine<MAT_ISO_SRI>(H.F64, H.cmap, H.Minv, H.nd, ds); break;
-      case MAT_ISO_FULL: launch_dense_from_fine<MAT_ISO_FULL>(H.F64, H.cmap, H.Minv, H.nd, ds); break;
-      default: launch_dense_from_fine<MAT_ORTHO>(H.F64, H.cmap, H.Minv, H.nd, ds); break;
+      case MAT_ISO_SRI: launch_dense_from_fine<MAT_ISO_SRI>(H.F64, H.cmap, H.Minv, ld, ds); break;
+      case MAT_ISO_FULL: launch_dense_from_fine<MAT_ISO_FULL>(H.F64, H.cmap, H.Minv, ld, ds); break;
+      default: launch_dense_from_fine<MAT_ORTHO>(H.F64, H.cmap, H.Minv, ld, ds); break;
     }
   } else {
-    launch_dense_from_stencil(V.A64, V.nx, V.ny, V.nz, H.cmap, H.Minv, H.nd, ds);
-    if (dr) launch_dense_add_entries((int)V.sparse.size(), dr, dc, dv, H.cmap, H.Minv, H.nd, ds);
-    launch_dense_add_terms(V.nterms, V.t_ptr, V.t_dof, V.t_val64, V.t_lam64, H.cmap, H.Minv, H.nd, ds);
+    launch_dense_from_stencil(V.A64, V.nx, V.ny, V.nz, H.cmap, H.Minv, ld, ds);
+    if (dr) launch_dense_add_entries((int)V.sparse.size(), dr, dc, dv, H.cmap, H.Minv, ld, ds);
+    launch_dense_add_terms(V.nterms, V.t_ptr, V.t_dof, V.t_val64, V.t_lam64, H.cmap, H.Minv, ld, ds);
   }
   FEB_CUDA(cudaMemsetAsync(H.dense_st, 0, sizeof(int), ds));
-  launch_dense_invert(H.Minv, H.nd, scratch, H.dense_st, ds);
+  FEB_TRY(launch_dense_invert(H.Minv, H.nd, scratch, H.dense_st, ds));
   FEB_CUDA(cudaGetLastError());
   FEB_CUDA(cudaMemcpyAsync(H.dense_st_h, H.dense_st, sizeof(int), cudaMemcpyDeviceToHost, ds));
   FEB_CUDA(cudaEventRecord(H.dense_ev, ds));
