@@ -4,6 +4,8 @@
 // rb/gpusolve.py:138-161); an explicit inverse turns the per-V-cycle solve into one coalesced GEMV.
 #include "dense.cuh"
 
+#include <cfloat>
+
 namespace feb {
 
 namespace {
@@ -75,46 +77,68 @@ __global__ void __launch_bounds__(256) k_mirror(double* __restrict__ M, int ld) 
 
 // Symmetric sweep of a 64 x 64 block held 4 x 4 per thread (rows 4 ty + u, columns 4 tx + v): step p turns
 // a_pp = d into -1/d, a_ip and a_pi into a_ip / d and a_ij into a_ij - a_ip a_pj / d; after all steps the block is
-// minus its inverse.  Row p travels through a double-buffered line of shared memory (its column is the same
-// numbers by symmetry), so a step costs one barrier.  A non-positive pivot sets *status and counts as 1.
-__device__ __forceinline__ void sweep_block(double (&a)[4][4], double (*line)[SB], int ty, int tx, int* status) {
+// minus its inverse.  Row p travels through a double-buffered line of shared memory (its column is the same numbers by
+// symmetry), so a step costs one barrier; the line also carries the next diagonal value before the step, so that
+// every thread forms the next pivot and its reciprocal while the step's update runs.  A non-positive pivot sets
+// *status and counts as 1.
+__device__ __forceinline__ double pivot_inverse(double d, bool& bad) {
+  const bool ok = d > 0.0 && d <= DBL_MAX;
+  bad |= !ok;
+  return 1.0 / (ok ? d : 1.0);
+}
+
+__device__ __forceinline__ void sweep_block(double (&a)[4][4], double (*line)[SB + 2], int ty, int tx, int* status) {
+  double ip = 0.0;
+  bool bad = false;
+#pragma unroll 1
   for (int pb = 0; pb < SB / 4; ++pb) {
 #pragma unroll
     for (int pu = 0; pu < 4; ++pu) {
       const int p = 4 * pb + pu;
-      double* row = line[p & 1];
+      double* row = line[pu & 1];
       if (ty == pb) {
-#pragma unroll
-        for (int v = 0; v < 4; ++v) row[4 * tx + v] = a[pu][v];
+        *reinterpret_cast<double2*>(row + 4 * tx) = make_double2(a[pu][0], a[pu][1]);
+        *reinterpret_cast<double2*>(row + 4 * tx + 2) = make_double2(a[pu][2], a[pu][3]);
       }
+      const int nb = pu < 3 ? pb : pb + 1;
+      if (ty == nb && tx == nb) row[SB] = a[(pu + 1) & 3][(pu + 1) & 3];
       __syncthreads();
-      double d = row[p];
-      if (!(d > 0.0) || !isfinite(d)) {
-        if (threadIdx.x == 0) atomicExch(status, FEB_ERR_COARSE);
-        d = 1.0;
-      }
-      const double ip = 1.0 / d;
+      if (p == 0) ip = pivot_inverse(row[0], bad);
       double ci[4], cj[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) { ci[u] = row[4 * ty + u] * ip; cj[u] = row[4 * tx + u]; }
+      for (int u = 0; u < 4; u += 2) {
+        const double2 x = *reinterpret_cast<const double2*>(row + 4 * ty + u);
+        const double2 y = *reinterpret_cast<const double2*>(row + 4 * tx + u);
+        ci[u] = x.x * ip; ci[u + 1] = x.y * ip; cj[u] = y.x; cj[u + 1] = y.y;
+      }
+      double next = 1.0;
+      if (p + 1 < SB) {
+        const double c = row[p + 1];
+        next = pivot_inverse(row[SB] - c * ip * c, bad);
+      }
 #pragma unroll
       for (int u = 0; u < 4; ++u)
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          const bool pr = ty == pb && u == pu, pc = tx == pb && v == pu;
-          if (pr && pc) a[u][v] = -ip;
-          else if (pr) a[u][v] = cj[v] * ip;
-          else if (pc) a[u][v] = ci[u];
-          else a[u][v] -= ci[u] * cj[v];
-        }
+        for (int v = 0; v < 4; ++v) a[u][v] -= ci[u] * cj[v];
+      if (ty == pb) {
+#pragma unroll
+        for (int v = 0; v < 4; ++v) a[pu][v] = cj[v] * ip;
+      }
+      if (tx == pb) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) a[u][pu] = ci[u];
+        if (ty == pb) a[pu][pu] = -ip;
+      }
+      ip = next;
     }
   }
+  if (bad && threadIdx.x == 0) atomicExch(status, FEB_ERR_COARSE);
 }
 
 // Dinv = inverse of the first pivot block.
 __global__ void __launch_bounds__(256)
 k_sweep_first(const double* __restrict__ M, int ld, double* __restrict__ Dinv, int* __restrict__ status) {
-  __shared__ double line[2][SB];
+  __shared__ __align__(16) double line[2][SB + 2];
   const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
   double a[4][4];
 #pragma unroll
@@ -128,65 +152,93 @@ k_sweep_first(const double* __restrict__ M, int ld, double* __restrict__ Dinv, i
     for (int v = 0; v < 4; ++v) Dinv[(4 * ty + u) * SB + 4 * tx + v] = -a[u][v];
 }
 
-// Pivot panel of step k: C_i = S_ik (from the lower triangle: S_ki^T for i < k), W_i = C_i Dinv; S_ik <- W_i,
-// S_kk <- -Dinv.  C and W are left transposed (k-major rows of length ld), as the update's operands.  A CTA takes
-// 16 rows of block row i: at 64 rows a CTA the panel would use a third of the SMs.
-__global__ void __launch_bounds__(256)
-k_sweep_panel(double* __restrict__ M, int ld, int k, const double* __restrict__ Dinv, double* __restrict__ CT,
-              double* __restrict__ WT) {
-  __shared__ __align__(16) double Ds[SB][SB];
-  __shared__ double Cs[16][SLD];
-  const int i = blockIdx.x, r0 = 16 * blockIdx.y, t = threadIdx.x;
-  const int row = i * SB + r0, kc = k * SB;
-  if (i == k) {
-    for (int e = t; e < 16 * SB; e += 256) M[(size_t)(row + e / SB) * ld + kc + e % SB] = -Dinv[(r0 + e / SB) * SB + e % SB];
-    return;
-  }
-  for (int e = t; e < SB * SB; e += 256) Ds[e / SB][e % SB] = Dinv[e];
-  for (int e = t; e < 16 * SB; e += 256) {
-    if (i > k) Cs[e / SB][e % SB] = M[(size_t)(row + e / SB) * ld + kc + e % SB];
-    else Cs[e % 16][e / 16] = M[(size_t)(kc + e / 16) * ld + row + e % 16];
-  }
-  __syncthreads();
-  for (int e = t; e < 16 * SB; e += 256) CT[(size_t)(e / 16) * ld + row + e % 16] = Cs[e % 16][e / 16];
-  const int r = t >> 4, c = (t & 15) * 4;
-  double w[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 8
-  for (int q = 0; q < SB; ++q) {
-    const double a = Cs[r][q];
-#pragma unroll
-    for (int v = 0; v < 4; ++v) w[v] += a * Ds[q][c + v];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int v = 0; v < 4; ++v) Cs[r][c + v] = w[v];
-  __syncthreads();
-  for (int e = t; e < 16 * SB; e += 256) {
-    const double x = Cs[e % 16][e / 16];
-    WT[(size_t)(e / 16) * ld + row + e % 16] = x;
-    if (i < k) M[(size_t)(kc + e / 16) * ld + row + e % 16] = x;
-    else M[(size_t)(row + e / SB) * ld + kc + e % SB] = Cs[e / SB][e % SB];
-  }
-}
-
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
                : "memory");
 }
 
-// Step k's update of the lower tiles outside the pivot panel: S_ij -= C_i W_j^T (64 x 64 x 64 a CTA, 4 x 4 a
-// thread).  The CTA of the next pivot block (block 0, so that it starts first) inverts it on the spot: the serial
-// part of the sweep runs beside the other tiles instead of between two steps.
-//
-// With 32-wide pivot blocks over the whole matrix and the pivot, row, column and finish passes as kernels of their
-// own, the inverse of 3510 dofs took 13.9 ms (77.7 us an update, 2.5 TB/s of matrix traffic, 40 us of serial kernels
-// a step) and that of 2457 dofs 6.3 ms; this form's times stand at launch_dense_invert.
+// Pivot panel of step k: C_i = S_ik (from the lower triangle: S_ki^T for i < k), W_i = C_i Dinv; S_ik <- W_i,
+// S_kk <- -Dinv.  -C and W are left transposed (k-major rows of length ld), as the update's operands.  A CTA takes
+// 16 rows of block row i: at 64 rows a CTA the panel would use a third of the SMs.
+__global__ void __launch_bounds__(256)
+k_sweep_panel(double* __restrict__ M, int ld, int k, const double* __restrict__ Dinv, double* __restrict__ CT,
+              double* __restrict__ WT) {
+  __shared__ __align__(16) double Ds[SB][SB];
+  __shared__ __align__(16) double Cs[SB][16];     // C_i^T
+  const int i = blockIdx.x, r0 = 16 * blockIdx.y, t = threadIdx.x;
+  const int row = i * SB + r0, kc = k * SB;
+  if (i == k) {
+#pragma unroll
+    for (int e = t; e < 16 * SB; e += 256) M[(size_t)(row + e / SB) * ld + kc + e % SB] = -Dinv[(r0 + e / SB) * SB + e % SB];
+    return;
+  }
+#pragma unroll
+  for (int e = t; e < SB * SB / 2; e += 256) cp_async16(&Ds[0][0] + 2 * e, Dinv + 2 * e);
+  if (i > k) {
+    double2 v[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int e = t + 256 * h;
+      v[h] = *reinterpret_cast<const double2*>(M + (size_t)(row + e / 32) * ld + kc + 2 * (e % 32));
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int e = t + 256 * h;
+      Cs[2 * (e % 32)][e / 32] = v[h].x;
+      Cs[2 * (e % 32) + 1][e / 32] = v[h].y;
+    }
+  } else {
+#pragma unroll
+    for (int e = t; e < 8 * SB; e += 256) cp_async16(&Cs[e / 8][2 * (e % 8)], M + (size_t)(kc + e / 8) * ld + row + 2 * (e % 8));
+  }
+  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+#pragma unroll
+  for (int e = t; e < 8 * SB; e += 256)
+    {
+    const double2 x = *reinterpret_cast<const double2*>(&Cs[e / 8][2 * (e % 8)]);
+    *reinterpret_cast<double2*>(CT + (size_t)(e / 8) * ld + row + 2 * (e % 8)) = make_double2(-x.x, -x.y);
+  }
+  // thread: row r, columns c .. c + 3 of W_i
+  const int r = t & 15, c = (t >> 4) * 4;
+  double w[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 16
+  for (int q = 0; q < SB; ++q) {
+    const double x = Cs[q][r];
+    const double2 d0 = *reinterpret_cast<const double2*>(&Ds[q][c]), d1 = *reinterpret_cast<const double2*>(&Ds[q][c + 2]);
+    w[0] += x * d0.x; w[1] += x * d0.y; w[2] += x * d1.x; w[3] += x * d1.y;
+  }
+#pragma unroll
+  for (int v = 0; v < 4; ++v) WT[(size_t)(c + v) * ld + row + r] = w[v];
+  if (i < k) {
+#pragma unroll
+    for (int v = 0; v < 4; ++v) M[(size_t)(kc + c + v) * ld + row + r] = w[v];
+  } else {
+    double2* p = reinterpret_cast<double2*>(M + (size_t)(row + r) * ld + kc + c);
+    p[0] = make_double2(w[0], w[1]);
+    p[1] = make_double2(w[2], w[3]);
+  }
+}
+
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
+
+// Step k's update of the lower tiles outside the pivot panel: S_ij -= C_i W_j^T (64 x 64 x 64 a CTA, 32 x 16 a
+// warp).  The FP64 matrix instruction has the scalar FMA's rate (64 a clock and SM) but needs a sixth of its operand
+// reads from shared memory, which bounded the scalar form (4 x 4 a thread: 12 TFLOP/s of 37).  The CTA of the next
+// pivot block (block 0, so that it starts first) inverts it on the spot: the serial part of the sweep runs beside
+// the other tiles instead of between two steps.
+constexpr int ULD = SB + 8;   // operand pitch: the four k rows of a fragment fall on both halves of the banks
+
 __global__ void __launch_bounds__(256)
 k_sweep_update(double* __restrict__ M, int ld, int k, const double* __restrict__ CT, const double* __restrict__ WT,
                double* __restrict__ Dinv, int* __restrict__ status) {
   extern __shared__ __align__(16) double sm[];
-  double (*As)[SB] = reinterpret_cast<double (*)[SB]>(sm);
-  double (*Bs)[SB] = reinterpret_cast<double (*)[SB]>(sm + SB * SB);
+  double (*As)[ULD] = reinterpret_cast<double (*)[ULD]>(sm);
+  double (*Bs)[ULD] = reinterpret_cast<double (*)[ULD]>(sm + SB * ULD);
   const int nt = ld / SB, t = threadIdx.x;
   const bool has_next = k + 1 < nt;
   // tiles a >= b over the nt - 1 block rows without k; linear index a (a + 1) / 2 + b; the next pivot (a = b = k) first
@@ -198,98 +250,111 @@ k_sweep_update(double* __restrict__ M, int ld, int k, const double* __restrict__
   while (a * (a + 1) / 2 > lin) --a;
   const int b = lin - a * (a + 1) / 2;
   const int i0 = (a + (a >= k)) * SB, j0 = (b + (b >= k)) * SB;
+#pragma unroll
   for (int e = t; e < SB * SB / 2; e += 256) {
     const int q = e / (SB / 2), c = 2 * (e % (SB / 2));
     cp_async16(&As[q][c], CT + (size_t)q * ld + i0 + c);
     cp_async16(&Bs[q][c], WT + (size_t)q * ld + j0 + c);
   }
   asm volatile("cp.async.commit_group;\n" ::: "memory");
-  const int ty = t >> 4, tx = t & 15;
-  double s[4][4];
+  const int lane = t & 31, w = t >> 5;
+  const int r = 32 * (w >> 2) + (lane >> 2), c = 16 * (w & 3) + 2 * (lane & 3);   // first row, column pair held
+  double s[4][2][2];
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const double2* p = reinterpret_cast<const double2*>(M + (size_t)(i0 + 4 * ty + u) * ld + j0 + 4 * tx);
-    const double2 x = p[0], y = p[1];
-    s[u][0] = x.x; s[u][1] = x.y; s[u][2] = y.x; s[u][3] = y.y;
-  }
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+      const double2 x = *reinterpret_cast<const double2*>(M + (size_t)(i0 + r + 8 * u) * ld + j0 + c + 8 * v);
+      s[u][v][0] = x.x;
+      s[u][v][1] = x.y;
+    }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   __syncthreads();
+  const double* Ap = &As[lane & 3][32 * (w >> 2) + (lane >> 2)];
+  const double* Bp = &Bs[lane & 3][16 * (w & 3) + (lane >> 2)];
 #pragma unroll 4
-  for (int q = 0; q < SB; ++q) {
-    double av[4], bv[4];
+  for (int q = 0; q < SB; q += 4) {
+    double av[4], bv[2];
 #pragma unroll
-    for (int u = 0; u < 4; u += 2) {
-      const double2 x = *reinterpret_cast<const double2*>(&As[q][4 * ty + u]);
-      const double2 y = *reinterpret_cast<const double2*>(&Bs[q][4 * tx + u]);
-      av[u] = x.x; av[u + 1] = x.y; bv[u] = y.x; bv[u + 1] = y.y;
-    }
+    for (int u = 0; u < 4; ++u) av[u] = Ap[q * ULD + 8 * u];
+#pragma unroll
+    for (int v = 0; v < 2; ++v) bv[v] = Bp[q * ULD + 8 * v];
 #pragma unroll
     for (int u = 0; u < 4; ++u)
 #pragma unroll
-      for (int v = 0; v < 4; ++v) s[u][v] -= av[u] * bv[v];
+      for (int v = 0; v < 2; ++v) dmma(s[u][v], av[u], bv[v]);
   }
   if (has_next && blockIdx.x == 0) {
     __syncthreads();
-    sweep_block(s, reinterpret_cast<double (*)[SB]>(sm), ty, tx, status);
 #pragma unroll
     for (int u = 0; u < 4; ++u)
 #pragma unroll
-      for (int v = 0; v < 4; ++v) Dinv[(4 * ty + u) * SB + 4 * tx + v] = -s[u][v];
+      for (int v = 0; v < 2; ++v)
+        *reinterpret_cast<double2*>(&As[r + 8 * u][c + 8 * v]) = make_double2(s[u][v][0], s[u][v][1]);
+    __syncthreads();
+    const int ty = t >> 4, tx = t & 15;
+    double d[4][4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) d[u][v] = As[4 * ty + u][4 * tx + v];
+    sweep_block(d, reinterpret_cast<double (*)[SB + 2]>(&Bs[0][0]), ty, tx, status);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) Dinv[(4 * ty + u) * SB + 4 * tx + v] = -d[u][v];
     return;
   }
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    double2* p = reinterpret_cast<double2*>(M + (size_t)(i0 + 4 * ty + u) * ld + j0 + 4 * tx);
-    p[0] = make_double2(s[u][0], s[u][1]);
-    p[1] = make_double2(s[u][2], s[u][3]);
-  }
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int v = 0; v < 2; ++v)
+      *reinterpret_cast<double2*>(M + (size_t)(i0 + r + 8 * u) * ld + j0 + c + 8 * v) =
+          make_double2(s[u][v][0], s[u][v][1]);
 }
 
-// x = Minv b on the coarsest level in one launch: the first brows blocks take 8 RPW rows each (RPW rows per warp), the
-// remaining blocks zero the entries of nodes outside the dense system (cmap < 0), a disjoint set.  A block gathers b
-// through klist into shared memory once, so that its warps stream their rows of Minv with 16-byte loads and nothing
-// else (the gather inside the row loop, one 8-byte load per value, ran 2457 dofs at 28.8 us and 1.7 TB/s from L2).
+// x = Minv b on the coarsest level in one launch: the first brows blocks take a row a warp, the remaining blocks zero
+// the entries of nodes outside the dense system (cmap < 0), a disjoint set.  A block gathers b through klist into
+// shared memory once, so that its warps stream their rows of Minv with 16-byte loads and nothing else.  Bound by
+// reading Minv.  2457 dofs: 28.8 us with the gather inside the row loop, 9 us from L2 and 17 us from memory now; two
+// or four rows a warp, deeper unrolling, smaller blocks and an L2 prefetch of the rows were no faster (up to 40 %
+// slower).
 constexpr int kSolveChunk = 4096;
+constexpr int kSolveThreads = 512;
 
-template <typename T, int RPW>
-__global__ void __launch_bounds__(256)
+template <typename T>
+__global__ void __launch_bounds__(kSolveThreads)
 k_dense_solve(const double* __restrict__ Minv, int nd, int ld, const int* __restrict__ klist,
               const int* __restrict__ cmap, int64_t n, const T* __restrict__ b, T* __restrict__ x, int brows,
               const int* __restrict__ skip) {
   if (skip && *skip) return;
   if ((int)blockIdx.x < brows) {
     __shared__ __align__(16) double bs[kSolveChunk];
-    const int lane = threadIdx.x & 31, row0 = (blockIdx.x * 8 + threadIdx.x / 32) * RPW;
-    double acc[RPW][2] = {};
+    const int lane = threadIdx.x & 31, row = blockIdx.x * (kSolveThreads / 32) + threadIdx.x / 32;
+    double a0 = 0.0, a1 = 0.0;
     for (int c0 = 0; c0 < nd; c0 += kSolveChunk) {
       const int len = min(kSolveChunk, ld - c0);      // a multiple of 64
       if (c0) __syncthreads();
-      for (int j = threadIdx.x; j < len; j += 256) {
-        const int q = c0 + j;
-        bs[j] = q < nd ? double(b[3 * (int64_t)klist[q / 3] + q % 3]) : 0.0;
+#pragma unroll 8
+      for (int j = threadIdx.x; j < len; j += kSolveThreads) {
+        const int q = min(c0 + j, nd - 1);
+        const double v = double(b[3 * (int64_t)klist[q / 3] + q % 3]);
+        bs[j] = c0 + j < nd ? v : 0.0;
       }
       __syncthreads();
-      if (row0 < nd) {        // rows past nd (< ld) are the identity's
-        const double2* m = reinterpret_cast<const double2*>(Minv + (size_t)row0 * ld + c0) + lane;
+      if (row < nd) {
+        const double2* m = reinterpret_cast<const double2*>(Minv + (size_t)row * ld + c0) + lane;
         const double2* bb = reinterpret_cast<const double2*>(bs) + lane;
 #pragma unroll 8
         for (int j = 0; j < len / 2; j += 32) {
-          const double2 v = bb[j];
-#pragma unroll
-          for (int r = 0; r < RPW; ++r) {
-            const double2 w = m[(size_t)r * (ld / 2) + j];
-            acc[r][0] += w.x * v.x;
-            acc[r][1] += w.y * v.y;
-          }
+          const double2 w = m[j], v = bb[j];
+          a0 += w.x * v.x;
+          a1 += w.y * v.y;
         }
       }
     }
-#pragma unroll
-    for (int r = 0; r < RPW; ++r) {
-      const double s = warp_sum(acc[r][0] + acc[r][1]);
-      const int row = row0 + r;
-      if (lane == 0 && row < nd) x[3 * (int64_t)klist[row / 3] + row % 3] = T(s);
-    }
+    const double s = warp_sum(a0 + a1);
+    if (lane == 0 && row < nd) x[3 * (int64_t)klist[row / 3] + row % 3] = T(s);
     return;
   }
   const int64_t e = (int64_t)(blockIdx.x - brows) * blockDim.x + threadIdx.x;
@@ -331,9 +396,12 @@ void launch_dense_add_entries(int nent, const int* rdof, const int* cdof, const 
 
 int dense_ld(int nd) { return div_up(nd, SB) * SB; }
 
+// Two launches a step.  Measured: the inverse of 1848 / 2457 / 3510 / 5265 dofs; an update takes 72 us at 5265 dofs
+// (25 TFLOP/s), and below about 3000 dofs the next pivot's chain of divisions (20 us) bounds it.  With 32-wide pivot
+// blocks over the whole matrix and five launches a step the inverse of 3510 dofs took 13.9 ms and that of 2457 6.3 ms.
 int launch_dense_invert(double* M, int nd, double* scratch, int* status, cudaStream_t s) {
   const int ld = dense_ld(nd), nt = ld / SB;
-  const int smem = 2 * SB * SB * (int)sizeof(double);
+  const int smem = 2 * SB * ULD * (int)sizeof(double);
   FEB_TRY(set_dyn_smem((const void*)k_sweep_update, smem));
   k_symmetrize<<<dim3(nt, nt), 256, 0, s>>>(M, nd, ld); note_launch();
   double* Dinv = scratch;
@@ -350,18 +418,12 @@ int launch_dense_invert(double* M, int nd, double* scratch, int* status, cudaStr
 
 size_t dense_scratch_doubles(int nd) { return (size_t)SB * SB + 2 * (size_t)SB * dense_ld(nd); }
 
-// Two rows a warp once one row a warp fills every SM twice (16 rows a block, 148 SMs): fewer gathers of b a row.
 template <typename T>
 void launch_dense_solve(const double* Minv, int nd, const int* klist, const int* cmap, int64_t n, const T* b, T* x,
                         const int* skip, cudaStream_t s) {
-  const int ld = dense_ld(nd), zero = div_up(3 * n, 256);
-  if (nd > 2 * 8 * kSmCount) {
-    const int brows = div_up(nd, 16);
-    k_dense_solve<T, 2><<<brows + zero, 256, 0, s>>>(Minv, nd, ld, klist, cmap, n, b, x, brows, skip);
-  } else {
-    const int brows = div_up(nd, 8);
-    k_dense_solve<T, 1><<<brows + zero, 256, 0, s>>>(Minv, nd, ld, klist, cmap, n, b, x, brows, skip);
-  }
+  const int brows = div_up(nd, kSolveThreads / 32);
+  k_dense_solve<T><<<brows + div_up(3 * n, kSolveThreads), kSolveThreads, 0, s>>>(Minv, nd, dense_ld(nd), klist, cmap, n,
+                                                                                  b, x, brows, skip);
   note_launch();
 }
 
