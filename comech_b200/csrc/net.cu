@@ -1,20 +1,22 @@
 // Learned warm start: the layers of a 3D convolutional encoder-decoder, its training steps, and its coupling to
 // the solve (network input from the solve's inputs, targets from solutions, the initial guess from a prediction).
 //
-// Convolutions are implicit GEMMs on the 5th-generation tensor cores.  A CTA of 128 threads owns 128 output rows
-// (256 for 3x3x3 convolutions, in two accumulators; rows are voxels of the padded grid) x NT output channels, its
-// FP32 accumulators in tensor memory.  The K loop runs over (tap group, 32-channel slice): each step stages the
-// gathered input rows x 32 channels (cp.async, zero fill for rows outside the grid) and the weight rows in a 3- or
-// 4-slot shared-memory ring, in the K-major unswizzled core-matrix layout, and one thread issues the step's
-// M128 x NT x K16 BF16 MMAs (2 per tap and accumulator) and commits them to the slot's mbarrier; the slot is
-// refilled once those MMAs have completed, so loads run ahead of the tensor core.  The epilogue reads the
-// accumulators back (tcgen05.ld), adds the bias, applies ReLU / the ReLU-gradient mask / accumulation, and stores
-// BF16 rows (direct, or scattered to the 8 fine cells of a transposed stride-2 conv).
+// Convolutions are implicit GEMMs on the 5th-generation tensor cores, FP32 accumulators in tensor memory, operands in
+// shared memory in the K-major unswizzled core-matrix layout.
+//   3x3x3 (k_conv3): persistent CTAs with producer, MMA and epilogue warps; one window of input rows in shared memory
+//   serves the nine (y, z) taps of a plane offset x, and the three z taps share one MMA as columns of N.
+//   2x2x2 stride 2, transposed and 1x1 (k_conv): a CTA of 128 threads owns 128 output rows x NT channels; each step of
+//   the K loop (tap, 32-channel slice) stages the gathered rows (cp.async, zero fill) and the weights in a 4-slot ring,
+//   one thread issues the step's two M128 x NT x K16 MMAs and commits them to the slot's mbarrier.
+// The epilogue reads the accumulators back (tcgen05.ld), adds the bias, applies ReLU / the ReLU-gradient mask /
+// accumulation, and stores BF16 rows (direct, or scattered to the 8 fine cells of a transposed stride-2 conv).
 //
 // Weight gradients (a reduction over voxels) use warp-level mma.sync with transposing ldmatrix loads of the
 // row-major activation tiles, split over row chunks with FP32 atomics into the gradient.
+#include <cuda.h>
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cfloat>
 
 #include "common.cuh"
@@ -30,22 +32,13 @@ using bf16 = __nv_bfloat16;
 constexpr int kConvThreads = 128;
 constexpr int kKS = 32;                          // channels per K step slice (two K16 MMAs per tap)
 
-// Shared-memory ring of the convolution.  A 3x3x3 (SHIFT) CTA owns 256 output rows (two M128 accumulators) and a
-// step covers the three z taps of one (x, y) offset: the rows they read are one window of 258 rows (stored as 264)
-// shifted by one row per tap, so one A tile serves the three taps and both halves through descriptors 16 bytes
-// apart (12 MMAs per step), and B holds the three taps' weights.  Other gathers: 128 rows, one tap per step.
-template <int NT, int GATHER> struct ConvSmem {
-  static constexpr bool kZ3 = GATHER == FEB_GATHER_SHIFT;
-  static constexpr int kM = kZ3 ? 256 : 128;     // output rows per CTA (kM / 128 accumulators of NT columns)
-  static constexpr int kHalves = kM / 128;
-  static constexpr int kARows = kZ3 ? kM + 8 : 128;
-  static constexpr int kAHalf = kARows * 16;     // bytes between 8-channel core-matrix columns of A
-  static constexpr int kA = kARows * kKS * 2;
-  static constexpr int kTaps = kZ3 ? 3 : 1;      // taps per step
-  static constexpr int kBTap = NT * kKS * 2;
-  static constexpr int kB = kTaps * kBTap;
+// Shared-memory ring of k_conv: 128 rows, one tap and 32-channel slice per step.
+template <int NT> struct ConvSmem {
+  static constexpr int kAHalf = 128 * 16;        // bytes between 8-channel core-matrix columns of A
+  static constexpr int kA = 128 * kKS * 2;
+  static constexpr int kB = NT * kKS * 2;
   static constexpr int kStage = kA + kB;
-  static constexpr int kStages = kZ3 ? 3 : 4;    // 3x3x3: 3 slots keep 3 CTAs per SM at N = 32
+  static constexpr int kStages = 4;
   static constexpr size_t kTotal = (size_t)kStages * kStage + 8 * kStages + 16;
 };
 
@@ -82,46 +75,32 @@ __device__ __forceinline__ int64_t fine_off(const FebNetGrid& f, int tap) {
   return ((int64_t)(tap >> 2) * (f.ny + 2) + ((tap >> 1) & 1)) * (f.nz + 2) + (tap & 1);
 }
 
-// one K step of A (gathered rows) and B (weights) into a ring slot.  SHIFT: step = ((x, y) offset p, channel slice),
-// A row i = input row m0 - 1 + i + offset(p), B = the weights of taps 3p, 3p+1, 3p+2 (dz = -1, 0, +1).  DOWN / ONE:
-// step = (tap, channel slice), A row i = the tap's source row of output row m0 + i.
+// one K step (tap, channel slice) of A (gathered rows: A row i = the tap's source row of output row m0 + i) and B
+// (weights) into a ring slot
 template <int NT, int GATHER>
 __device__ __forceinline__ void conv_load(const FebConv& P, int step, int kcs, uint32_t sA, int64_t m0, int64_t M,
-                                          int64_t Pin, const int64_t (&fbase)[4], int n0, int tid) {
-  using S = ConvSmem<NT, GATHER>;
-  const int grp = step / kcs, c0 = (step - grp * kcs) * kKS;
+                                          const int64_t (&fbase)[4], int n0, int tid) {
+  using S = ConvSmem<NT>;
+  const int tap = step / kcs, c0 = (step - tap * kcs) * kKS;
   const bf16* in = reinterpret_cast<const bf16*>(P.in);
-  if (GATHER == FEB_GATHER_SHIFT) {
-    const int dx = grp / 3 - 1, dy = grp % 3 - 1;
-    const int64_t off = ((int64_t)dx * (P.grid.ny + 2) + dy) * (P.grid.nz + 2);
-    for (int e = tid; e < S::kARows * 4; e += kConvThreads) {
-      const int row = e >> 2, ch = e & 3;
-      int64_t src = m0 - 1 + row + off;
-      if (row >= S::kM + 2 || src < 0 || src >= Pin) src = -1;
-      const bf16* g = src >= 0 ? in + src * P.in_ld + P.in_c0 + c0 + ch * 8 : in;
-      cp16(sA + ch * S::kAHalf + row * 16, g, src >= 0 ? 16 : 0);
-    }
-  } else {
-    const int ch = tid & 3;
-    const int64_t off = GATHER == FEB_GATHER_DOWN ? fine_off(P.fine, grp) : 0;
+  const int ch = tid & 3;
+  const int64_t off = GATHER == FEB_GATHER_DOWN ? fine_off(P.fine, tap) : 0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int row = (tid >> 2) + 32 * i;
-      const int64_t m = m0 + row;
-      int64_t src;
-      if (GATHER == FEB_GATHER_DOWN) src = fbase[i] >= 0 ? fbase[i] + off : -1;
-      else src = m < M ? m : -1;
-      const bf16* g = src >= 0 ? in + src * P.in_ld + P.in_c0 + c0 + ch * 8 : in;
-      cp16(sA + ch * S::kAHalf + row * 16, g, src >= 0 ? 16 : 0);
-    }
+  for (int i = 0; i < 4; ++i) {
+    const int row = (tid >> 2) + 32 * i;
+    const int64_t m = m0 + row;
+    int64_t src;
+    if (GATHER == FEB_GATHER_DOWN) src = fbase[i] >= 0 ? fbase[i] + off : -1;
+    else src = m < M ? m : -1;
+    const bf16* g = src >= 0 ? in + src * P.in_ld + P.in_c0 + c0 + ch * 8 : in;
+    cp16(sA + ch * S::kAHalf + row * 16, g, src >= 0 ? 16 : 0);
   }
   const bf16* wt = reinterpret_cast<const bf16*>(P.wt);
   const uint32_t sB = sA + S::kA;
-  const int tap0 = GATHER == FEB_GATHER_SHIFT ? 3 * grp : grp;
 #pragma unroll
-  for (int i = 0; i < S::kTaps * NT / 32; ++i) {
-    const int e = tid + kConvThreads * i, t = e / (4 * NT), rem = e - t * 4 * NT, n = rem >> 2, c = rem & 3;
-    cp16(sB + t * S::kBTap + c * (NT * 16) + n * 16, wt + ((int64_t)(tap0 + t) * P.n + n0 + n) * P.kc + c0 + c * 8, 16);
+  for (int i = 0; i < NT / 32; ++i) {
+    const int e = tid + kConvThreads * i, n = e >> 2, c = e & 3;
+    cp16(sB + c * (NT * 16) + n * 16, wt + ((int64_t)tap * P.n + n0 + n) * P.kc + c0 + c * 8, 16);
   }
 }
 
@@ -146,24 +125,65 @@ __device__ __forceinline__ uint4 pack8(const float* v) {
   return q;
 }
 
+// 32 channels of one output row from the accumulator values: bias (of these channels; may be null), ReLU, accumulation,
+// ReLU-gradient mask, BF16 store
+__device__ __forceinline__ void conv_store(const FebConv& P, const float* bias, int64_t orow, int ocol, float (&v)[32]) {
+  if (bias) {
+#pragma unroll
+    for (int q = 0; q < 32; ++q) v[q] += bias[q];
+  }
+  if (P.relu) {
+#pragma unroll
+    for (int q = 0; q < 32; ++q) v[q] = fmaxf(v[q], 0.f);
+  }
+  uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(P.out) + orow * P.out_ld + P.out_c0 + ocol);
+  if (P.accumulate) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float o[8];
+      unpack8(dst[q], o);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[8 * q + e] += o[e];
+    }
+  }
+  if (P.mask) {
+    const uint4* mk =
+        reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(P.mask) + orow * P.mask_ld + P.mask_c0 + ocol);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float o[8];
+      unpack8(mk[q], o);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[8 * q + e] = o[e] > 0.f ? v[8 * q + e] : 0.f;
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) dst[q] = pack8(v + 8 * q);
+}
+
+__device__ __forceinline__ void conv_zero(const FebConv& P, int64_t orow, int ocol) {
+  uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(P.out) + orow * P.out_ld + P.out_c0 + ocol);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) dst[q] = make_uint4(0u, 0u, 0u, 0u);
+}
+
 template <int NT, int GATHER, int SCATTER>
-__global__ void __launch_bounds__(kConvThreads) k_conv(const FebConv P, int64_t M, int64_t Pin) {
+__global__ void __launch_bounds__(kConvThreads) k_conv(const FebConv P, int64_t M) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  using S = ConvSmem<NT, GATHER>;
+  using S = ConvSmem<NT>;
   constexpr int kStages = S::kStages;
   uint64_t* mbar = reinterpret_cast<uint64_t*>(smem + kStages * S::kStage);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + kStages);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int64_t m0 = (int64_t)blockIdx.x * S::kM;
+  const int64_t m0 = (int64_t)blockIdx.x * 128;
   const int n0 = blockIdx.y * NT;
-  constexpr uint32_t kCols = NT * S::kHalves;
 
   if (tid == 0) {
 #pragma unroll
     for (int s = 0; s < kStages; ++s) tc::mbar_init(mbar + s, 1);
     tc::mbar_fence_init();
   }
-  if (warp == 0) tc::tmem_alloc(tslot, kCols);
+  if (warp == 0) tc::tmem_alloc(tslot, NT);
 
   // DOWN gather: the fine row of cell 2V of this thread's four A rows (-1 for shell / out-of-range rows)
   int64_t fbase[4] = {-1, -1, -1, -1};
@@ -176,12 +196,11 @@ __global__ void __launch_bounds__(kConvThreads) k_conv(const FebConv P, int64_t 
     }
   }
   const int kcs = P.kc / kKS;
-  const int ngroups = GATHER == FEB_GATHER_SHIFT ? 9 : (GATHER == FEB_GATHER_DOWN ? 8 : 1);
-  const int nk = ngroups * kcs;
+  const int nk = (GATHER == FEB_GATHER_DOWN ? 8 : 1) * kcs;
   const uint32_t base = tc::smem_addr(smem);
 #pragma unroll
   for (int s = 0; s < kStages - 1; ++s) {
-    if (s < nk) conv_load<NT, GATHER>(P, s, kcs, base + s * S::kStage, m0, M, Pin, fbase, n0, tid);
+    if (s < nk) conv_load<NT, GATHER>(P, s, kcs, base + s * S::kStage, m0, M, fbase, n0, tid);
     cp_commit();
   }
   tc::sync_for_tensor_core();
@@ -197,20 +216,16 @@ __global__ void __launch_bounds__(kConvThreads) k_conv(const FebConv P, int64_t 
     if (tid == 0) {
       const uint32_t a = base + slot * S::kStage, b = a + S::kA;
 #pragma unroll
-      for (int h = 0; h < S::kHalves; ++h)
-#pragma unroll
-        for (int t = 0; t < S::kTaps; ++t)
-#pragma unroll
-          for (int s = 0; s < 2; ++s)
-            tc::mma_bf16(tmem + (uint32_t)(h * NT), tc::smem_desc(a + (h * 128 + t) * 16 + 2 * s * S::kAHalf, S::kAHalf, 128),
-                         tc::smem_desc(b + t * S::kBTap + 2 * s * NT * 16, NT * 16, 128), idesc, (it | t | s) != 0);
+      for (int s = 0; s < 2; ++s)
+        tc::mma_bf16(tmem, tc::smem_desc(a + 2 * s * S::kAHalf, S::kAHalf, 128),
+                     tc::smem_desc(b + 2 * s * NT * 16, NT * 16, 128), idesc, (it | s) != 0);
       tc::commit(mbar + slot);
     }
     const int nxt = it + kStages - 1;
     if (nxt < nk) {
       // the slot of step nxt was last read by the MMAs of step it - 1
       if (it >= 1) ok = tc::mbar_wait(tc::smem_addr(mbar + (it - 1) % kStages), (uint32_t)(((it - 1) / kStages) & 1));
-      if (ok) conv_load<NT, GATHER>(P, nxt, kcs, base + (nxt % kStages) * S::kStage, m0, M, Pin, fbase, n0, tid);
+      if (ok) conv_load<NT, GATHER>(P, nxt, kcs, base + (nxt % kStages) * S::kStage, m0, M, fbase, n0, tid);
     }
     cp_commit();
   }
@@ -219,75 +234,238 @@ __global__ void __launch_bounds__(kConvThreads) k_conv(const FebConv P, int64_t 
   ok = __syncthreads_and(ok ? 1 : 0) != 0;
 
   if (ok) {
-   bf16* out = reinterpret_cast<bf16*>(P.out);
-   const bf16* mask = reinterpret_cast<const bf16*>(P.mask);
-#pragma unroll 1
-   for (int h = 0; h < S::kHalves; ++h) {
-    const int64_t m = m0 + h * 128 + 32 * warp + lane;
+    const int64_t m = m0 + 32 * warp + lane;
     int x = 0, y = 0, z = 0;
     const bool inside = m < M && row_cell(P.grid, m, x, y, z);
 #pragma unroll 1
     for (int cc = 0; cc < NT; cc += 32) {
       float v[32];
-      tc::tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(h * NT + cc), v);
+      tc::tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)cc, v);
       tc::wait_ld();
       const int n = n0 + cc;
-      int64_t orow;
-      int ocol;
       if (SCATTER) {
         if (!inside) continue;
         const int t = n / P.scatter_c;
-        ocol = n - t * P.scatter_c;
-        orow = prow(P.fine, 2 * x + (t >> 2), 2 * y + ((t >> 1) & 1), 2 * z + (t & 1));
+        conv_store(P, P.bias ? P.bias + (n - t * P.scatter_c) : nullptr,
+                   prow(P.fine, 2 * x + (t >> 2), 2 * y + ((t >> 1) & 1), 2 * z + (t & 1)), n - t * P.scatter_c, v);
       } else {
         if (m >= M) continue;
-        orow = m;
-        ocol = n;
-        if (!inside) {
-          uint4* dst = reinterpret_cast<uint4*>(out + orow * P.out_ld + P.out_c0 + ocol);
-#pragma unroll
-          for (int q = 0; q < 4; ++q) dst[q] = make_uint4(0u, 0u, 0u, 0u);
-          continue;
-        }
+        if (inside) conv_store(P, P.bias ? P.bias + n : nullptr, m, n, v);
+        else conv_zero(P, m, n);
       }
-      if (P.bias) {
-#pragma unroll
-        for (int q = 0; q < 32; ++q) v[q] += P.bias[ocol + q];
-      }
-      if (P.relu) {
-#pragma unroll
-        for (int q = 0; q < 32; ++q) v[q] = fmaxf(v[q], 0.f);
-      }
-      uint4* dst = reinterpret_cast<uint4*>(out + orow * P.out_ld + P.out_c0 + ocol);
-      if (P.accumulate) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          float o[8];
-          unpack8(dst[q], o);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) v[8 * q + e] += o[e];
-        }
-      }
-      if (mask) {
-        const uint4* mk = reinterpret_cast<const uint4*>(mask + orow * P.mask_ld + P.mask_c0 + ocol);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          float o[8];
-          unpack8(mk[q], o);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) v[8 * q + e] = o[e] > 0.f ? v[8 * q + e] : 0.f;
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q) dst[q] = pack8(v + 8 * q);
     }
-   }
   } else if (tid == 0 && P.status) {
     atomicExch(P.status, 1);
   }
   cp_wait<0>();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (warp == 0) tc::tmem_free(tmem, NT);
+}
+
+// ------------------------------------------------------------------------------------------ 3x3x3 convolution
+// A tap of the 3x3x3 kernel is a fixed distance in rows of the padded grid: dx PP + dy Pz + dz.  A step of the K loop
+// is (x offset, 32-channel slice): its A operand is one window of input rows in shared memory, and the operand of
+// (dy, half of the tile) is the same window from another first row (16 bytes a row, so any row is a legal start).  The
+// three dz taps are three column groups of one M128 x N96 x K16 MMA,
+//   D[i][t] = sum over x, dy of in[base + i + dx PP + dy Pz] . W(dx, dy, t),   out[r] = D[r - 1][0] + D[r][1] + D[r + 1][2],
+// so A is read from shared memory once for three taps (at N = 32 its 4 KB a MMA, 32 clocks, were twice the math's 16), and
+// 128 accumulator rows give 126 outputs; the neighbour rows' sums meet in the epilogue by shuffles and, at warp edges,
+// through shared memory.
+//
+// Persistent CTAs, one per SM, take tiles of H x 126 rows x 32 channels.  Four epilogue warps for each 126 rows, then a
+// producer warp and an MMA warp (one thread of each works).  The accumulators are double-buffered in tensor memory, so the
+// epilogue of a tile runs beside the next one's MMAs.
+//
+// A and B arrive by TMA (rows outside the grid read as zeros) in the 64-byte swizzle: rows of 32 channels, any row a legal
+// start.  cp.async into the unswizzled core-matrix layout filled 14 bytes a clock and SM (each 16 bytes of a row lands in
+// another column) and bounded every layer.
+//
+// When the window of three dy offsets would leave room for fewer than two slots (grids of some 500 cells along z), a step
+// takes one (x, y) offset instead (ndy = 1), with a window of the tile's rows alone.
+constexpr int kC3Rows = 126;                     // outputs of 128 accumulator rows
+constexpr int kC3Row = kKS * 2;                  // bytes of an operand row
+constexpr int kC3B = 96 * kC3Row;                // weight bytes of one (x, y) offset and slice: three dz taps x 32 columns
+constexpr int kC3Tail = 8 * (4 + 4 + 2 + 2) + 16 + 2 * (2 * 2 * 4 + 4) * 32 * 4;   // barriers, TMEM slot, edge rows, bias
+
+struct Conv3Plan {
+  int ndy, slots, boxes, box, stage;             // dy offsets a step, ring slots, A boxes a step and rows a box, slot bytes
+};
+
+inline Conv3Plan conv3_plan(int nz, int halves) {
+  const int budget = 220 * 1024 - kC3Tail;
+  Conv3Plan p{};
+  for (int ndy = 3; ndy >= 1; ndy -= 2) {
+    const int64_t rows = (int64_t)kC3Rows * (halves - 1) + 128 + (int64_t)(ndy - 1) * (nz + 2);
+    const int64_t boxes = (rows + 255) / 256, box = ((rows + boxes - 1) / boxes + 15) / 16 * 16;   // slots stay 1 KB aligned
+    const int64_t stage = boxes * box * kC3Row + ndy * kC3B;
+    if (ndy == 3 && 2 * stage > budget) continue;
+    p.ndy = ndy; p.boxes = (int)boxes; p.box = (int)box; p.stage = (int)stage;
+    p.slots = (int)std::min<int64_t>(4, budget / stage);
+    break;
+  }
+  return p;
+}
+
+template <int H> constexpr int conv3_threads() { return 128 * H + 64; }
+
+template <int H>
+__global__ void __launch_bounds__(conv3_threads<H>(), 1)
+k_conv3(const FebConv P, const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, int64_t M,
+        Conv3Plan L, int mtiles, int ntiles) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + (size_t)L.slots * L.stage);
+  uint64_t* empty = full + 4;
+  uint64_t* tfull = empty + 4;
+  uint64_t* tempty = tfull + 2;
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(tempty + 2);
+  volatile uint32_t* dead = tslot + 1;
+  float (*edge)[2][2][4][32] = reinterpret_cast<float (*)[2][2][4][32]>(tslot + 4);   // [half][parity][direction][warp]
+  float (*sbias)[4][32] = reinterpret_cast<float (*)[4][32]>(edge + 2);               // [half][warp][channel]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  constexpr uint32_t kCols = 128 * 2 * H;        // 96 columns used of each 128
+  if (tid == 0) {
+    for (int s = 0; s < 4; ++s) { tc::mbar_init(full + s, 1); tc::mbar_init(empty + s, 1); }
+    for (int s = 0; s < 2; ++s) { tc::mbar_init(tfull + s, 1); tc::mbar_init(tempty + s, 4 * H); }
+    tc::mbar_fence_init();
+    *dead = 0;
+  }
+  if (warp == 0) tc::tmem_alloc(tslot, kCols);
+  tc::sync_for_tensor_core();
+  const uint32_t tmem = *tslot;
+  const int Pz = P.grid.nz + 2, PP = (P.grid.ny + 2) * Pz;
+  const int kcs = P.kc / kKS, groups = L.ndy == 3 ? 3 : 9, nst = groups * kcs;
+  const int ntile = mtiles * ntiles;
+  const uint32_t base = tc::smem_addr(smem);
+  const uint32_t bytesA = (uint32_t)(L.boxes * L.box * kC3Row);
+
+  if (warp == 4 * H) {                           // ---- producer
+    if (lane == 0) {
+      int it = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < ntile && ok; tile += gridDim.x) {
+        const int mt = tile / ntiles, n0 = (tile - mt * ntiles) * 32;
+        const int row0 = mt * (kC3Rows * H) - 1;                     // input row of accumulator row 0 at offset 0
+        for (int g = 0; g < groups && ok; ++g) {
+          const int src0 = row0 + (L.ndy == 3 ? (g - 1) * PP - Pz : (g / 3 - 1) * PP + (g % 3 - 1) * Pz);
+          for (int c0 = 0; c0 < P.kc; c0 += kKS, ++it) {
+            const int slot = it % L.slots;
+            if (it >= L.slots && (!tc::mbar_wait(tc::smem_addr(empty + slot), (uint32_t)((it / L.slots - 1) & 1)) || *dead)) {
+              ok = false;
+              break;
+            }
+            const uint32_t d = base + slot * L.stage;
+            tc::mbar_expect_tx(full + slot, (uint32_t)L.stage);
+            for (int q = 0; q < L.boxes; ++q)
+              tc::tma_load_2d(d + q * L.box * kC3Row, &mapA, P.in_c0 + c0, src0 + q * L.box, full + slot);
+            tc::tma_load_3d(d + bytesA, &mapB, c0, n0, g * L.ndy * 3, full + slot);
+          }
+        }
+      }
+      if (!ok) {                                 // the copies in flight land before the CTA leaves
+        *dead = 1;
+        for (int j = it > L.slots ? it - L.slots : 0; j < it; ++j)
+          tc::mbar_wait(tc::smem_addr(full + j % L.slots), (uint32_t)((j / L.slots) & 1));
+      }
+    }
+    __syncwarp();
+  } else if (warp == 4 * H + 1) {                // ---- MMA issue
+    if (lane == 0) {
+      constexpr uint32_t idesc = tc::idesc_bf16(128, 96);
+      int it = 0, nt = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < ntile && ok; tile += gridDim.x, ++nt) {
+        const int buf = nt & 1;
+        if (nt >= 2 && (!tc::mbar_wait(tc::smem_addr(tempty + buf), (uint32_t)(((nt >> 1) - 1) & 1)) || *dead)) {
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        for (int st = 0; st < nst; ++st, ++it) {
+          const int slot = it % L.slots;
+          if (!tc::mbar_wait(tc::smem_addr(full + slot), (uint32_t)((it / L.slots) & 1)) || *dead) { ok = false; break; }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t a = base + slot * L.stage, b = a + bytesA;
+          for (int dy = 0; dy < L.ndy; ++dy)
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+              const uint64_t bd = tc::smem_desc_sw64(b + dy * kC3B + s * 32);
+#pragma unroll
+              for (int h = 0; h < H; ++h)
+                tc::mma_bf16(tmem + (uint32_t)((buf * H + h) * 128),
+                             tc::smem_desc_sw64(a + (kC3Rows * h + dy * Pz) * kC3Row + s * 32), bd, idesc, (st | dy | s) != 0);
+            }
+          tc::commit(empty + slot);
+        }
+        if (ok) tc::commit(tfull + buf);
+      }
+      if (!ok) *dead = 1;
+    }
+    __syncwarp();
+  } else {                                       // ---- epilogue of half h
+    const int h = warp >> 2, w = warp & 3, i = 32 * w + lane;
+    int nt = 0;
+    for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x, ++nt) {
+      const int buf = nt & 1, mt = tile / ntiles, n0 = (tile - mt * ntiles) * 32;
+      if (P.bias && (nt == 0 || ntiles > 1)) {
+        __syncwarp();
+        sbias[h][w][lane] = P.bias[n0 + lane];
+        __syncwarp();
+      }
+      const int m = mt * (kC3Rows * H) + kC3Rows * h + i - 1;
+      const bool mine = i >= 1 && i <= kC3Rows && m < M;
+      const int q1 = m / Pz, z = m - q1 * Pz, x = q1 / (P.grid.ny + 2), y = q1 - x * (P.grid.ny + 2);
+      const bool inside = z >= 1 && z <= P.grid.nz && y >= 1 && y <= P.grid.ny && x >= 1 && x <= P.grid.nx;
+      const bool ok = tc::mbar_wait(tc::smem_addr(tfull + buf), (uint32_t)((nt >> 1) & 1)) && !*dead;
+      if (!tc::barrier_and(1 + h, 128, ok)) {
+        *dead = 1;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      float v[32], lo[32], hi[32];
+      const uint32_t ta = tmem + ((uint32_t)(32 * w) << 16) + (uint32_t)((buf * H + h) * 128);
+      tc::tmem_ld32(ta, lo);
+      tc::tmem_ld32(ta + 32, v);
+      tc::tmem_ld32(ta + 64, hi);
+      tc::wait_ld();
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(tempty + buf);
+      float (*ed)[4][32] = edge[h][nt & 1];
+      if (lane == 31) {
+#pragma unroll
+        for (int q = 0; q < 32; q += 4)
+          *reinterpret_cast<float4*>(&ed[0][w][q]) = make_float4(lo[q], lo[q + 1], lo[q + 2], lo[q + 3]);
+      }
+      if (lane == 0) {
+#pragma unroll
+        for (int q = 0; q < 32; q += 4)
+          *reinterpret_cast<float4*>(&ed[1][w][q]) = make_float4(hi[q], hi[q + 1], hi[q + 2], hi[q + 3]);
+      }
+      asm volatile("bar.sync %0, 128;" ::"r"(1 + h) : "memory");
+#pragma unroll
+      for (int q = 0; q < 32; ++q) {
+        lo[q] = __shfl_up_sync(0xffffffffu, lo[q], 1);
+        hi[q] = __shfl_down_sync(0xffffffffu, hi[q], 1);
+      }
+      if (lane == 0 && w > 0) {
+#pragma unroll
+        for (int q = 0; q < 32; ++q) lo[q] = ed[0][w - 1][q];
+      }
+      if (lane == 31 && w < 3) {
+#pragma unroll
+        for (int q = 0; q < 32; ++q) hi[q] = ed[1][w + 1][q];
+      }
+#pragma unroll
+      for (int q = 0; q < 32; ++q) v[q] = lo[q] + v[q] + hi[q];
+      if (!mine) continue;
+      if (inside) conv_store(P, P.bias ? sbias[h][w] : nullptr, m, n0, v);
+      else conv_zero(P, m, n0);
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (tid == 0 && *dead && P.status) atomicExch(P.status, 1);
   if (warp == 0) tc::tmem_free(tmem, kCols);
 }
 
@@ -777,22 +955,77 @@ __global__ void k_net_to_nodes(FebNetGrid net, Axes A, const float* __restrict__
 }
 
 template <int NT, int GATHER, int SCATTER>
-int launch_conv(const FebConv& c, int64_t M, int64_t Pin, cudaStream_t s) {
-  // set on every launch (microseconds): the attribute belongs to the current device, and a process may use several
-  FEB_CUDA(cudaFuncSetAttribute(k_conv<NT, GATHER, SCATTER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)ConvSmem<NT, GATHER>::kTotal));
-  const dim3 grid(div_up(M, ConvSmem<NT, GATHER>::kM), c.n / NT);
-  k_conv<NT, GATHER, SCATTER><<<grid, kConvThreads, ConvSmem<NT, GATHER>::kTotal, s>>>(c, M, Pin);
+int launch_conv(const FebConv& c, int64_t M, cudaStream_t s) {
+  FEB_TRY(set_dyn_smem((const void*)k_conv<NT, GATHER, SCATTER>, (int)ConvSmem<NT>::kTotal));
+  const dim3 grid(div_up(M, 128), c.n / NT);
+  k_conv<NT, GATHER, SCATTER><<<grid, kConvThreads, ConvSmem<NT>::kTotal, s>>>(c, M);
   note_launch();
   FEB_CUDA(cudaGetLastError());
   return FEB_OK;
 }
 
+// cuTensorMapEncodeTiled of the loaded driver (the library does not link libcuda); null without a driver
+using TensorMapEncode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                     const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                     CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+TensorMapEncode tensor_map_encode() {
+  static const TensorMapEncode fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult r{};
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &r) != cudaSuccess ||
+        r != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      return (TensorMapEncode) nullptr;
+    }
+    return (TensorMapEncode)p;
+  }();
+  return fn;
+}
+
+// tensor map of BF16 boxes of 32 channels in the 64-byte swizzle, zeros outside the tensor
+int conv3_map(CUtensorMap* m, const void* p, int rank, const cuuint64_t* dim, const cuuint64_t* stride, const cuuint32_t* box) {
+  const TensorMapEncode encode = tensor_map_encode();
+  const cuuint32_t one[3] = {1, 1, 1};
+  const CUresult r = !encode ? CUDA_ERROR_NOT_FOUND
+                             : encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(p), dim, stride, box,
+                                      one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+                                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r == CUDA_SUCCESS) return FEB_OK;
+  set_last_error("feb_net_conv: cuTensorMapEncodeTiled failed (%d)", (int)r);
+  return FEB_ERR_CUDA;
+}
+
+template <int H>
+int launch_conv3_tile(const FebConv& c, int64_t M, cudaStream_t s) {
+  const Conv3Plan p = conv3_plan(c.grid.nz, H);
+  CUtensorMap mapA, mapB;
+  const cuuint64_t dimA[2] = {(cuuint64_t)c.in_ld, (cuuint64_t)M}, strA[1] = {(cuuint64_t)c.in_ld * 2};
+  const cuuint32_t boxA[2] = {kKS, (cuuint32_t)p.box};
+  FEB_TRY(conv3_map(&mapA, c.in, 2, dimA, strA, boxA));
+  const cuuint64_t dimB[3] = {(cuuint64_t)c.kc, (cuuint64_t)c.n, 27}, strB[2] = {(cuuint64_t)c.kc * 2, (cuuint64_t)c.n * c.kc * 2};
+  const cuuint32_t boxB[3] = {kKS, 32, (cuuint32_t)(3 * p.ndy)};
+  FEB_TRY(conv3_map(&mapB, c.wt, 3, dimB, strB, boxB));
+  FEB_TRY(set_dyn_smem((const void*)k_conv3<H>, 227 * 1024));
+  const int mtiles = div_up(M, (int64_t)kC3Rows * H), ntiles = c.n / 32;
+  k_conv3<H><<<(int)std::min<int64_t>((int64_t)mtiles * ntiles, kSmCount), conv3_threads<H>(), p.slots * p.stage + kC3Tail, s>>>(
+      c, mapA, mapB, M, p, mtiles, ntiles);
+  note_launch();
+  FEB_CUDA(cudaGetLastError());
+  return FEB_OK;
+}
+
+// Tiles of 126 rows when all of them fit one wave (more SMs share a small layer), of 252 otherwise (half the weight
+// traffic a row).
+int launch_conv3(const FebConv& c, int64_t M, cudaStream_t s) {
+  if ((int64_t)div_up(M, kC3Rows) * (c.n / 32) <= kSmCount) return launch_conv3_tile<1>(c, M, s);
+  return launch_conv3_tile<2>(c, M, s);
+}
+
 template <int GATHER, int SCATTER>
-int dispatch_nt(const FebConv& c, int64_t M, int64_t Pin, cudaStream_t s) {
-  if (c.n % 128 == 0) return launch_conv<128, GATHER, SCATTER>(c, M, Pin, s);
-  if (c.n % 64 == 0) return launch_conv<64, GATHER, SCATTER>(c, M, Pin, s);
-  return launch_conv<32, GATHER, SCATTER>(c, M, Pin, s);
+int dispatch_nt(const FebConv& c, int64_t M, cudaStream_t s) {
+  if (c.n % 128 == 0) return launch_conv<128, GATHER, SCATTER>(c, M, s);
+  if (c.n % 64 == 0) return launch_conv<64, GATHER, SCATTER>(c, M, s);
+  return launch_conv<32, GATHER, SCATTER>(c, M, s);
 }
 
 template <int TA, int TB, int MODE>
@@ -856,11 +1089,10 @@ extern "C" int feb_net_conv(const FebConv* c, void* stream) {
   }
   cudaStream_t s = (cudaStream_t)stream;
   const int64_t M = grid_rows(c->grid);
-  const int64_t Pin = c->gather == FEB_GATHER_DOWN ? grid_rows(c->fine) : M;
-  if (c->scatter) return dispatch_nt<FEB_GATHER_ONE, 1>(*c, M, Pin, s);
-  if (c->gather == FEB_GATHER_SHIFT) return dispatch_nt<FEB_GATHER_SHIFT, 0>(*c, M, Pin, s);
-  if (c->gather == FEB_GATHER_DOWN) return dispatch_nt<FEB_GATHER_DOWN, 0>(*c, M, Pin, s);
-  return dispatch_nt<FEB_GATHER_ONE, 0>(*c, M, Pin, s);
+  if (c->scatter) return dispatch_nt<FEB_GATHER_ONE, 1>(*c, M, s);
+  if (c->gather == FEB_GATHER_SHIFT) return launch_conv3(*c, M, s);
+  if (c->gather == FEB_GATHER_DOWN) return dispatch_nt<FEB_GATHER_DOWN, 0>(*c, M, s);
+  return dispatch_nt<FEB_GATHER_ONE, 0>(*c, M, s);
 }
 
 extern "C" int feb_net_wgrad(const FebWgrad* w, void* stream) {

@@ -19,6 +19,13 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
          ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | (1ull << 46);
 }
 
+// The same for rows of 64 bytes in the 64-byte swizzle (16-byte chunk c of row r at chunk c ^ ((r >> 1) & 3)), 8-row groups
+// 512 bytes apart.  The swizzle is a function of the address, so a matrix may start at any row of a region that is
+// aligned to 512 bytes, and 32 bytes into it for the second K16 step.
+__device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t addr) {
+  return smem_desc(addr, 16, 512) | (4ull << 61);
+}
+
 // Instruction descriptor of kind::f16 with BF16 A and B (both K-major), FP32 D, tile M x N.
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
@@ -42,6 +49,40 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {
 }
 
 __device__ __forceinline__ void mbar_fence_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+
+// one arrival that also announces `bytes` of asynchronous copies into the barrier's phase
+__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
+}
+
+// TMA tile load into shared memory, completion counted on the mbarrier; `map` is a CUtensorMap in kernel parameter space
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* map, int x, int y, uint64_t* bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
+               "l"(map), "r"(smem_addr(bar)), "r"(x), "r"(y)
+               : "memory");
+}
+
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const void* map, int x, int y, int z, uint64_t* bar) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
+                   dst),
+               "l"(map), "r"(smem_addr(bar)), "r"(x), "r"(y), "r"(z)
+               : "memory");
+}
+
+// named barrier over `threads` threads with the AND of `ok`
+__device__ __forceinline__ bool barrier_and(int id, int threads, bool ok) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %3, 0;\n\tbarrier.cta.red.and.pred q, %1, %2, p;\n\tselp.b32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(r)
+      : "r"(id), "r"(threads), "r"((uint32_t)ok)
+      : "memory");
+  return r != 0;
+}
 
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   for (int i = 0; i < kWaitPolls; ++i) {
