@@ -26,6 +26,13 @@ __device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t addr) {
   return smem_desc(addr, 16, 512) | (4ull << 61);
 }
 
+// Operand read along its rows (MN-major): M or N runs over 32 channels of a row, then over blocks of 32 whose rows lie
+// `lbo` bytes apart (any multiple of a row: blocks may overlap); K runs over the rows.  Goes with kIdescMnMajor.
+__device__ __forceinline__ uint64_t smem_desc_sw64_mn(uint32_t addr, uint32_t lbo) {
+  return smem_desc(addr, lbo, 512) | (4ull << 61);
+}
+constexpr uint32_t kIdescMnMajor = (1u << 15) | (1u << 16);    // A and B both MN-major
+
 // Instruction descriptor of kind::f16 with BF16 A and B (both K-major), FP32 D, tile M x N.
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);

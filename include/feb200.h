@@ -378,7 +378,8 @@ FEB_API int feb_net_conv(const FebConv* c, void* stream);
 
 /* Weight gradient: dw[t][a][b] += sum over rows r of P[rowP(r, t)][p_c0 + a] * Q[rowQ(r, t)][q_c0 + b], rows r over
  * `grid`; mode SHIFT: rowP = r, rowQ = r + tap offset; DOWN: rowP = r (coarse), rowQ = fine cell 2V + t; UP:
- * rowP = fine cell 2V + t, rowQ = r (coarse).  na, nb multiples of 32.  dw [dev] fp32, accumulated. */
+ * rowP = fine cell 2V + t, rowQ = r (coarse).  na, nb multiples of 32.  dw [dev] fp32, accumulated.  A bounded
+ * tensor-core wait that ran out (mode SHIFT) leaves NaN in dw. */
 typedef struct FebWgrad {
   int32_t mode, pad_;
   FebNetGrid grid, fine;
