@@ -163,6 +163,14 @@ __device__ __forceinline__ void conv_zero(const FebConv& P, int64_t orow, int oc
   for (int q = 0; q < 4; ++q) dst[q] = make_uint4(0u, 0u, 0u, 0u);
 }
 
+__device__ __forceinline__ void load32(const float* p, float (&v)[32]) {   // 16-byte aligned
+#pragma unroll
+  for (int q = 0; q < 32; q += 4) {
+    const float4 f = *reinterpret_cast<const float4*>(p + q);
+    v[q] = f.x; v[q + 1] = f.y; v[q + 2] = f.z; v[q + 3] = f.w;
+  }
+}
+
 template <int NT, int GATHER, int SCATTER>
 __global__ void __launch_bounds__(kConvThreads) k_conv(const FebConv P, int64_t M) {
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -262,7 +270,7 @@ __global__ void __launch_bounds__(kConvThreads) k_conv(const FebConv P, int64_t 
 // ------------------------------------------------------------------------------------------ 3x3x3 convolution
 // A tap of the 3x3x3 kernel is a fixed distance in rows of the padded grid: dx PP + dy Pz + dz.  A step of the K loop
 // is (x offset, 32-channel slice): its A operand is one window of input rows in shared memory, and the operand of
-// (dy, half of the tile) is the same window from another first row (16 bytes a row, so any row is a legal start).  The
+// (dy, half of the tile) is the same window from another first row.  The
 // three dz taps are three column groups of one M128 x N96 x K16 MMA,
 //   D[i][t] = sum over x, dy of in[base + i + dx PP + dy Pz] . W(dx, dy, t),   out[r] = D[r - 1][0] + D[r][1] + D[r + 1][2],
 // so A is read from shared memory once for three taps (at N = 32 its 4 KB a MMA, 32 clocks, were twice the math's 16), and
@@ -273,56 +281,77 @@ __global__ void __launch_bounds__(kConvThreads) k_conv(const FebConv P, int64_t 
 // producer warp and an MMA warp (one thread of each works).  The accumulators are double-buffered in tensor memory, so the
 // epilogue of a tile runs beside the next one's MMAs.
 //
-// A and B arrive by TMA (rows outside the grid read as zeros) in the 64-byte swizzle: rows of 32 channels, any row a legal
-// start.  cp.async into the unswizzled core-matrix layout filled 14 bytes a clock and SM (each 16 bytes of a row lands in
+// A and B arrive by TMA (rows outside the grid read as zeros) in the swizzle of their rows of 32 or 64 channels: any row is a
+// legal start.  cp.async into the unswizzled core-matrix layout filled 14 bytes a clock and SM (each 16 bytes of a row lands in
 // another column) and bounded every layer.
 //
 // When the window of three dy offsets would leave room for fewer than two slots (grids of some 500 cells along z), a step
 // takes one (x, y) offset instead (ndy = 1), with a window of the tile's rows alone.
+//
+// Loads bound the layers (an SM takes a row of an operand window about every three clocks, 64 or 128 bytes alike), so rows are
+// 64 channels long where the channel count allows it (SL), and the weights of a CTA's 32 output channels stay in shared
+// memory when they leave room for two A slots (a CTA then keeps to its channel tile).
 constexpr int kC3Rows = 126;                     // outputs of 128 accumulator rows
-constexpr int kC3Row = kKS * 2;                  // bytes of an operand row
-constexpr int kC3B = 96 * kC3Row;                // weight bytes of one (x, y) offset and slice: three dz taps x 32 columns
-constexpr int kC3Tail = 8 * (4 + 4 + 2 + 2) + 16 + 2 * (2 * 2 * 4 + 4) * 32 * 4;   // barriers, TMEM slot, edge rows, bias
+constexpr int kC3Row = kKS * 2;                  // bytes of a 32-channel operand row
+constexpr int kC3Tail = 8 * (4 + 4 + 2 + 2 + 1) + 24 + 2 * (2 * 2 * 4 + 4) * 32 * 4;   // barriers, TMEM slot, edge rows, bias
 
 struct Conv3Plan {
   int ndy, slots, boxes, box, stage;             // dy offsets a step, ring slots, A boxes a step and rows a box, slot bytes
+  int resident;                                  // bytes of the resident weights; 0: a step brings its own
 };
 
-inline Conv3Plan conv3_plan(int nz, int halves) {
-  const int budget = 220 * 1024 - kC3Tail;
+// sl: channels a slice; halves: 126-row parts a tile
+inline Conv3Plan conv3_plan(int nz, int halves, int sl, int kc) {
+  const int64_t budget = 220 * 1024 - kC3Tail, row = sl * 2, all = (int64_t)27 * 32 * kc * 2;
   Conv3Plan p{};
   for (int ndy = 3; ndy >= 1; ndy -= 2) {
     const int64_t rows = (int64_t)kC3Rows * (halves - 1) + 128 + (int64_t)(ndy - 1) * (nz + 2);
     const int64_t boxes = (rows + 255) / 256, box = ((rows + boxes - 1) / boxes + 15) / 16 * 16;   // slots stay 1 KB aligned
-    const int64_t stage = boxes * box * kC3Row + ndy * kC3B;
-    if (ndy == 3 && 2 * stage > budget) continue;
-    p.ndy = ndy; p.boxes = (int)boxes; p.box = (int)box; p.stage = (int)stage;
-    p.slots = (int)std::min<int64_t>(4, budget / stage);
+    const int64_t a = boxes * box * row, both = a + ndy * 96 * row;
+    if (ndy == 3 && 2 * both > budget) continue;
+    p.ndy = ndy; p.boxes = (int)boxes; p.box = (int)box;
+    p.resident = all + 2 * a <= budget ? (int)all : 0;
+    p.stage = (int)(p.resident ? a : both);
+    p.slots = (int)std::min<int64_t>(4, (budget - p.resident) / p.stage);
     break;
   }
   return p;
 }
 
+// Position in a ring of slots and the parity of its pass; kept by counting (integer divisions in the one thread that issues
+// the MMAs idled the tensor cores for more than half of the time).
+struct RingPos {
+  int slot = 0;
+  uint32_t pass = 0;
+  __device__ __forceinline__ void next(int slots) {
+    if (++slot == slots) { slot = 0; ++pass; }
+  }
+};
+
 template <int H> constexpr int conv3_threads() { return 128 * H + 64; }
 
-template <int H>
+template <int H, int SL>
 __global__ void __launch_bounds__(conv3_threads<H>(), 1)
 k_conv3(const FebConv P, const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, int64_t M,
         Conv3Plan L, int mtiles, int ntiles) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + (size_t)L.slots * L.stage);
+  constexpr int kRow = SL * 2;                   // bytes of an operand row
+  const uint32_t ring = (uint32_t)(L.slots * L.stage);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + ring + L.resident);
   uint64_t* empty = full + 4;
   uint64_t* tfull = empty + 4;
   uint64_t* tempty = tfull + 2;
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(tempty + 2);
+  uint64_t* wfull = tempty + 2;
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(wfull + 1);
   volatile uint32_t* dead = tslot + 1;
-  float (*edge)[2][2][4][32] = reinterpret_cast<float (*)[2][2][4][32]>(tslot + 4);   // [half][parity][direction][warp]
+  float (*edge)[2][2][4][32] = reinterpret_cast<float (*)[2][2][4][32]>(wfull + 4);   // [half][parity][direction][warp]
   float (*sbias)[4][32] = reinterpret_cast<float (*)[4][32]>(edge + 2);               // [half][warp][channel]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   constexpr uint32_t kCols = 128 * 2 * H;        // 96 columns used of each 128
   if (tid == 0) {
     for (int s = 0; s < 4; ++s) { tc::mbar_init(full + s, 1); tc::mbar_init(empty + s, 1); }
     for (int s = 0; s < 2; ++s) { tc::mbar_init(tfull + s, 1); tc::mbar_init(tempty + s, 4 * H); }
+    tc::mbar_init(wfull, 1);
     tc::mbar_fence_init();
     *dead = 0;
   }
@@ -330,70 +359,86 @@ k_conv3(const FebConv P, const __grid_constant__ CUtensorMap mapA, const __grid_
   tc::sync_for_tensor_core();
   const uint32_t tmem = *tslot;
   const int Pz = P.grid.nz + 2, PP = (P.grid.ny + 2) * Pz;
-  const int kcs = P.kc / kKS, groups = L.ndy == 3 ? 3 : 9, nst = groups * kcs;
-  const int ntile = mtiles * ntiles;
+  const int kcs = P.kc / SL, groups = L.ndy == 3 ? 3 : 9;
+  // tiles: channel tile blockIdx.x mod ntiles for good, row tiles from blockIdx.x / ntiles on (the grid is a multiple of
+  // ntiles, or has one tile a CTA)
+  const int n0 = (int)(blockIdx.x % ntiles) * 32, mt0 = blockIdx.x / ntiles, mstep = max(1, (int)gridDim.x / ntiles);
   const uint32_t base = tc::smem_addr(smem);
-  const uint32_t bytesA = (uint32_t)(L.boxes * L.box * kC3Row);
+  const uint32_t bytesA = (uint32_t)(L.boxes * L.box * kRow);
 
   if (warp == 4 * H) {                           // ---- producer
     if (lane == 0) {
-      int it = 0;
+      RingPos at;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < ntile && ok; tile += gridDim.x) {
-        const int mt = tile / ntiles, n0 = (tile - mt * ntiles) * 32;
+      if (L.resident) {                          // [slice][tap][n]
+        tc::mbar_expect_tx(wfull, (uint32_t)L.resident);
+        for (int q = 0; q < kcs; ++q) tc::tma_load_3d(base + ring + q * (27 * 32 * kRow), &mapB, q * SL, n0, 0, wfull);
+      }
+      for (int mt = mt0; mt < mtiles && ok; mt += mstep) {
         const int row0 = mt * (kC3Rows * H) - 1;                     // input row of accumulator row 0 at offset 0
         for (int g = 0; g < groups && ok; ++g) {
           const int src0 = row0 + (L.ndy == 3 ? (g - 1) * PP - Pz : (g / 3 - 1) * PP + (g % 3 - 1) * Pz);
-          for (int c0 = 0; c0 < P.kc; c0 += kKS, ++it) {
-            const int slot = it % L.slots;
-            if (it >= L.slots && (!tc::mbar_wait(tc::smem_addr(empty + slot), (uint32_t)((it / L.slots - 1) & 1)) || *dead)) {
+          for (int c0 = 0; c0 < P.kc; c0 += SL, at.next(L.slots)) {
+            if (at.pass && (!tc::mbar_wait(tc::smem_addr(empty + at.slot), (at.pass - 1) & 1) || *dead)) {
               ok = false;
               break;
             }
-            const uint32_t d = base + slot * L.stage;
-            tc::mbar_expect_tx(full + slot, (uint32_t)L.stage);
+            const uint32_t d = base + at.slot * L.stage;
+            tc::mbar_expect_tx(full + at.slot, (uint32_t)L.stage);
             for (int q = 0; q < L.boxes; ++q)
-              tc::tma_load_2d(d + q * L.box * kC3Row, &mapA, P.in_c0 + c0, src0 + q * L.box, full + slot);
-            tc::tma_load_3d(d + bytesA, &mapB, c0, n0, g * L.ndy * 3, full + slot);
+              tc::tma_load_2d(d + q * L.box * kRow, &mapA, P.in_c0 + c0, src0 + q * L.box, full + at.slot);
+            if (!L.resident) tc::tma_load_3d(d + bytesA, &mapB, c0, n0, g * L.ndy * 3, full + at.slot);
           }
         }
       }
       if (!ok) {                                 // the copies in flight land before the CTA leaves
         *dead = 1;
-        for (int j = it > L.slots ? it - L.slots : 0; j < it; ++j)
-          tc::mbar_wait(tc::smem_addr(full + j % L.slots), (uint32_t)((j / L.slots) & 1));
+        if (L.resident) tc::mbar_wait(tc::smem_addr(wfull), 0);
+        for (int j = 0; j < L.slots; ++j)        // slot j's last load: of this pass before the position, of the last one after
+          if (j < at.slot || at.pass) tc::mbar_wait(tc::smem_addr(full + j), (j < at.slot ? at.pass : at.pass - 1) & 1);
       }
     }
     __syncwarp();
   } else if (warp == 4 * H + 1) {                // ---- MMA issue
     if (lane == 0) {
       constexpr uint32_t idesc = tc::idesc_bf16(128, 96);
-      int it = 0, nt = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < ntile && ok; tile += gridDim.x, ++nt) {
-        const int buf = nt & 1;
-        if (nt >= 2 && (!tc::mbar_wait(tc::smem_addr(tempty + buf), (uint32_t)(((nt >> 1) - 1) & 1)) || *dead)) {
+      using D = tc::DescSwz<kRow>;
+      const uint32_t stepA = (uint32_t)(Pz * kRow) / 16, stepW = 27 * 32 * kRow;
+      RingPos at, buf;
+      bool ok = !L.resident || tc::mbar_wait(tc::smem_addr(wfull), 0);
+      for (int mt = mt0; mt < mtiles && ok; mt += mstep, buf.next(2)) {
+        if ((buf.pass && !tc::mbar_wait(tc::smem_addr(tempty + buf.slot), (buf.pass - 1) & 1)) || *dead) {
           ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        for (int st = 0; st < nst; ++st, ++it) {
-          const int slot = it % L.slots;
-          if (!tc::mbar_wait(tc::smem_addr(full + slot), (uint32_t)((it / L.slots) & 1)) || *dead) { ok = false; break; }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a = base + slot * L.stage, b = a + bytesA;
-          for (int dy = 0; dy < L.ndy; ++dy)
+        int acc = 0;
+        uint32_t wg = base + ring;               // resident weights of the group's first tap, slice 0
+        for (int g = 0; g < groups && ok; ++g, wg += L.ndy * (96 * kRow)) {
+          uint32_t wq = wg;
+          for (int q = 0; q < kcs; ++q, wq += stepW, at.next(L.slots)) {
+            ok = tc::mbar_wait(tc::smem_addr(full + at.slot), at.pass & 1);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t a = base + at.slot * L.stage;
+            // one thread issues, so its instructions count: descriptors move by their low word alone
+            const uint32_t da = D::lo(a), db = D::lo(L.resident ? wq : a + bytesA);
 #pragma unroll
-            for (int s = 0; s < 2; ++s) {
-              const uint64_t bd = tc::smem_desc_sw64(b + dy * kC3B + s * 32);
+            for (int dy = 0; dy < 3; ++dy) {
+              if (dy >= L.ndy) break;
 #pragma unroll
-              for (int h = 0; h < H; ++h)
-                tc::mma_bf16(tmem + (uint32_t)((buf * H + h) * 128),
-                             tc::smem_desc_sw64(a + (kC3Rows * h + dy * Pz) * kC3Row + s * 32), bd, idesc, (st | dy | s) != 0);
+              for (int s = 0; s < SL / 16; ++s)
+#pragma unroll
+                for (int h = 0; h < H; ++h)
+                  tc::mma_bf16(tmem + (uint32_t)((buf.slot * H + h) * 128),
+                               tc::desc_join(da + dy * stepA + (kC3Rows * h * kRow + s * 32) / 16, D::kHi),
+                               tc::desc_join(db + (dy * (96 * kRow) + s * 32) / 16, D::kHi), idesc, dy | s ? 1 : acc);
             }
-          tc::commit(empty + slot);
+            acc = 1;
+            tc::commit(empty + at.slot);
+          }
         }
-        if (ok) tc::commit(tfull + buf);
+        if (ok) tc::commit(tfull + buf.slot);
       }
       if (!ok) *dead = 1;
     }
@@ -401,13 +446,12 @@ k_conv3(const FebConv P, const __grid_constant__ CUtensorMap mapA, const __grid_
   } else {                                       // ---- epilogue of half h
     const int h = warp >> 2, w = warp & 3, i = 32 * w + lane;
     int nt = 0;
-    for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x, ++nt) {
-      const int buf = nt & 1, mt = tile / ntiles, n0 = (tile - mt * ntiles) * 32;
-      if (P.bias && (nt == 0 || ntiles > 1)) {
-        __syncwarp();
-        sbias[h][w][lane] = P.bias[n0 + lane];
-        __syncwarp();
-      }
+    if (P.bias) {
+      sbias[h][w][lane] = P.bias[n0 + lane];
+      __syncwarp();
+    }
+    for (int mt = mt0; mt < mtiles; mt += mstep, ++nt) {
+      const int buf = nt & 1;
       const int m = mt * (kC3Rows * H) + kC3Rows * h + i - 1;
       const bool mine = i >= 1 && i <= kC3Rows && m < M;
       const int q1 = m / Pz, z = m - q1 * Pz, x = q1 / (P.grid.ny + 2), y = q1 - x * (P.grid.ny + 2);
@@ -444,18 +488,17 @@ k_conv3(const FebConv P, const __grid_constant__ CUtensorMap mapA, const __grid_
         lo[q] = __shfl_up_sync(0xffffffffu, lo[q], 1);
         hi[q] = __shfl_down_sync(0xffffffffu, hi[q], 1);
       }
-      if (lane == 0 && w > 0) {
-#pragma unroll
-        for (int q = 0; q < 32; ++q) lo[q] = ed[0][w - 1][q];
-      }
-      if (lane == 31 && w < 3) {
-#pragma unroll
-        for (int q = 0; q < 32; ++q) hi[q] = ed[1][w + 1][q];
-      }
+      if (lane == 0 && w > 0) load32(ed[0][w - 1], lo);
+      if (lane == 31 && w < 3) load32(ed[1][w + 1], hi);
 #pragma unroll
       for (int q = 0; q < 32; ++q) v[q] = lo[q] + v[q] + hi[q];
       if (!mine) continue;
-      if (inside) conv_store(P, P.bias ? sbias[h][w] : nullptr, m, n0, v);
+      if (P.bias) {
+        load32(sbias[h][w], lo);
+#pragma unroll
+        for (int q = 0; q < 32; ++q) v[q] += lo[q];
+      }
+      if (inside) conv_store(P, nullptr, m, n0, v);
       else conv_zero(P, m, n0);
     }
   }
@@ -653,48 +696,52 @@ k_wgrad3(const FebWgrad W, const __grid_constant__ CUtensorMap mapP, const __gri
   if (warp == 4) {                               // ---- producer
     if (lane == 0) {
       bool ok = true;
-      int it = 0;
-      for (int st = st0; st < st1; ++st, ++it) {
-        const int slot = it % L.slots;
-        if (it >= L.slots && (!tc::mbar_wait(tc::smem_addr(empty + slot), (uint32_t)((it / L.slots - 1) & 1)) || *dead)) {
+      RingPos at;
+      for (int st = st0; st < st1; ++st, at.next(L.slots)) {
+        if (at.pass && (!tc::mbar_wait(tc::smem_addr(empty + at.slot), (at.pass - 1) & 1) || *dead)) {
           ok = false;
           break;
         }
         const int r = st * kWgRows - (L.ndy == 3 ? Pz : 0);       // first row r of the step
-        const uint32_t d = base + slot * L.stage;
-        tc::mbar_expect_tx(full + slot, (uint32_t)L.stage);
+        const uint32_t d = base + at.slot * L.stage;
+        tc::mbar_expect_tx(full + at.slot, (uint32_t)L.stage);
         for (int q = 0; q < L.boxes; ++q)
-          tc::tma_load_2d(d + q * L.box * kC3Row, &mapP, W.p_c0 + a0, r - (L.ndy == 3 ? Pz : 0) + q * L.box, full + slot);
+          tc::tma_load_2d(d + q * L.box * kC3Row, &mapP, W.p_c0 + a0, r - (L.ndy == 3 ? Pz : 0) + q * L.box, full + at.slot);
         for (int g = 0; g < nq; ++g) {
           const int off = L.ndy == 3 ? (g - 1) * PP : (g / 3 - 1) * PP + (g % 3 - 1) * Pz;
-          tc::tma_load_2d(d + bytesP + g * (kWgQ * kC3Row), &mapQ, W.q_c0 + b0, r + off - 1, full + slot);
+          tc::tma_load_2d(d + bytesP + g * (kWgQ * kC3Row), &mapQ, W.q_c0 + b0, r + off - 1, full + at.slot);
         }
       }
       if (!ok) {                                 // the copies in flight land before the CTA leaves
         *dead = 1;
-        for (int j = it > L.slots ? it - L.slots : 0; j < it; ++j)
-          tc::mbar_wait(tc::smem_addr(full + j % L.slots), (uint32_t)((j / L.slots) & 1));
+        for (int j = 0; j < L.slots; ++j)        // slot j's last load: of this pass before the position, of the last one after
+          if (j < at.slot || at.pass) tc::mbar_wait(tc::smem_addr(full + j), (j < at.slot ? at.pass : at.pass - 1) & 1);
       }
     }
     __syncwarp();
   } else if (warp == 5) {                        // ---- MMA issue
     if (lane == 0) {
       const uint32_t idesc = tc::idesc_bf16(128, 32 * L.ndy) | tc::kIdescMnMajor;
+      const uint32_t dcol = L.ndy == 3 ? 128 : 32;
       bool ok = true;
-      int it = 0;
-      for (int st = st0; st < st1; ++st, ++it) {
-        const int slot = it % L.slots;
-        if (!tc::mbar_wait(tc::smem_addr(full + slot), (uint32_t)((it / L.slots) & 1)) || *dead) { ok = false; break; }
+      int acc = 0;
+      RingPos at;
+      for (int st = st0; st < st1; ++st, at.next(L.slots)) {
+        ok = tc::mbar_wait(tc::smem_addr(full + at.slot), at.pass & 1);
+        if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t p = base + slot * L.stage, q = p + bytesP;
-        for (int g = 0; g < nq; ++g) {
+        const uint32_t p = base + at.slot * L.stage;
+        const uint32_t dp = tc::DescSwz64Mn::lo(p, Pz * kC3Row), dq = tc::DescSwz64Mn::lo(p + bytesP, kC3Row);
+#pragma unroll
+        for (int g = 0; g < 9; ++g) {
+          if (g >= nq) break;
 #pragma unroll
           for (int k = 0; k < kWgRows / 16; ++k)
-            tc::mma_bf16(tmem + (uint32_t)(g * (L.ndy == 3 ? 128 : 32)),
-                         tc::smem_desc_sw64_mn(q + g * (kWgQ * kC3Row) + k * 16 * kC3Row, kC3Row),
-                         tc::smem_desc_sw64_mn(p + k * 16 * kC3Row, Pz * kC3Row), idesc, (it | k) != 0);
+            tc::mma_bf16(tmem + g * dcol, tc::desc_join(dq + (g * kWgQ + k * 16) * (kC3Row / 16), tc::DescSwz64Mn::kHi),
+                         tc::desc_join(dp + k * kC3Row, tc::DescSwz64Mn::kHi), idesc, k ? 1 : acc);
         }
-        tc::commit(empty + slot);
+        acc = 1;
+        tc::commit(empty + at.slot);
       }
       if (ok) tc::commit(done);
       else *dead = 1;
@@ -1155,33 +1202,36 @@ TensorMapEncode tensor_map_encode() {
   return fn;
 }
 
-// tensor map of BF16 boxes of 32 channels in the 64-byte swizzle, zeros outside the tensor
+// tensor map of BF16 boxes of 32 or 64 channels in the swizzle of their 64- or 128-byte rows, zeros outside the tensor
 int conv3_map(CUtensorMap* m, const void* p, int rank, const cuuint64_t* dim, const cuuint64_t* stride, const cuuint32_t* box) {
   const TensorMapEncode encode = tensor_map_encode();
   const cuuint32_t one[3] = {1, 1, 1};
   const CUresult r = !encode ? CUDA_ERROR_NOT_FOUND
                              : encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(p), dim, stride, box,
-                                      one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+                                      one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                      box[0] == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
                                       CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r == CUDA_SUCCESS) return FEB_OK;
   set_last_error("network layer: cuTensorMapEncodeTiled failed (%d)", (int)r);
   return FEB_ERR_CUDA;
 }
 
-template <int H>
+template <int H, int SL>
 int launch_conv3_tile(const FebConv& c, int64_t M, cudaStream_t s) {
-  const Conv3Plan p = conv3_plan(c.grid.nz, H);
+  const Conv3Plan p = conv3_plan(c.grid.nz, H, SL, c.kc);
   CUtensorMap mapA, mapB;
   const cuuint64_t dimA[2] = {(cuuint64_t)c.in_ld, (cuuint64_t)M}, strA[1] = {(cuuint64_t)c.in_ld * 2};
-  const cuuint32_t boxA[2] = {kKS, (cuuint32_t)p.box};
+  const cuuint32_t boxA[2] = {SL, (cuuint32_t)p.box};
   FEB_TRY(conv3_map(&mapA, c.in, 2, dimA, strA, boxA));
   const cuuint64_t dimB[3] = {(cuuint64_t)c.kc, (cuuint64_t)c.n, 27}, strB[2] = {(cuuint64_t)c.kc * 2, (cuuint64_t)c.n * c.kc * 2};
-  const cuuint32_t boxB[3] = {kKS, 32, (cuuint32_t)(3 * p.ndy)};
+  const cuuint32_t boxB[3] = {SL, 32, (cuuint32_t)(p.resident ? 27 : 3 * p.ndy)};
   FEB_TRY(conv3_map(&mapB, c.wt, 3, dimB, strB, boxB));
-  FEB_TRY(set_dyn_smem((const void*)k_conv3<H>, 227 * 1024));
+  FEB_TRY(set_dyn_smem((const void*)k_conv3<H, SL>, 227 * 1024));
   const int mtiles = div_up(M, (int64_t)kC3Rows * H), ntiles = c.n / 32;
-  k_conv3<H><<<(int)std::min<int64_t>((int64_t)mtiles * ntiles, kSmCount), conv3_threads<H>(), p.slots * p.stage + kC3Tail, s>>>(
-      c, mapA, mapB, M, p, mtiles, ntiles);
+  // one CTA an SM, a whole number of rounds over the channel tiles (each CTA keeps to one)
+  const int64_t grid = std::min<int64_t>((int64_t)mtiles * ntiles, std::max(1, kSmCount / ntiles) * (int64_t)ntiles);
+  k_conv3<H, SL><<<(unsigned)grid, conv3_threads<H>(), p.slots * p.stage + p.resident + kC3Tail, s>>>(c, mapA, mapB, M, p, mtiles,
+                                                                                                  ntiles);
   note_launch();
   FEB_CUDA(cudaGetLastError());
   return FEB_OK;
@@ -1190,8 +1240,9 @@ int launch_conv3_tile(const FebConv& c, int64_t M, cudaStream_t s) {
 // Tiles of 126 rows when all of them fit one wave (more SMs share a small layer), of 252 otherwise (half the weight
 // traffic a row).
 int launch_conv3(const FebConv& c, int64_t M, cudaStream_t s) {
-  if ((int64_t)div_up(M, kC3Rows) * (c.n / 32) <= kSmCount) return launch_conv3_tile<1>(c, M, s);
-  return launch_conv3_tile<2>(c, M, s);
+  const bool one = (int64_t)div_up(M, kC3Rows) * (c.n / 32) <= kSmCount;
+  if (c.kc % 64 == 0) return one ? launch_conv3_tile<1, 64>(c, M, s) : launch_conv3_tile<2, 64>(c, M, s);
+  return one ? launch_conv3_tile<1, 32>(c, M, s) : launch_conv3_tile<2, 32>(c, M, s);
 }
 
 template <int GATHER, int SCATTER>

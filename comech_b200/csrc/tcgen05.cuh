@@ -19,18 +19,30 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
          ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | (1ull << 46);
 }
 
-// The same for rows of 64 bytes in the 64-byte swizzle (16-byte chunk c of row r at chunk c ^ ((r >> 1) & 3)), 8-row groups
-// 512 bytes apart.  The swizzle is a function of the address, so a matrix may start at any row of a region that is
-// aligned to 512 bytes, and 32 bytes into it for the second K16 step.
-__device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t addr) {
-  return smem_desc(addr, 16, 512) | (4ull << 61);
+// The two words of a descriptor, for loops that move its start address: the low word grows by one per 16 bytes.
+__device__ __forceinline__ uint64_t desc_join(uint32_t lo, uint32_t hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
+  return d;
 }
 
-// Operand read along its rows (MN-major): M or N runs over 32 channels of a row, then over blocks of 32 whose rows lie
-// `lbo` bytes apart (any multiple of a row: blocks may overlap); K runs over the rows.  Goes with kIdescMnMajor.
-__device__ __forceinline__ uint64_t smem_desc_sw64_mn(uint32_t addr, uint32_t lbo) {
-  return smem_desc(addr, lbo, 512) | (4ull << 61);
-}
+// K-major operand in rows of 64 or 128 bytes in the swizzle of that width (16-byte chunk c of row r at chunk
+// c ^ ((r >> 1) & 3) or c ^ (r & 7)), 8-row groups contiguous.  The swizzle is a function of the address, so a matrix may
+// start at any row of a region that is aligned to 8 rows, and a multiple of 32 bytes into it for the next K16 step.
+template <int ROW>
+struct DescSwz {
+  static_assert(ROW == 64 || ROW == 128, "rows of 32 or 64 BF16 values");
+  static constexpr uint32_t kHi = (8 * ROW >> 4) | (1u << 14) | (ROW == 64 ? 4u << 29 : 2u << 29);
+  static __device__ __forceinline__ uint32_t lo(uint32_t addr) { return ((addr >> 4) & 0x3FFF) | (1u << 16); }
+};
+
+// Operand in rows of 64 bytes read along its rows (MN-major): M or N runs over 32 channels of a row, then over blocks of
+// 32 whose rows lie `lbo` bytes apart (any multiple of a row: blocks may overlap); K runs over the rows.  Goes with
+// kIdescMnMajor.
+struct DescSwz64Mn {
+  static constexpr uint32_t kHi = DescSwz<64>::kHi;
+  static __device__ __forceinline__ uint32_t lo(uint32_t addr, uint32_t lbo) { return ((addr >> 4) & 0x3FFF) | ((lbo >> 4) << 16); }
+};
 constexpr uint32_t kIdescMnMajor = (1u << 15) | (1u << 16);    // A and B both MN-major
 
 // Instruction descriptor of kind::f16 with BF16 A and B (both K-major), FP32 D, tile M x N.
