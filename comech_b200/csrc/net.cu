@@ -121,13 +121,17 @@ __device__ __forceinline__ uint4 pack8(const float* v) {
   return q;
 }
 
-// 32 channels of one output row from the accumulator values: bias (of these channels; may be null), ReLU, accumulation,
-// ReLU-gradient mask, BF16 store
-__device__ __forceinline__ void conv_store(const FebConv& P, const float* bias, int64_t orow, int ocol, float (&v)[32]) {
-  if (bias) {
+// the ReLU-gradient mask's values of 32 channels of an output row
+__device__ __forceinline__ void conv_mask(const FebConv& P, int64_t orow, int ocol, uint4 (&mk)[4]) {
+  const uint4* p =
+      reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(P.mask) + orow * P.mask_ld + P.mask_c0 + ocol);
 #pragma unroll
-    for (int q = 0; q < 32; ++q) v[q] += bias[q];
-  }
+  for (int q = 0; q < 4; ++q) mk[q] = p[q];
+}
+
+// 32 channels of one output row from the accumulator values (bias added): ReLU, accumulation, ReLU-gradient mask (mk, when
+// the layer has one), BF16 store
+__device__ __forceinline__ void conv_store(const FebConv& P, const uint4 (&mk)[4], int64_t orow, int ocol, float (&v)[32]) {
   if (P.relu) {
 #pragma unroll
     for (int q = 0; q < 32; ++q) v[q] = fmaxf(v[q], 0.f);
@@ -143,8 +147,6 @@ __device__ __forceinline__ void conv_store(const FebConv& P, const float* bias, 
     }
   }
   if (P.mask) {
-    const uint4* mk =
-        reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(P.mask) + orow * P.mask_ld + P.mask_c0 + ocol);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       float o[8];
@@ -246,17 +248,24 @@ __global__ void __launch_bounds__(kConvThreads) k_conv(const FebConv P, int64_t 
       float v[32];
       tc::tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)cc, v);
       tc::wait_ld();
-      const int n = n0 + cc;
+      if (m >= M || (SCATTER && !inside)) continue;
+      int col = n0 + cc;
+      int64_t row = m;
       if (SCATTER) {
-        if (!inside) continue;
-        const int t = n / P.scatter_c;
-        conv_store(P, P.bias ? P.bias + (n - t * P.scatter_c) : nullptr,
-                   prow(P.fine, 2 * x + (t >> 2), 2 * y + ((t >> 1) & 1), 2 * z + (t & 1)), n - t * P.scatter_c, v);
-      } else {
-        if (m >= M) continue;
-        if (inside) conv_store(P, P.bias ? P.bias + n : nullptr, m, n, v);
-        else conv_zero(P, m, n);
+        const int t = col / P.scatter_c;
+        col -= t * P.scatter_c;
+        row = prow(P.fine, 2 * x + (t >> 2), 2 * y + ((t >> 1) & 1), 2 * z + (t & 1));
+      } else if (!inside) {
+        conv_zero(P, row, col);
+        continue;
       }
+      uint4 mk[4] = {};
+      if (P.mask) conv_mask(P, row, col, mk);
+      if (P.bias) {
+#pragma unroll
+        for (int q = 0; q < 32; ++q) v[q] += P.bias[col + q];
+      }
+      conv_store(P, mk, row, col, v);
     }
   } else if (tid == 0 && P.status) {
     atomicExch(P.status, 1);
@@ -456,6 +465,8 @@ k_conv3(const FebConv P, const __grid_constant__ CUtensorMap mapA, const __grid_
       const bool mine = i >= 1 && i <= kC3Rows && m < M;
       const int q1 = m / Pz, z = m - q1 * Pz, x = q1 / (P.grid.ny + 2), y = q1 - x * (P.grid.ny + 2);
       const bool inside = z >= 1 && z <= P.grid.nz && y >= 1 && y <= P.grid.ny && x >= 1 && x <= P.grid.nx;
+      uint4 mk[4] = {};
+      if (P.mask && mine && inside) conv_mask(P, m, n0, mk);         // on its way while the MMAs finish
       const bool ok = tc::mbar_wait(tc::smem_addr(tfull + buf), (uint32_t)((nt >> 1) & 1)) && !*dead;
       if (!tc::barrier_and(1 + h, 128, ok)) {
         *dead = 1;
@@ -498,7 +509,7 @@ k_conv3(const FebConv P, const __grid_constant__ CUtensorMap mapA, const __grid_
 #pragma unroll
         for (int q = 0; q < 32; ++q) v[q] += lo[q];
       }
-      if (inside) conv_store(P, nullptr, m, n0, v);
+      if (inside) conv_store(P, mk, m, n0, v);
       else conv_zero(P, m, n0);
     }
   }
