@@ -70,6 +70,22 @@ __global__ void k_csr_add(int nrow, const int* __restrict__ row_dof, const int* 
 }
 
 template <typename T>
+__device__ __forceinline__ void restrict_grid_at(const TransferDev& P, int jx, int jy, int jz, int fnx, int fny, const T* rf,
+                                                 T& s0, T& s1, T& s2) {
+  int Ix[3], Iy[3], Iz[3];
+  double wx[3], wy[3], wz[3];
+  int nxs = axis_fan(P.ax[0], jx, Ix, wx), nys = axis_fan(P.ax[1], jy, Iy, wy), nzs = axis_fan(P.ax[2], jz, Iz, wz);
+  s0 = s1 = s2 = T(0);
+  for (int c = 0; c < nzs; ++c)
+    for (int b = 0; b < nys; ++b)
+      for (int a = 0; a < nxs; ++a) {
+        int64_t f = Ix[a] + (int64_t)fnx * (Iy[b] + (int64_t)fny * Iz[c]);
+        T w = T(wx[a] * wy[b] * wz[c]);
+        s0 += w * rf[3 * f]; s1 += w * rf[3 * f + 1]; s2 += w * rf[3 * f + 2];
+      }
+}
+
+template <typename T>
 __global__ void k_restrict_grid(TransferDev P, int fnx, int fny, const T* __restrict__ rf, T* __restrict__ rc,
                                 const int* __restrict__ skip, T* __restrict__ zero, int nzero) {
   if (skip && *skip) return;
@@ -79,33 +95,17 @@ __global__ void k_restrict_grid(TransferDev P, int fnx, int fny, const T* __rest
   const int jx = blockIdx.x * blockDim.x + threadIdx.x, jy = blockIdx.y, jz = blockIdx.z;
   if (jx >= cnx) return;
   const int64_t J = jx + (int64_t)cnx * (jy + (int64_t)cny * jz);
-  int Ix[3], Iy[3], Iz[3];
-  double wx[3], wy[3], wz[3];
-  int nxs = axis_fan(P.ax[0], jx, Ix, wx), nys = axis_fan(P.ax[1], jy, Iy, wy), nzs = axis_fan(P.ax[2], jz, Iz, wz);
-  T s0 = 0, s1 = 0, s2 = 0;
-  for (int c = 0; c < nzs; ++c)
-    for (int b = 0; b < nys; ++b)
-      for (int a = 0; a < nxs; ++a) {
-        int64_t f = Ix[a] + (int64_t)fnx * (Iy[b] + (int64_t)fny * Iz[c]);
-        T w = T(wx[a] * wy[b] * wz[c]);
-        s0 += w * rf[3 * f]; s1 += w * rf[3 * f + 1]; s2 += w * rf[3 * f + 2];
-      }
+  T s0, s1, s2;
+  restrict_grid_at(P, jx, jy, jz, fnx, fny, rf, s0, s1, s2);
   rc[3 * J] = s0; rc[3 * J + 1] = s1; rc[3 * J + 2] = s2;
 }
 
 // r_c = P^T r_f for even coarsening: coarse node J gathers fine nodes 2 J + a, a in {-1, 0, 1} per axis, with
 // weight 1 (a = 0) or 1/2 (a = +-1)
 template <typename T>
-__global__ void k_restrict_even(int cnx, int cny, int fnx, int fny, int fnz, const T* __restrict__ rf,
-                                T* __restrict__ rc, const int* __restrict__ skip, T* __restrict__ zero, int nzero,
-                                const int* __restrict__ cp_ptr, const int* __restrict__ cp_copy,
-                                const double* __restrict__ cp_w, int64_t fnnode) {
-  if (skip && *skip) return;
-  if (nzero && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0)
-    for (int e = threadIdx.x; e < nzero; e += blockDim.x) zero[e] = T(0);
-  const int jx = blockIdx.x * blockDim.x + threadIdx.x, jy = blockIdx.y, jz = blockIdx.z;
-  if (jx >= cnx) return;
-  T s0 = 0, s1 = 0, s2 = 0;
+__device__ __forceinline__ void restrict_even_at(int jx, int jy, int jz, int fnx, int fny, int fnz, const T* rf, T& s0, T& s1,
+                                                 T& s2) {
+  s0 = s1 = s2 = T(0);
 #pragma unroll
   for (int c = -1; c <= 1; ++c) {
     const int fk = 2 * jz + c;
@@ -124,6 +124,20 @@ __global__ void k_restrict_even(int cnx, int cny, int fnx, int fny, int fnz, con
       }
     }
   }
+}
+
+template <typename T>
+__global__ void k_restrict_even(int cnx, int cny, int fnx, int fny, int fnz, const T* __restrict__ rf,
+                                T* __restrict__ rc, const int* __restrict__ skip, T* __restrict__ zero, int nzero,
+                                const int* __restrict__ cp_ptr, const int* __restrict__ cp_copy,
+                                const double* __restrict__ cp_w, int64_t fnnode) {
+  if (skip && *skip) return;
+  if (nzero && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0)
+    for (int e = threadIdx.x; e < nzero; e += blockDim.x) zero[e] = T(0);
+  const int jx = blockIdx.x * blockDim.x + threadIdx.x, jy = blockIdx.y, jz = blockIdx.z;
+  if (jx >= cnx) return;
+  T s0, s1, s2;
+  restrict_even_at(jx, jy, jz, fnx, fny, fnz, rf, s0, s1, s2);
   const int64_t J = jx + (int64_t)cnx * (jy + (int64_t)cny * jz);
   if (cp_ptr) {   // split copies restricting into J, in ascending copy order
     for (int e = cp_ptr[J]; e < cp_ptr[J + 1]; ++e) {
@@ -139,7 +153,7 @@ __global__ void k_restrict_even(int cnx, int cny, int fnx, int fny, int fnz, con
 // one the mean of its two neighbours
 // even coarsening: the interpolated coarse value at fine grid position (pi, pj, pk)
 template <typename T>
-__device__ __forceinline__ void even_interp(int cnx, int cny, int pi, int pj, int pk, const T* __restrict__ xc,
+__device__ __forceinline__ void even_interp(int cnx, int cny, int pi, int pj, int pk, const T* xc,
                                             T& s0, T& s1, T& s2) {
   const int ni = (pi & 1) + 1, nj = (pj & 1) + 1, nk = (pk & 1) + 1;
   const T wi = T(ni == 2 ? 0.5 : 1.0), wj = T(nj == 2 ? 0.5 : 1.0), wk = T(nk == 2 ? 0.5 : 1.0);
@@ -206,7 +220,7 @@ __global__ void k_restrict_copies(TransferDev P, int fnx, int fny, int64_t fnnod
 }
 
 template <typename T>
-__device__ __forceinline__ void prolong_at(const TransferDev& P, int pi, int pj, int pk, const T* __restrict__ xc,
+__device__ __forceinline__ void prolong_at(const TransferDev& P, int pi, int pj, int pk, const T* xc,
                                            T& s0, T& s1, T& s2) {
   int Jx[2], Jy[2], Jz[2];
   double wx[2], wy[2], wz[2];
@@ -711,7 +725,7 @@ struct SlotVals {
 };
 
 template <typename T, bool CMP, bool H, int Q>
-__device__ __forceinline__ void sym_load(const SymView<T>& L, const T* __restrict__ u, int n, int pn, int ic, int j,
+__device__ __forceinline__ void sym_load(const SymView<T>& L, const T* u, int n, int pn, int ic, int j,
                                          int k, int tn, const T* sp, const T* sm, SlotVals<T>& v) {
   constexpr int o = 13 + Q;
   constexpr int dx = o % 3 - 1, dy = (o / 3) % 3 - 1, dz = o / 9 - 1;
@@ -768,46 +782,26 @@ __device__ __forceinline__ void sym_acc(const SlotVals<T>& v, T& a0, T& a1, T& a
 }
 
 template <typename T, bool CMP, bool H, int Q>
-__device__ __forceinline__ void sym_slot(const SymView<T>& L, const T* __restrict__ u, int n, int pn, int ic, int j,
+__device__ __forceinline__ void sym_slot(const SymView<T>& L, const T* u, int n, int pn, int ic, int j,
                                          int k, int tn, const T* sp, const T* sm, T& a0, T& a1, T& a2) {
   SlotVals<T> v;
   sym_load<T, CMP, H, Q>(L, u, n, pn, ic, j, k, tn, sp, sm, v);
   sym_acc<T, Q>(v, a0, a1, a2);
 }
 
-// CMP: the level carries the compressed single-material blocks (tags); without them the pattern code is not
-// compiled into the kernel at all.  Offsets within the stencil planes are 32-bit (126 x the padded node count
-// < 2^31 is checked at launch).  H (with CT, FP32): the stored blocks are read from the 16-bit copy Sh and the
-// slot sums scaled by hscale before the entries and terms are added.
-template <typename T, int EPI, bool CMP, bool CT, bool H>
-__global__ void __launch_bounds__(128)
-k_sym(SymView<T> L, const T* __restrict__ u, T* __restrict__ y, const T* __restrict__ b, T* __restrict__ r,
-      T* __restrict__ d_out, T* __restrict__ x, const LevelParams* __restrict__ lp, int kstep,
-      const int* __restrict__ skip, TermAcc<T> acc) {
-  if (skip && *skip) return;
-  __shared__ T red[4][3][32];
-  __shared__ T spat[2][CMP ? 126 : 1];
-  __shared__ T smat[CMP ? 128 : 1][2];
-  const int lane = threadIdx.x, w = threadIdx.y;
-  if constexpr (CMP) {
-    const int tid = w * 32 + lane;
-    for (int e = tid; e < 252; e += 128) spat[e / 126][e % 126] = L.pat[e];
-    for (int e = tid; e < 256; e += 128) smat[e / 2][e % 2] = L.tmat[e];
-    __syncthreads();
-  }
-  const int i = blockIdx.x * 32 + lane, j = blockIdx.y, k = blockIdx.z;
+// One 32-node tile of the product: node n (lane's, clamped to the row; pn its padded position) and the share of warp w of 4
+// of its sum, without the epilogue.  CMP: the level carries the compressed single-material blocks (tags; patterns sp, sm in
+// shared memory); without them the pattern code is not compiled into the kernel at all.  Offsets within the stencil planes
+// are 32-bit (126 x the padded node count < 2^31 is checked at launch).  H (with CT, FP32): the stored blocks are read
+// from the 16-bit copy Sh and the slot sums scaled by hscale before the entries and terms are added.
+template <typename T, bool CMP, bool CT, bool H>
+__device__ __forceinline__ void sym_product(const SymView<T>& L, const T* u, int n, int pn, int ic, int j, int k, bool valid,
+                                            int lane, int w, const T* sp, const T* sm, T& a0, T& a1, T& a2) {
   const int nx = L.nx, ny = L.ny, nz = L.nz;
-  const bool valid = i < nx;
-  const int ic = valid ? i : nx - 1;
-  const int n = ic + nx * (j + ny * k);
-  const int N = (int)L.n;
   const int nxp = L.nxp, NP = (int)L.np;          // row-padded stencil planes
-  const int pn = ic + nxp * (j + ny * k);
   int tn = 0;
   if constexpr (CMP) tn = L.tag[n];
-  T a0 = 0, a1 = 0, a2 = 0;
-  const T* sp = CMP ? &spat[0][0] : nullptr;
-  const T* sm = CMP ? &smat[0][0] : nullptr;
+  a0 = a1 = a2 = T(0);
   if constexpr (CT) {
     // the 14 slots over the 4 warps (warp-uniform switch): 0 4 8 12 | 1 5 9 13 | 2 6 10 | 3 7 11
 #define FEB_SLOT(Q) sym_slot<T, CMP, H, Q>(L, u, n, pn, ic, j, k, tn, sp, sm, a0, a1, a2)
@@ -892,45 +886,90 @@ k_sym(SymView<T> L, const T* __restrict__ u, T* __restrict__ y, const T* __restr
       a2 += dot * L.tn_coef[3 * p + 2];
     }
   }
-  red[w][0][lane] = a0; red[w][1][lane] = a1; red[w][2][lane] = a2;
-  // epilogue operands that do not depend on the product, read before the barrier (r is rewritten after it)
-  const int c = w;
-  T rold0 = 0, rold1 = 0, rold2 = 0, bc = 0, uc = 0, xc = 0, D0 = 0, D1 = 0, D2 = 0;
-  if (c < 3 && valid) {
-    if constexpr (EPI == EPI_RESID) bc = b[3 * n + c];
-    if constexpr (EPI == EPI_CHEB) {
-      rold0 = r[3 * n]; rold1 = r[3 * n + 1]; rold2 = r[3 * n + 2];
-      uc = u[3 * n + c]; xc = x[3 * n + c];
-      D0 = L.Dinv[(3 * c) * N + n]; D1 = L.Dinv[(3 * c + 1) * N + n]; D2 = L.Dinv[(3 * c + 2) * N + n];   // 9 N < 2^31
+}
+
+// Epilogue operands of one node that do not depend on the product; thread of component c.  r_in: the residual before the
+// step (EPI_CHEB); u and x_in: the direction and the iterate at the node.
+template <typename T, int EPI>
+struct SymOps {
+  T r0, r1, r2, u, x, D0, D1, D2;
+  __device__ __forceinline__ void load(const SymView<T>& L, int n, int c, const T* ui, const T* b, const T* r_in,
+                                       const T* x_in) {
+    const int N = (int)L.n;                       // 9 N < 2^31
+    if constexpr (EPI == EPI_RESID) r0 = b[3 * n + c];
+    if constexpr (EPI == EPI_CHEB || EPI == EPI_START) {
+      const T* q = EPI == EPI_START ? b : r_in;
+      r0 = q[3 * n]; r1 = q[3 * n + 1]; r2 = q[3 * n + 2];
+      u = ui[3 * n + c];
+      if constexpr (EPI == EPI_CHEB) x = x_in[3 * n + c];
+      D0 = L.Dinv[(3 * c) * N + n]; D1 = L.Dinv[(3 * c + 1) * N + n]; D2 = L.Dinv[(3 * c + 2) * N + n];
     }
   }
-  __syncthreads();
-  if (c >= 3 || !valid) return;
+};
+
+// Finishes component c of node n from the four warps' partial sums red[w][component][lane].
+template <typename T, int EPI>
+__device__ __forceinline__ void sym_finish(const SymOps<T, EPI>& o, const T (*red)[3][32], int lane, int n, int c, T* y, T* r,
+                                           T* d_out, T* x_out, const LevelParams* lp, int kstep, const TermAcc<T>& acc) {
+  auto sum = [&](int q) { return red[0][q][lane] + red[1][q][lane] + red[2][q][lane] + red[3][q][lane]; };
   if constexpr (EPI == EPI_APPLY) {
-    y[3 * n + c] = red[0][c][lane] + red[1][c][lane] + red[2][c][lane] + red[3][c][lane];
+    y[3 * n + c] = sum(c);
   } else if constexpr (EPI == EPI_RESID) {
-    r[3 * n + c] = bc - (red[0][c][lane] + red[1][c][lane] + red[2][c][lane] + red[3][c][lane]);
+    r[3 * n + c] = o.r0 - sum(c);
   } else {
-    const T A0 = red[0][0][lane] + red[1][0][lane] + red[2][0][lane] + red[3][0][lane];
-    const T A1 = red[0][1][lane] + red[1][1][lane] + red[2][1][lane] + red[3][1][lane];
-    const T A2 = red[0][2][lane] + red[1][2][lane] + red[2][2][lane] + red[3][2][lane];
-    const T r0 = rold0 - A0, r1 = rold1 - A1, r2 = rold2 - A2;
-    const T rc = c == 0 ? r0 : (c == 1 ? r1 : r2);
-    const T c1 = T(lp->a1[kstep]), c2 = T(lp->a2[kstep]);
-    const T z = D0 * r0 + D1 * r1 + D2 * r2;
-    const T e = c1 * uc + c2 * z;
-    r[3 * n + c] = rc;
+    const T r0 = o.r0 - sum(0), r1 = o.r1 - sum(1), r2 = o.r2 - sum(2);
+    const T z = o.D0 * r0 + o.D1 * r1 + o.D2 * r2;
+    T e, x;
+    if constexpr (EPI == EPI_CHEB) {
+      e = T(lp->a1[kstep]) * o.u + T(lp->a2[kstep]) * z;
+      x = o.x + e;
+    } else {
+      e = T(lp->c_init) * z;
+      x = o.u + e;
+    }
+    r[3 * n + c] = c == 0 ? r0 : (c == 1 ? r1 : r2);
     d_out[3 * n + c] = e;
-    x[3 * n + c] = xc + e;
+    x_out[3 * n + c] = x;
     term_acc1(acc, n, c, e);
   }
+}
+
+template <typename T, int EPI, bool CMP, bool CT, bool H>
+__global__ void __launch_bounds__(128)
+k_sym(SymView<T> L, const T* __restrict__ u, T* __restrict__ y, const T* __restrict__ b, const T* r_in, T* r,
+      T* __restrict__ d_out, const T* x_in, T* x_out, const LevelParams* __restrict__ lp, int kstep,
+      const int* __restrict__ skip, TermAcc<T> acc) {
+  if (skip && *skip) return;
+  __shared__ T red[4][3][32];
+  __shared__ T spat[2][CMP ? 126 : 1];
+  __shared__ T smat[CMP ? 128 : 1][2];
+  const int lane = threadIdx.x, w = threadIdx.y;
+  if constexpr (CMP) {
+    const int tid = w * 32 + lane;
+    for (int e = tid; e < 252; e += 128) spat[e / 126][e % 126] = L.pat[e];
+    for (int e = tid; e < 256; e += 128) smat[e / 2][e % 2] = L.tmat[e];
+    __syncthreads();
+  }
+  const int i = blockIdx.x * 32 + lane, j = blockIdx.y, k = blockIdx.z;
+  const bool valid = i < L.nx;
+  const int ic = valid ? i : L.nx - 1;
+  const int n = ic + L.nx * (j + L.ny * k), pn = ic + L.nxp * (j + L.ny * k);
+  T a0, a1, a2;
+  sym_product<T, CMP, CT, H>(L, u, n, pn, ic, j, k, valid, lane, w, CMP ? &spat[0][0] : nullptr, CMP ? &smat[0][0] : nullptr,
+                             a0, a1, a2);
+  red[w][0][lane] = a0; red[w][1][lane] = a1; red[w][2][lane] = a2;
+  // epilogue operands, read before the barrier (r is rewritten after it)
+  SymOps<T, EPI> o;
+  if (w < 3 && valid) o.load(L, n, w, u, b, r_in, x_in);
+  __syncthreads();
+  if (w < 3 && valid) sym_finish<T, EPI>(o, red, lane, n, w, y, r, d_out, x_out, lp, kstep, acc);
 }
 
 }  // namespace
 
 template <typename T>
-void launch_sym(const SymView<T>& L0, int epi, const T* u, T* y, const T* b, T* r, T* d_out, T* x,
-                const LevelParams* lp, int k, const int* skip, cudaStream_t s, const T* tdot_in,
+void launch_sym(const SymView<T>& L0, int epi, const T* u, T* y, const T* b, const T* r_in, T* r, T* d_out, const T* x_in,
+                T* x, const LevelParams* lp, int k, const int* skip, cudaStream_t s, const T* tdot_in,
                 const TermAcc<T>& acc) {
   const dim3 g(div_up(L0.nx, 32), L0.ny, L0.nz), blk(32, 4);
   SymView<T> L = L0;
@@ -947,13 +986,14 @@ void launch_sym(const SymView<T>& L0, int epi, const T* u, T* y, const T* b, T* 
   }
   const bool cmp = L.tag != nullptr;
   const bool ct = L.slots == 2 || (L.slots == 0 && std::is_same<T, float>::value);
-#define FEB_SYM(E, C, CT_) k_sym<T, E, C, CT_, false><<<g, blk, 0, s>>>(L, u, y, b, r, d_out, x, lp, k, skip, acc)
+#define FEB_SYM(E, C, CT_) k_sym<T, E, C, CT_, false><<<g, blk, 0, s>>>(L, u, y, b, r_in, r, d_out, x_in, x, lp, k, skip, acc)
 #define FEB_SYM2(E, C) do { if (ct) FEB_SYM(E, C, true); else FEB_SYM(E, C, false); } while (0)
   if constexpr (std::is_same<T, float>::value) {
     if (L.Sh) {   // 16-bit storage: uncompressed levels, compile-time slots (the builder sets it only then)
-#define FEB_SYMH(E) k_sym<T, E, false, true, true><<<g, blk, 0, s>>>(L, u, y, b, r, d_out, x, lp, k, skip, acc)
+#define FEB_SYMH(E) k_sym<T, E, false, true, true><<<g, blk, 0, s>>>(L, u, y, b, r_in, r, d_out, x_in, x, lp, k, skip, acc)
       if (epi == EPI_APPLY) FEB_SYMH(EPI_APPLY);
       else if (epi == EPI_RESID) FEB_SYMH(EPI_RESID);
+      else if (epi == EPI_START) FEB_SYMH(EPI_START);
       else FEB_SYMH(EPI_CHEB);
 #undef FEB_SYMH
       note_launch();
@@ -964,6 +1004,8 @@ void launch_sym(const SymView<T>& L0, int epi, const T* u, T* y, const T* b, T* 
     if (cmp) FEB_SYM2(EPI_APPLY, true); else FEB_SYM2(EPI_APPLY, false);
   } else if (epi == EPI_RESID) {
     if (cmp) FEB_SYM2(EPI_RESID, true); else FEB_SYM2(EPI_RESID, false);
+  } else if (epi == EPI_START) {
+    if (cmp) FEB_SYM2(EPI_START, true); else FEB_SYM2(EPI_START, false);
   } else {
     if (cmp) FEB_SYM2(EPI_CHEB, true); else FEB_SYM2(EPI_CHEB, false);
   }
@@ -986,12 +1028,12 @@ void launch_stencil_to_sym(const double* A, int nx, int ny, int nz, T* S, cudaSt
   k_stencil_to_sym<T><<<div_up(np, kThreads), kThreads, 0, s>>>(A, nx, sym_nxp(nx), n, np, S); note_launch();
 }
 
-template void launch_sym<float>(const SymView<float>&, int, const float*, float*, const float*, float*, float*,
-                                float*, const LevelParams*, int, const int*, cudaStream_t, const float*,
+template void launch_sym<float>(const SymView<float>&, int, const float*, float*, const float*, const float*, float*, float*,
+                                const float*, float*, const LevelParams*, int, const int*, cudaStream_t, const float*,
                                 const TermAcc<float>&);
-template void launch_sym<double>(const SymView<double>&, int, const double*, double*, const double*, double*,
-                                 double*, double*, const LevelParams*, int, const int*, cudaStream_t, const double*,
-                                 const TermAcc<double>&);
+template void launch_sym<double>(const SymView<double>&, int, const double*, double*, const double*, const double*, double*,
+                                 double*, const double*, double*, const LevelParams*, int, const int*, cudaStream_t,
+                                 const double*, const TermAcc<double>&);
 void launch_galerkin_axis(const AxisDev& ax, int d, const double* Ain, int inx, int iny, int inz, double* Aout,
                           int onx, int ony, int onz, cudaStream_t s) {
   const int64_t no = (int64_t)onx * ony * onz;

@@ -91,15 +91,16 @@ struct SymView {
   const float* hscale = nullptr;
 };
 
-// Fused level kernels: EPI_APPLY y = A u; EPI_RESID r = b - A u; EPI_CHEB Chebyshev step with ping-pong
-// directions: t = A d_in, r -= t, d_out = a1 d_in + a2 Dinv r, x += d_out.
-enum SymEpi : int { EPI_APPLY = 0, EPI_RESID = 1, EPI_CHEB = 2 };
+// Fused level kernels: EPI_APPLY y = A u; EPI_RESID r = b - A u; EPI_CHEB Chebyshev step with ping-pong directions
+// (u the direction): r = r_in - A u, d_out = a1 u + a2 Dinv r, x = x_in + d_out; EPI_START start of a smoothing from the
+// iterate u: r = b - A u, d_out = c_init Dinv r, x = u + d_out (x another buffer than u).
+enum SymEpi : int { EPI_APPLY = 0, EPI_RESID = 1, EPI_CHEB = 2, EPI_START = 3 };
 struct LevelParams;
 // tdot_in: the rank-1 term dots of u, formed by u's producer (TermAcc); null: a k_term_dots pass forms them
 // first.  acc (EPI_CHEB): the dots of the new direction d_out are accumulated for the next product.
 template <typename T>
-void launch_sym(const SymView<T>& L, int epi, const T* u, T* y, const T* b, T* r, T* d_out, T* x,
-                const LevelParams* lp, int k, const int* skip, cudaStream_t s, const T* tdot_in = nullptr,
+void launch_sym(const SymView<T>& L, int epi, const T* u, T* y, const T* b, const T* r_in, T* r, T* d_out, const T* x_in,
+                T* x, const LevelParams* lp, int k, const int* skip, cudaStream_t s, const T* tdot_in = nullptr,
                 const TermAcc<T>& acc = TermAcc<T>());
 // full [243][n] FP64 stencil of an nx x ny x nz level -> row-padded half storage in T ([126][sym_np])
 template <typename T>

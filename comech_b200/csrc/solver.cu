@@ -1109,7 +1109,7 @@ struct FebHandle {
         default: launch_fine_apply<T, MAT_ORTHO>(F, u, y, skip, cfg, s); break;
       }
     } else {
-      launch_sym<T>(symview<T>(L[l]), EPI_APPLY, u, y, nullptr, nullptr, nullptr, nullptr, nullptr, 0, skip, s);
+      launch_sym<T>(symview<T>(L[l]), EPI_APPLY, u, y, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, skip, s);
     }
   }
   template <typename T>
@@ -1173,19 +1173,27 @@ struct FebHandle {
       const int deg = opt.cheb_degree, base = zero_start ? 1 : deg;
       auto buf = [&](int i) { return B ? B + (size_t)i * V.nterms : nullptr; };
       T* tdx = buf(0);
+      const T *r_in = r, *x_in = x;              // the first step reads b from a zero start, the start's iterate otherwise
       if (zero_start) {
-        launch_cheb_first<T>(b, r, d, x, D, lp + l, V.ntotal, skip, s,
+        launch_cheb_first<T>(b, nullptr, d, x, D, lp + l, V.ntotal, skip, s,
                              term_acc<T>(V, deg > 1 ? buf(base) : nullptr, tdx));
+        r_in = b;
+      } else if (deg > 1) {                      // residual and first direction in one product
+        T* xs = vt<T>(V);
+        launch_sym<T>(SV, EPI_START, x, nullptr, b, nullptr, r, d, nullptr, xs, lp + l, 0, skip, s, tdx,
+                      term_acc<T>(V, buf(base), nullptr));
+        x_in = xs;
       } else {
-        launch_sym<T>(SV, EPI_RESID, x, nullptr, b, r, nullptr, nullptr, nullptr, 0, skip, s, tdx);
-        launch_cheb_from_r<T>(r, d, x, D, lp + l, V.ntotal, skip, s,
-                              term_acc<T>(V, deg > 1 ? buf(base) : nullptr, nullptr));
+        launch_sym<T>(SV, EPI_RESID, x, nullptr, b, nullptr, r, nullptr, nullptr, nullptr, nullptr, 0, skip, s, tdx);
+        launch_cheb_from_r<T>(r, d, x, D, lp + l, V.ntotal, skip, s, term_acc<T>(V, nullptr, nullptr));
       }
       for (int k = 0; k + 1 < deg; ++k) {
         const bool last = k + 2 == deg;
-        launch_sym<T>(SV, EPI_CHEB, d, nullptr, nullptr, r, e, x, lp + l, k, skip, s, buf(base + k),
+        launch_sym<T>(SV, EPI_CHEB, d, nullptr, nullptr, r_in, r, e, x_in, x, lp + l, k, skip, s, buf(base + k),
                       term_acc<T>(V, last ? nullptr : buf(base + k + 1), zero_start ? tdx : nullptr));
         std::swap(d, e);
+        r_in = r;
+        x_in = x;
       }
       return;
     }
@@ -1267,7 +1275,7 @@ struct FebHandle {
     T *t = vt<T>(V), *r = vr<T>(V);
     T* tdx = tdb<T>(V);   // level l's iterate dots (buffer 0; null at level 0 and on levels without terms)
     if (l > 0) {
-      launch_sym<T>(symview<T>(V), EPI_RESID, x, nullptr, b, r, nullptr, nullptr, nullptr, 0, skip, s, tdx);
+      launch_sym<T>(symview<T>(V), EPI_RESID, x, nullptr, b, nullptr, r, nullptr, nullptr, nullptr, nullptr, 0, skip, s, tdx);
     } else {
       apply<T>(l, x, t, skip);
       launch_residual<T>(b, t, r, 3 * V.ntotal, skip, s);

@@ -203,7 +203,7 @@ __global__ void k_cheb_first(const T* __restrict__ b, T* __restrict__ r, T* __re
   const T c = T(lp->c_init);
   T r0 = b[3 * i], r1 = b[3 * i + 1], r2 = b[3 * i + 2], z0, z1, z2;
   bj(D, nn, i, r0, r1, r2, z0, z1, z2);
-  r[3 * i] = r0; r[3 * i + 1] = r1; r[3 * i + 2] = r2;
+  if (r) { r[3 * i] = r0; r[3 * i + 1] = r1; r[3 * i + 2] = r2; }
   z0 *= c; z1 *= c; z2 *= c;
   d[3 * i] = z0; d[3 * i + 1] = z1; d[3 * i + 2] = z2;
   x[3 * i] = z0; x[3 * i + 1] = z1; x[3 * i + 2] = z2;

@@ -90,7 +90,7 @@ template <typename Ta, typename Tb>
 void launch_dot_finalize(int kind, const Ta* a, const Tb* b, int64_t n, double* partials, unsigned int* ctr,
                          CgState* st, const int* skip, cudaStream_t s);
 
-// Chebyshev smoother pieces (Dinv SoA [9][nn], vectors AoS [3 nn])
+// Chebyshev smoother pieces (Dinv SoA [9][nn], vectors AoS [3 nn]); cheb_first: r (a copy of b) may be null
 template <typename T>
 void launch_cheb_first(const T* b, T* r, T* d, T* x, const T* Dinv, const LevelParams* lp, int64_t nn,
                        const int* skip, cudaStream_t s, const TermAcc<T>& acc = TermAcc<T>());
