@@ -1725,7 +1725,7 @@ std::vector<int> wave_chunks(FebHandle* h, int wy, bool smooth) {
   std::vector<int> zcs = {8, 16, 32};
   for (int waves = 1; waves <= 4; ++waves) {
     const int nbz = std::max(1, (waves * sms * per_sm) / std::max(txy, 1));
-    zcs.push_back(std::max(2, div_up(nzn, nbz)));
+    zcs.push_back(div_up(nzn, nbz));
   }
   std::sort(zcs.begin(), zcs.end());
   zcs.erase(std::unique(zcs.begin(), zcs.end()), zcs.end());
