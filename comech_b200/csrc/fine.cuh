@@ -41,15 +41,26 @@ struct KuConfig {
 template <typename T, int MODE>
 void launch_fine_apply(const FineView<T>& F, const T* u, T* y, const int* skip, KuConfig cfg, cudaStream_t s);
 
-// Sparse part of the level-0 operator only (irregular cells, penalties, extra entries), added with atomics
-// into acc (3 per node).
-template <typename T, int MODE>
-void launch_fine_sparse_into(const FineView<T>& F, const T* u, T* acc, const int* skip, cudaStream_t s);
-
 // ------------------------------------------------------------------------------------------------ paired K.u
-// Operator of the paired-row kernel (fine_pair.cu): regular cells by 7-bit material ids, the sparse part
-// through the accumulator tsp (zero between products), the smoother update fused in the epilogue.
+// Operator of the paired-row kernel (fine_pair.cu): regular cells by 7-bit material ids, penalty springs as a diagonal,
+// the nodes that irregular cells or extra entries reach (and the split copies) as a list of rows, the smoother update
+// fused in the epilogue.
 constexpr int kMaxMatIds = 128;   // ids 1..127; 0 = no regular cell
+
+// Nodes finished from their cells one by one: node[r], the codes of its up to 8 cells (cell[8 r + q]: the cell of which the node
+// is corner q), its penalties (kd) and its extra entries (dof columns; those of component c are ex[r][c] .. ex[r][c + 1]).
+template <typename T>
+struct PairRows {
+  int n = 0;
+  const int* node = nullptr;
+  const int* cell = nullptr;
+  const int* irr_cell = nullptr;
+  const int* irr_nodes = nullptr;
+  const T* irr_mat = nullptr;
+  const int4* ex = nullptr;
+  const int* ecol = nullptr;
+  const T* eval = nullptr;
+};
 
 template <typename T>
 struct PairView {
@@ -64,7 +75,9 @@ struct PairView {
   double h;
   const T* dx; const T* dy; const T* dz;      // cell widths per axis (general core)
   const T* idx; const T* idy; const T* idz;
-  T* tsp;                    // sparse-part accumulator, 3 per node (ntotal), zero between products
+  const T* kd;               // penalty diagonal, 3 per node (read at flagged nodes)
+  const uint8_t* rowflag;    // node is in the row list (read at flagged nodes)
+  PairRows<T> rows;
   const T* dinv6;            // symmetric block-Jacobi inverse [6][ntotal]: 00 11 22 01 02 12
 };
 
@@ -95,8 +108,8 @@ struct PairConfig {
 
 // y = K u (S null) or the smoother step S; returns a status
 template <typename T, int MODE>
-int launch_fine_pair(const PairView<T>& F, const FineView<T>& G, const T* u, T* y, const SmoothArgs<T>* S,
-                     const int* skip, PairConfig cfg, cudaStream_t s);
+int launch_fine_pair(const PairView<T>& F, const T* u, T* y, const SmoothArgs<T>* S, const int* skip, PairConfig cfg,
+                     cudaStream_t s);
 // sets the shared-memory limits of every paired-kernel variant of this model on the current device (call
 // before any stream capture)
 int prepare_fine_pair(int mode, bool cube);
@@ -109,6 +122,12 @@ void launch_mat_ids(const double* mat_s, int64_t ncell, unsigned long long* keys
                     int* status, cudaStream_t s);
 void launch_flag_nodes(const int* pen_node, int npen, const int* irr_nodes, int nirr, const int* row_dof, int nrow,
                        int64_t nnode, uint8_t* flag, cudaStream_t s);
+// set-up of the row list: flags of its nodes (with the irregular cell of every cell and the first CSR row of every node's extra
+// entries, both preset to -1), the penalty diagonal, the rows (ids: material id of every regular cell)
+void launch_row_flags(const FineView<double>& F, uint8_t* flag, int* cmap, int* start, cudaStream_t s);
+void launch_pen_diag(const int* node, const double* k, int n, double* kd, cudaStream_t s);
+void launch_rows(const FineView<double>& F, const int* node, int nrow, const int* orig_copy, const int* cmap, const int* start,
+                 const uint8_t* ids, int* cell, int4* ex, cudaStream_t s);
 template <int W>
 void launch_pack_pairs(int nx, int ny, int nz, int mp, const uint8_t* ids, const uint8_t* flag, const double* mat_s,
                        const double* vals, uint16_t* cellpair, int* status, cudaStream_t s);

@@ -1,13 +1,15 @@
 // Level-0 K.u on the voxel grid with paired node rows, and the smoother steps fused into its epilogue.
 //
-// Work split (one product y = K u, or one Chebyshev / residual step of the smoother):
-//   * the sparse remainder of the level-0 operator (cells touching split copies, penalty springs, extra
-//     entries) is accumulated first, with atomics, into the scratch vector `tsp` (k_fine_sparse);
-//   * k_fine_pair then computes the regular cells matrix-free.  A grid node whose 8 cells are all handled
-//     here (the bulk) is finished in registers: its product is stored, or the smoother update of that node
-//     runs on the spot (r -= K d, z = Dinv r, d' = a1 d + a2 z, x += d').  A node flagged "special" adds
-//     and clears its `tsp` entry first; split copies (ids >= nnode) are finished by tail blocks of the
-//     same launch from `tsp` alone.  `tsp` is zero again when the launch ends.
+// Work split of one launch (a product y = K u, or one Chebyshev / residual step of the smoother):
+//   * tile CTAs compute the regular cells matrix-free.  A grid node whose 8 cells are all handled here (the bulk) is
+//     finished in registers: its product is stored, or the smoother update of that node runs on the spot (r -= K d,
+//     z = Dinv r, d' = a1 d + a2 z, x += d').  A node flagged "special" with a penalty spring adds its diagonal first; one
+//     that cells touching split copies or extra entries reach is left out (its row flag is set).
+//   * those nodes and the split copies (PairRows) are finished by groups of eight lanes, one cell each, spread over all
+//     CTAs: each does its few while its first planes are on their way.  There are not many (1 % of the nodes of a
+//     160 x 112 x 96 foot).  As a kernel of its own ahead of the tiles, summing cells with atomics into a vector that the
+//     tiles added and cleared, this part took 5.3 / 6.2 / 9.2 us a product (24x18x16 / 96x64x48 / 160x112x96, FP32)
+//     however little there was to do; with assembled 3x3-block rows instead of cells it was bound by reading them.
 //
 // Tiling: a warp holds 32 node columns (30 owned, one halo column on each side) of two neighbouring node
 // rows; a CTA of WY warps holds 2 WY rows (2 WY - 2 owned) and marches in z over `zchunk` node planes.
@@ -30,6 +32,8 @@ namespace feb {
 namespace {
 
 constexpr int kXOwn = 30;
+// cell codes of the row list: an irregular cell's index, a regular cell's material id as kRegularCell - id, or none
+constexpr int kNoCell = -1, kRegularCell = -1;
 #ifndef FEB_PAIR_MINB
 #define FEB_PAIR_MINB 1
 #endif
@@ -195,6 +199,98 @@ __device__ __forceinline__ void node_update(const SmoothArgs<T>& S, T a1, T a2, 
   }
 }
 
+// the Chebyshev coefficients of the step (a residual-only step carries no parameters)
+template <typename T>
+__device__ __forceinline__ void pair_coef(const SmoothArgs<T>& S, T& a1, T& a2) {
+  if (S.lp && S.updates()) {
+    a1 = S.k < 0 ? T(0) : T(S.lp->a1[S.k]);
+    a2 = S.k < 0 ? T(S.lp->c_init) : T(S.lp->a2[S.k]);
+  }
+}
+
+// One node of the row list by a group of eight lanes, one cell each: the cell's force at its corner by the element operator
+// (the modal form of the tiles, back-transformed for that corner alone), summed over the group with the node's penalties
+// and extra entries.  Rows past the end: the group idles along.
+template <typename T, int MODE, bool CUBE, bool SMOOTH>
+__device__ __forceinline__ void finish_row(const PairView<T>& F, const T* __restrict__ u, T* __restrict__ y,
+                                           const SmoothArgs<T>& S, T a1, T a2, int row) {
+  constexpr int W = MatWidth<MODE>::value;
+  const PairRows<T>& R = F.rows;
+  const int q = threadIdx.x & 7, rc = min(row, R.n - 1);
+  const bool live = row < R.n;
+  const int n = R.node[rc], code = R.cell[8 * rc + q];
+  const int4 ex = R.ex[rc];
+  NodeOps<T> o;
+  if constexpr (SMOOTH) {
+    if (live && q == 0) load_node_ops(F, S, u, a1 != T(0), n, o);
+  }
+  T t[3] = {T(0), T(0), T(0)};
+  if (q < 3) t[q == 2 ? 2 : q] = F.kd[3 * n + q] * u[3 * n + q];
+  for (int e = ex.x + q; e < ex.w; e += 8) {
+    const T x = R.eval[e] * u[R.ecol[e]];
+    if (e < ex.y) t[0] += x;
+    else if (e < ex.z) t[1] += x;
+    else t[2] += x;
+  }
+  if (code != kNoCell) {
+    int id[8];
+    T m[W];
+    int cell = 0;                                // x-fastest cell index, for the widths of the general geometry
+    if (code >= 0) {
+      const int4 lo = reinterpret_cast<const int4*>(R.irr_nodes)[2 * code], hi = reinterpret_cast<const int4*>(R.irr_nodes)[2 * code + 1];
+      id[0] = lo.x; id[1] = lo.y; id[2] = lo.z; id[3] = lo.w; id[4] = hi.x; id[5] = hi.y; id[6] = hi.z; id[7] = hi.w;
+#pragma unroll
+      for (int p = 0; p < W; ++p) m[p] = R.irr_mat[(size_t)W * code + p];
+      if constexpr (!CUBE) cell = R.irr_cell[code];
+    } else {                                     // a regular cell around grid node n
+      const int n0 = n - (q & 1) - F.nxn * (((q >> 1) & 1) + F.nyn * (q >> 2));
+#pragma unroll
+      for (int l = 0; l < 8; ++l) id[l] = n0 + (l & 1) + F.nxn * (((l >> 1) & 1) + F.nyn * (l >> 2));
+#pragma unroll
+      for (int p = 0; p < W; ++p) m[p] = T(F.mtab[W * (kRegularCell - code) + p]);
+      if constexpr (!CUBE) {
+        const int i = n0 % F.nxn, j = (n0 / F.nxn) % F.nyn, k = n0 / (F.nxn * F.nyn);
+        cell = i + F.nx * (j + F.ny * k);
+      }
+    }
+    T X[8], Y[8], Z[8], FX[8], FY[8], FZ[8];
+#pragma unroll
+    for (int l = 0; l < 8; ++l) { X[l] = u[3 * id[l]]; Y[l] = u[3 * id[l] + 1]; Z[l] = u[3 * id[l] + 2]; }
+    T a = T(F.h), b = a, c = a, ia = T(1.0 / F.h), ib = ia, ic = ia;
+    if constexpr (!CUBE) {
+      const int i = cell % F.nx, j = (cell / F.nx) % F.ny, k = cell / (F.nx * F.ny);
+      a = F.dx[i]; b = F.dy[j]; c = F.dz[k];
+      ia = F.idx[i]; ib = F.idy[j]; ic = F.idz[k];
+    }
+    butterfly_fwd(X);
+    butterfly_fwd(Y);
+    butterfly_fwd(Z);
+    hex8_modal<T, MODE != MAT_ISO_SRI>(X, Y, Z, make_coef(a, b, c, ia, ib, ic, make_material<T, MODE>(m)), FX, FY, FZ);
+    const T sx = (q & 1) ? T(1) : T(-1), sy = (q & 2) ? T(1) : T(-1), sz = (q & 4) ? T(1) : T(-1);
+    auto at_corner = [&](const T (&f)[8]) {
+      T g[4];
+#pragma unroll
+      for (int l = 0; l < 4; ++l) g[l] = f[2 * l] + sx * f[2 * l + 1];
+      return (g[0] + sy * g[1]) + sz * (g[2] + sy * g[3]);
+    };
+    t[0] += at_corner(FX);
+    t[1] += at_corner(FY);
+    t[2] += at_corner(FZ);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int e = 1; e < 8; e <<= 1) t[c] += __shfl_xor_sync(0xffffffffu, t[c], e);
+  if (!live || q != 0) return;
+  if constexpr (SMOOTH) {
+    node_update(S, a1, a2, n, t, o);
+  } else {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) y[3 * n + c] = t[c];
+  }
+}
+
 template <typename T, int MODE, bool CUBE, int WY>
 constexpr size_t pair_smem_bytes() {
   return 4 * sizeof(V2<T>) * 3 * WY * 32 + sizeof(T) * kMaxMatIds * (CUBE ? 2 : MatWidth<MODE>::value);
@@ -203,12 +299,13 @@ constexpr size_t pair_smem_bytes() {
 template <typename T, int MODE, bool CUBE, int WY, bool SMOOTH>
 __global__ void __launch_bounds__(32 * WY, FEB_PAIR_MINB)
 k_fine_pair(PairView<T> F, const T* __restrict__ u, T* __restrict__ y, SmoothArgs<T> S, const int* __restrict__ skip,
-            int zchunk, int nbx, int nby, int nbz) {
+            int zchunk, int nbx, int nby) {
   if (skip && *skip) return;
   constexpr int W = MatWidth<MODE>::value;
   constexpr bool HAS12 = (MODE != MAT_ISO_SRI);
   constexpr int OY = 2 * WY - 2;
   constexpr int MW = CUBE ? 2 : W;
+  constexpr int kRowGroups = 4 * WY;
   // FP32 smoothing loads the epilogue operands one step ahead; FP64 (no register room) loads them in finish()
   constexpr bool PREF = SMOOTH && std::is_same<T, float>::value;
   using V = P2<T>;
@@ -220,29 +317,7 @@ k_fine_pair(PairView<T> F, const T* __restrict__ u, T* __restrict__ y, SmoothArg
   T (*sMat)[MW] = reinterpret_cast<T (*)[MW]>(smem_raw + 4 * sizeof(V2<T>) * 3 * WY * 32);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   T a1 = T(0), a2 = T(0);
-  if constexpr (SMOOTH) {   // the Chebyshev coefficients (a residual-only step carries no parameters)
-    if (S.lp && S.updates()) {
-      a1 = S.k < 0 ? T(0) : T(S.lp->a1[S.k]);
-      a2 = S.k < 0 ? T(S.lp->c_init) : T(S.lp->a2[S.k]);
-    }
-  }
-  const int64_t ntiles = (int64_t)nbx * nby * nbz;
-  if (blockIdx.x >= ntiles) {   // split copies: finished from the sparse accumulator alone
-    const int64_t n = F.nnode + (int64_t)(blockIdx.x - ntiles) * (32 * WY) + threadIdx.x;
-    if (n >= F.ntotal) return;
-    T t[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) { t[c] = F.tsp[3 * n + c]; F.tsp[3 * n + c] = T(0); }
-    if constexpr (SMOOTH) {
-      NodeOps<T> o;
-      load_node_ops(F, S, u, a1 != T(0), (int)n, o);
-      node_update(S, a1, a2, (int)n, t, o);
-    } else {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) y[3 * n + c] = t[c];
-    }
-    return;
-  }
+  if constexpr (SMOOTH) pair_coef(S, a1, a2);
   for (int q = threadIdx.x; q < kMaxMatIds; q += blockDim.x) {
     if constexpr (CUBE) {
       sMat[q][0] = q < F.nmat ? T(F.mtab[W * q] * F.h / 16.0) : T(0);
@@ -252,7 +327,7 @@ k_fine_pair(PairView<T> F, const T* __restrict__ u, T* __restrict__ y, SmoothArg
       for (int p = 0; p < W; ++p) sMat[q][p] = q < F.nmat ? T(F.mtab[W * q + p]) : T(0);
     }
   }
-  const int bx = int(blockIdx.x % nbx), by = int((blockIdx.x / nbx) % nby), bz = int(blockIdx.x / ((int64_t)nbx * nby));
+  const int bx = blockIdx.x % nbx, by = (blockIdx.x / nbx) % nby, bz = blockIdx.x / (nbx * nby);
   const int i = bx * kXOwn - 1 + lane;
   const int r0 = by * OY - 1 + 2 * w, r1 = r0 + 1;
   const int m = by * (OY / 2) + w;    // row pair (2m-1, 2m) of the cell-pair words
@@ -336,27 +411,30 @@ k_fine_pair(PairView<T> F, const T* __restrict__ u, T* __restrict__ y, SmoothArg
     if (kk < K0 || kk >= K1) return;
     const int n0 = n0base + plane * kk, n1 = n1base + plane * kk;
     T t0[3] = {out[0].lo(), out[1].lo(), out[2].lo()}, t1[3] = {out[0].hi(), out[1].hi(), out[2].hi()};
+    bool f0 = own0, f1 = own1;   // the node is finished here
     if (own0 && (flags & 0x80u)) {
+      f0 = !F.rowflag[n0];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) { t0[c] += F.tsp[3 * n0 + c]; F.tsp[3 * n0 + c] = T(0); }
+      for (int c = 0; c < 3; ++c) t0[c] += F.kd[3 * n0 + c] * u[3 * n0 + c];
     }
     if (own1 && (flags & 0x8000u)) {
+      f1 = !F.rowflag[n1];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) { t1[c] += F.tsp[3 * n1 + c]; F.tsp[3 * n1 + c] = T(0); }
+      for (int c = 0; c < 3; ++c) t1[c] += F.kd[3 * n1 + c] * u[3 * n1 + c];
     }
     if constexpr (PREF) {
-      if (own0) node_update(S, a1, a2, n0, t0, o0);
-      if (own1) node_update(S, a1, a2, n1, t1, o1);
+      if (f0) node_update(S, a1, a2, n0, t0, o0);
+      if (f1) node_update(S, a1, a2, n1, t1, o1);
     } else if constexpr (SMOOTH) {
       NodeOps<T> o;
-      if (own0) { load_node_ops(F, S, u, need_dir, n0, o); node_update(S, a1, a2, n0, t0, o); }
-      if (own1) { load_node_ops(F, S, u, need_dir, n1, o); node_update(S, a1, a2, n1, t1, o); }
+      if (f0) { load_node_ops(F, S, u, need_dir, n0, o); node_update(S, a1, a2, n0, t0, o); }
+      if (f1) { load_node_ops(F, S, u, need_dir, n1, o); node_update(S, a1, a2, n1, t1, o); }
     } else {
-      if (own0) {
+      if (f0) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) y[3 * n0 + c] = t0[c];
       }
-      if (own1) {
+      if (f1) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) y[3 * n1 + c] = t1[c];
       }
@@ -378,12 +456,14 @@ k_fine_pair(PairView<T> F, const T* __restrict__ u, T* __restrict__ y, SmoothArg
       }
     }
   };
-  {   // prologue: face of plane K0-1
+  {   // prologue: face of plane K0-1; the CTA's share of the row list while its planes are on their way
     V v0[3], E[3][2];
     load_plane(K0 - 1, v0);
     load_plane(K0, va);
     load_plane(K0 + 1, vb);
     ca = load_cells(K0 - 1);
+    for (int row0 = blockIdx.x * kRowGroups; row0 < F.rows.n; row0 += gridDim.x * kRowGroups)
+      finish_row<T, MODE, CUBE, SMOOTH>(F, u, y, S, a1, a2, row0 + (int)(threadIdx.x >> 3));
     edge(v0, E);
     put_edge(slot(K0 - 1), E);
     __syncthreads();
@@ -500,11 +580,11 @@ int launch_pair_kernel(const PairView<T>& F, const T* u, T* y, const SmoothArgs<
                        cudaStream_t s) {
   constexpr int OY = 2 * WY - 2;
   const int nbx = div_up(F.nxn, kXOwn), nby = div_up(F.nyn, OY), nbz = div_up(F.nzn, zc);
-  const int64_t blocks = (int64_t)nbx * nby * nbz + div_up(F.ntotal - F.nnode, 32 * WY);
+  const int64_t blocks = (int64_t)nbx * nby * nbz;
   constexpr size_t smem = pair_smem_bytes<T, MODE, CUBE, WY>();
   auto kern = k_fine_pair<T, MODE, CUBE, WY, SMOOTH>;
   FEB_TRY(set_dyn_smem((const void*)kern, (int)smem));
-  kern<<<(unsigned)blocks, 32 * WY, smem, s>>>(F, u, y, A, skip, zc, nbx, nby, nbz);
+  kern<<<(unsigned)blocks, 32 * WY, smem, s>>>(F, u, y, A, skip, zc, nbx, nby);
   note_launch();
   return FEB_OK;
 }
@@ -592,6 +672,64 @@ __global__ void k_mat_ids(const double* __restrict__ mat_s, int64_t ncell, unsig
   atomicOr(status, 1);
 }
 
+// Row flags: nodes of the row list (corners of irregular cells, nodes of extra entries, split copies); cmap:
+// the irregular cell of every cell (-1 elsewhere, preset); start: first CSR row of a node's extra entries (-1, preset).
+__global__ void k_row_flags(const int* __restrict__ irr_cell, const int* __restrict__ irr_nodes, int nirr,
+                            const int* __restrict__ row_dof, int nrow, int64_t nnode, int64_t ntotal,
+                            uint8_t* __restrict__ flag, int* __restrict__ cmap, int* __restrict__ start) {
+  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (e < nirr) cmap[irr_cell[e]] = (int)e;
+  if (e < 8 * (int64_t)nirr) flag[irr_nodes[e]] = 1;
+  if (e < nrow) {
+    const int n = row_dof[e] / 3;
+    flag[n] = 1;
+    if (e == 0 || row_dof[e - 1] / 3 != n) start[n] = (int)e;
+  }
+  if (e < ntotal - nnode) flag[nnode + e] = 1;
+}
+
+// diagonal of the penalty springs, 3 per node (several springs on a node add up)
+__global__ void k_pen_diag(const int* __restrict__ node, const double* __restrict__ k, int n, double* __restrict__ kd) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= n) return;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) atomicAdd(kd + 3 * (int64_t)node[e] + c, k[3 * e + c]);
+}
+
+// Row list: per row node n and corner q the code of the cell of which n is corner q (a regular cell's corners are grid nodes),
+// and the bounds of the extra entries of the node's dofs (consecutive CSR rows, some may be missing).
+__global__ void k_rows(FineView<double> F, const int* __restrict__ node, int nrow, const int* __restrict__ orig_copy,
+                       const int* __restrict__ cmap, const int* __restrict__ start, const uint8_t* __restrict__ ids,
+                       int* __restrict__ cell, int4* __restrict__ ex) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int row = t >> 3, q = t & 7;
+  if (row >= nrow) return;
+  const int n = node[row];
+  const int g = n < F.nnode ? n : orig_copy[n - F.nnode];
+  const int i = g % F.nxn - (q & 1), j = (g / F.nxn) % F.nyn - ((q >> 1) & 1), k = g / (F.nxn * F.nyn) - (q >> 2);
+  int code = kNoCell;
+  if (i >= 0 && j >= 0 && k >= 0 && i < F.nx && j < F.ny && k < F.nz) {
+    const int64_t c = i + (int64_t)F.nx * (j + (int64_t)F.ny * k);
+    const int e = cmap[c];
+    if (e >= 0) { if (F.irr_nodes[8 * (int64_t)e + q] == n) code = e; }
+    else if (ids[c] && n < F.nnode) code = kRegularCell - (int)ids[c];
+  }
+  cell[8 * row + q] = code;
+  if (q) return;
+  int4 x = make_int4(0, 0, 0, 0);
+  int e = start[n];
+  if (e >= 0) {
+    int p[4];
+    p[0] = F.row_ptr[e];
+    for (int c = 0; c < 3; ++c) {
+      if (e < F.nrow && F.row_dof[e] == 3 * n + c) { p[c + 1] = F.row_ptr[e + 1]; ++e; }
+      else p[c + 1] = p[c];
+    }
+    x = make_int4(p[0], p[1], p[2], p[3]);
+  }
+  ex[row] = x;
+}
+
 // node flags: grid nodes that receive a sparse contribution (penalty, extra entry, irregular cell corner)
 __global__ void k_flag_nodes(const int* __restrict__ pen_node, int npen, const int* __restrict__ irr_nodes, int nirr,
                              const int* __restrict__ row_dof, int nrow, int64_t nnode, uint8_t* __restrict__ flag) {
@@ -665,9 +803,8 @@ __global__ void k_cheb_first6(const T* __restrict__ b, const T* __restrict__ D, 
 }  // namespace
 
 template <typename T, int MODE>
-int launch_fine_pair(const PairView<T>& F, const FineView<T>& G, const T* u, T* y, const SmoothArgs<T>* S,
-                     const int* skip, PairConfig cfg, cudaStream_t s) {
-  if (G.nirr + G.npen + G.nrow > 0) launch_fine_sparse_into<T, MODE>(G, u, F.tsp, skip, s);
+int launch_fine_pair(const PairView<T>& F, const T* u, T* y, const SmoothArgs<T>* S, const int* skip, PairConfig cfg,
+                     cudaStream_t s) {
   if (S) return launch_pair_wy<T, MODE, true>(F, u, y, *S, skip, cfg, s);
   return launch_pair_wy<T, MODE, false>(F, u, y, SmoothArgs<T>{}, skip, cfg, s);
 }
@@ -738,6 +875,22 @@ void launch_pack_pairs(int nx, int ny, int nz, int mp, const uint8_t* ids, const
   k_pack_pairs<W><<<div_up(total, kThreads), kThreads, 0, s>>>(nx, ny, nz, mp, ids, flag, mat_s, vals, cellpair, status);
   note_launch();
 }
+void launch_row_flags(const FineView<double>& F, uint8_t* flag, int* cmap, int* start, cudaStream_t s) {
+  const int64_t n = std::max<int64_t>(std::max<int64_t>(8 * (int64_t)F.nirr, F.nrow), F.ntotal - F.nnode);
+  if (n > 0) {
+    k_row_flags<<<div_up(n, kThreads), kThreads, 0, s>>>(F.irr_cell, F.irr_nodes, F.nirr, F.row_dof, F.nrow, F.nnode, F.ntotal,
+                                                         flag, cmap, start);
+    note_launch();
+  }
+}
+void launch_pen_diag(const int* node, const double* k, int n, double* kd, cudaStream_t s) {
+  if (n > 0) { k_pen_diag<<<div_up(n, kThreads), kThreads, 0, s>>>(node, k, n, kd); note_launch(); }
+}
+void launch_rows(const FineView<double>& F, const int* node, int nrow, const int* orig_copy, const int* cmap, const int* start,
+                 const uint8_t* ids, int* cell, int4* ex, cudaStream_t s) {
+  k_rows<<<div_up(8 * (int64_t)nrow, kThreads), kThreads, 0, s>>>(F, node, nrow, orig_copy, cmap, start, ids, cell, ex);
+  note_launch();
+}
 template <typename T>
 void launch_dinv6(const double* D9, int64_t n, T* out, cudaStream_t s) {
   k_dinv6<T><<<div_up(n, kThreads), kThreads, 0, s>>>(D9, n, out); note_launch();
@@ -749,8 +902,8 @@ void launch_cheb_first6(const T* b, const T* D6, const LevelParams* lp, T* d, T*
 }
 
 #define INST(T, M)                                                                                          \
-  template int launch_fine_pair<T, M>(const PairView<T>&, const FineView<T>&, const T*, T*, const SmoothArgs<T>*, \
-                                      const int*, PairConfig, cudaStream_t);
+  template int launch_fine_pair<T, M>(const PairView<T>&, const T*, T*, const SmoothArgs<T>*, const int*, PairConfig, \
+                                      cudaStream_t);
 INST(float, MAT_ISO_SRI) INST(float, MAT_ISO_FULL) INST(float, MAT_ORTHO)
 INST(double, MAT_ISO_SRI) INST(double, MAT_ISO_FULL) INST(double, MAT_ORTHO)
 #undef INST

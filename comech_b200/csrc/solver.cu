@@ -1037,13 +1037,6 @@ struct FebHandle {
     return coarse_fail ? coarse_error() : FEB_OK;
   }
 
-  // the level-0 products share their sparse-part accumulators with the level-0 power iteration: a product on
-  // s waits (on the device) for that chain while it may still run
-  int wait_fine() {
-    if (pending && coarsest > 0) FEB_CUDA(cudaStreamWaitEvent(s, aux_ev[0], 0));
-    return FEB_OK;
-  }
-
   // the rigid-mode coefficients' stream (set with the rigid groups) and its fork / join events
   cudaStream_t rs = nullptr;
   cudaEvent_t rs_fork = nullptr, rs_join = nullptr;
@@ -1088,9 +1081,9 @@ struct FebHandle {
   template <typename T>
   void pair_run(const T* u, T* y, const SmoothArgs<T>* S, const int* skip) {
     switch (mode) {
-      case MAT_ISO_SRI: launch_fine_pair<T, MAT_ISO_SRI>(pview<T>(), fine<T>(), u, y, S, skip, pcfg<T>(), s); break;
-      case MAT_ISO_FULL: launch_fine_pair<T, MAT_ISO_FULL>(pview<T>(), fine<T>(), u, y, S, skip, pcfg<T>(), s); break;
-      default: launch_fine_pair<T, MAT_ORTHO>(pview<T>(), fine<T>(), u, y, S, skip, pcfg<T>(), s); break;
+      case MAT_ISO_SRI: launch_fine_pair<T, MAT_ISO_SRI>(pview<T>(), u, y, S, skip, pcfg<T>(), s); break;
+      case MAT_ISO_FULL: launch_fine_pair<T, MAT_ISO_FULL>(pview<T>(), u, y, S, skip, pcfg<T>(), s); break;
+      default: launch_fine_pair<T, MAT_ORTHO>(pview<T>(), u, y, S, skip, pcfg<T>(), s); break;
     }
   }
 
@@ -1842,6 +1835,61 @@ int autotune_ku(FebHandle* h) {
 // bit c of l.  Read off the device element operator for the unit cube, checked to be those integers, laid
 // out as the kernel's B table: [face cz][node row b][output n][4a + c] in BF16 (exact).  Leaves tc_ok false
 // for other grids or models.
+// Row list of the paired-row operator (ids: material id of every regular cell) and its penalty diagonal.
+int setup_rows(FebHandle* h, const uint8_t* ids) {
+  FebHandle& H = *h;
+  const FineView<double>& F = H.F64;
+  const int64_t ncell = (int64_t)H.nx * H.ny * H.nz;
+  const size_t n3 = 3 * (size_t)H.ntotal;
+  uint8_t* flag = nullptr;
+  double* kd64 = nullptr;
+  float* kd32 = nullptr;
+  int *cmap = nullptr, *start = nullptr;
+  FEB_TRY(H.pool.zeros(&flag, H.ntotal));
+  FEB_TRY(H.pool.zeros(&kd64, n3));
+  FEB_TRY(H.pool.alloc(&kd32, n3));
+  FEB_TRY(H.pool.alloc(&cmap, ncell));
+  FEB_TRY(H.pool.alloc(&start, H.ntotal));
+  FEB_CUDA(cudaMemsetAsync(cmap, 0xff, ncell * sizeof(int), H.s));
+  FEB_CUDA(cudaMemsetAsync(start, 0xff, H.ntotal * sizeof(int), H.s));
+  launch_row_flags(F, flag, cmap, start, H.s);
+  launch_pen_diag(F.pen_node, F.pen_k, F.npen, kd64, H.s);
+  launch_convert<double, float>(kd64, kd32, (int64_t)n3, nullptr, H.s);
+  FEB_CUDA(cudaGetLastError());
+  H.P64.kd = kd64; H.P32.kd = kd32;
+  H.P64.rowflag = H.P32.rowflag = flag;
+  H.P64.rows = PairRows<double>{};
+  H.P32.rows = PairRows<float>{};
+  // room for every node that may be flagged
+  const int64_t cap = std::min<int64_t>(H.ntotal, 8 * (int64_t)F.nirr + F.nrow + (H.ntotal - H.nnode));
+  if (cap > 0) {
+    int *node = nullptr, *cnt = nullptr, *cell = nullptr;
+    int4* ex = nullptr;
+    uint8_t* tmp = nullptr;
+    size_t tb = 0;
+    thrust::counting_iterator<int> it(0);
+    FEB_TRY(H.pool.alloc(&node, cap));
+    FEB_TRY(H.pool.alloc(&cnt, 1));
+    FEB_CUDA(cub::DeviceSelect::Flagged(nullptr, tb, it, flag, node, cnt, (int)H.ntotal, H.s));
+    FEB_TRY(H.pool.alloc(&tmp, tb));
+    FEB_CUDA(cub::DeviceSelect::Flagged(tmp, tb, it, flag, node, cnt, (int)H.ntotal, H.s));
+    int n = 0;
+    FEB_CUDA(cudaMemcpyAsync(&n, cnt, sizeof(int), cudaMemcpyDeviceToHost, H.s));
+    FEB_CUDA(cudaStreamSynchronize(H.s));
+    FEB_TRY(H.pool.alloc(&cell, 8 * (size_t)n));
+    FEB_TRY(H.pool.alloc(&ex, n));
+    launch_rows(F, node, n, H.orig_copy, cmap, start, ids, cell, ex, H.s);
+    FEB_CUDA(cudaGetLastError());
+    H.P64.rows = PairRows<double>{n, node, cell, F.irr_cell, F.irr_nodes, F.irr_mat, ex, F.col, F.val};
+    H.P32.rows = PairRows<float>{n, node, cell, F.irr_cell, F.irr_nodes, H.F32.irr_mat, ex, H.F32.col, H.F32.val};
+    H.pool.free(tmp);
+    H.pool.free(cnt);
+  }
+  H.pool.free(cmap);
+  H.pool.free(start);
+  return FEB_OK;
+}
+
 // Paired-row level-0 operator (fine_pair.cu): material ids of the regular cells (FEB_KU_PAIR=0 keeps the
 // per-cell kernels), flags of the grid nodes that receive sparse contributions, the cell-pair words, the
 // sparse accumulators and the symmetric level-0 block-Jacobi inverse.  Leaves pair_ok false when more than
@@ -1873,20 +1921,17 @@ int setup_pair(FebHandle* h, const double* mat_s64) {
   int st = 0;
   FEB_CUDA(cudaMemcpyAsync(&st, status, sizeof(int), cudaMemcpyDeviceToHost, H.s));
   FEB_CUDA(cudaStreamSynchronize(H.s));
-  H.pool.free(ids);
   H.pool.free(flag);
   H.pool.free(keys);
   H.pool.free(status);
   if (st != 0) {
+    H.pool.free(ids);
     H.pool.free(cellpair);
     H.pool.free(vals);
     return FEB_OK;
   }
-  const size_t n3 = 3 * (size_t)H.ntotal;
-  float* tsp32 = nullptr;
-  double* tsp64 = nullptr;
-  FEB_TRY(H.pool.zeros(&tsp32, n3));
-  FEB_TRY(H.pool.zeros(&tsp64, n3));
+  FEB_TRY(setup_rows(h, ids));
+  H.pool.free(ids);
   FEB_TRY(H.pool.alloc(&H.D6_32, 6 * (size_t)H.ntotal));
   FEB_TRY(H.pool.alloc(&H.D6_64, 6 * (size_t)H.ntotal));
   launch_dinv6<float>(H.L[0].Dinv64, H.ntotal, H.D6_32, H.s);
@@ -1899,16 +1944,16 @@ int setup_pair(FebHandle* h, const double* mat_s64) {
     return true;
   };
   const bool cube = H.mode == MAT_ISO_SRI && hc > 0.0 && uniform(H.xe) && uniform(H.ye) && uniform(H.ze);
-  auto fill = [&](auto& P, const auto& F, auto* tsp, const auto* d6) {
+  auto fill = [&](auto& P, const auto& F, const auto* d6) {
     P.nx = H.nx; P.ny = H.ny; P.nz = H.nz; P.nxn = nxn; P.nyn = nyn; P.nzn = nzn; P.mp = mp;
     P.nnode = H.nnode; P.ntotal = H.ntotal;
     P.cellpair = cellpair; P.mtab = vals; P.nmat = kMaxMatIds;
     P.cube = cube; P.h = hc;
     P.dx = F.dx; P.dy = F.dy; P.dz = F.dz; P.idx = F.idx; P.idy = F.idy; P.idz = F.idz;
-    P.tsp = tsp; P.dinv6 = d6;
+    P.dinv6 = d6;
   };
-  fill(H.P32, H.F32, tsp32, H.D6_32);
-  fill(H.P64, H.F64, tsp64, H.D6_64);
+  fill(H.P32, H.F32, H.D6_32);
+  fill(H.P64, H.F64, H.D6_64);
   FEB_TRY(prepare_fine_pair(H.mode, cube));
   H.pc32 = PairConfig{cube ? 16 : 8, 16};
   H.pc64 = PairConfig{8, 16};
@@ -2896,7 +2941,6 @@ int feb_set_rigid_groups(FebHandle* h, int32_t ngroups, const int64_t* offsets, 
   FEB_TRY(H.pool.alloc(&col, 3 * (size_t)H.ntotal));
   FEB_TRY(H.pool.alloc(&kcol, 3 * (size_t)H.ntotal));
   FEB_TRY(H.pool.alloc(&Ecd, (size_t)nc * nc));
-  FEB_TRY(H.wait_fine());
   if (!H.rs) {
     H.rs = g_streams.stream();
     if (!H.rs_fork) H.rs_fork = g_streams.event();
@@ -3140,7 +3184,6 @@ int feb_solve_batch(FebHandle* const* hs, int32_t n, const double* const* f, con
 int feb_apply(FebHandle* h, int32_t prec, const void* u, void* y) {
   if (!h || !u || !y) { set_last_error("feb_apply: null argument"); return FEB_ERR_ARG; }
   FEB_TRY(h->sync_in());
-  FEB_TRY(h->wait_fine());
   if (prec == 0) h->apply<double>(0, (const double*)u, (double*)y, nullptr);
   else h->apply<float>(0, (const float*)u, (float*)y, nullptr);
   FEB_CUDA(cudaGetLastError());
