@@ -91,7 +91,9 @@ template <typename T>
 struct SmoothArgs {
   const T* r_in = nullptr;
   T* r_out = nullptr;
-  const T* x_in = nullptr;
+  const T* x_in = nullptr;     // the iterate x_out = x_in (+ x_add) (+ d if x_lag) + d': directions that earlier steps left out
+  const T* x_add = nullptr;
+  bool x_lag = false;
   T* x_out = nullptr;
   T* d_out = nullptr;
   double* x_out64 = nullptr;   // the new iterate in FP64 (instead of, or besides, x_out): the V-cycle's result
@@ -104,9 +106,10 @@ struct PairConfig {
   int wy = 16;            // warps per CTA of products (2 node rows each); 16 only on the cubic SRI path in FP32
   int zchunk = 16;        // node planes per CTA of products
   int zchunk_smooth = 16; // node planes per CTA of the smoothing steps (always 8 warps per CTA)
+  bool split = false;     // smoothing steps in two launches: product (its shape), update of all nodes
 };
 
-// y = K u (S null) or the smoother step S; returns a status
+// y = K u (S null), the residual or the smoother step S; y takes K u of a step split in two launches (null: not split)
 template <typename T, int MODE>
 int launch_fine_pair(const PairView<T>& F, const T* u, T* y, const SmoothArgs<T>* S, const int* skip, PairConfig cfg,
                      cudaStream_t s);

@@ -3,7 +3,7 @@
 // Work split of one launch (a product y = K u, or one Chebyshev / residual step of the smoother):
 //   * tile CTAs compute the regular cells matrix-free.  A grid node whose 8 cells are all handled here (the bulk) is
 //     finished in registers: its product is stored, or the smoother update of that node runs on the spot (r -= K d,
-//     z = Dinv r, d' = a1 d + a2 z, x += d').  A node flagged "special" with a penalty spring adds its diagonal first; one
+//     z = Dinv r, d' = a1 d + a2 z, x += d').  On large grids the update is a launch of its own (k_pair_update).  A node flagged "special" with a penalty spring adds its diagonal first; one
 //     that cells touching split copies or extra entries reach is left out (its row flag is set).
 //   * those nodes and the split copies (PairRows) are finished by groups of eight lanes, one cell each, spread over all
 //     CTAs: each does its few while its first planes are on their way.  There are not many (1 % of the nodes of a
@@ -34,9 +34,6 @@ namespace {
 constexpr int kXOwn = 30;
 // cell codes of the row list: an irregular cell's index, a regular cell's material id as kRegularCell - id, or none
 constexpr int kNoCell = -1, kRegularCell = -1;
-#ifndef FEB_PAIR_MINB
-#define FEB_PAIR_MINB 1
-#endif
 #ifndef FEB_PAIR_UNROLL
 #define FEB_PAIR_UNROLL 1
 #endif
@@ -143,41 +140,42 @@ __device__ __forceinline__ void pair_modal(P2<T> (&X)[8], P2<T> (&Y)[8], P2<T> (
     }
 }
 
-// Operands of the smoother update at one node, loaded a step before they are used: residual before the
-// product, iterate, direction (the product's input) and the symmetric block-Jacobi inverse.
+// What a launch does with t = K u at a node: store it, r_out = r_in - t, or the smoother update
+enum : int { kProduct = 0, kResidual = 1, kStep = 2 };
+
+// Operands of the smoother update at one node, loaded a step before they are used: residual before the product, direction (the
+// product's input), symmetric block-Jacobi inverse, and the parts of the iterate.
 template <typename T>
 struct NodeOps {
-  T r[3], x[3], d[3], D[6];
+  T r[3], x[3], xa[3], d[3], D[6];
 };
 
+// all but the residual
 template <typename T>
-__device__ __forceinline__ void load_node_ops(const PairView<T>& F, const SmoothArgs<T>& S, const T* __restrict__ u,
+__device__ __forceinline__ void load_step_ops(const PairView<T>& F, const SmoothArgs<T>& S, const T* __restrict__ u,
                                               bool need_dir, int n, NodeOps<T>& o) {
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    o.r[c] = S.r_in[3 * n + c];
     o.x[c] = S.x_in ? S.x_in[3 * n + c] : T(0);
+    o.xa[c] = S.x_add ? S.x_add[3 * n + c] : T(0);
     o.d[c] = need_dir ? u[3 * n + c] : T(0);
   }
-  if (S.updates()) {
-    const T* D = F.dinv6 + n;
+  const T* D = F.dinv6 + n;
 #pragma unroll
-    for (int q = 0; q < 6; ++q) o.D[q] = D[(size_t)q * F.ntotal];
-  }
+  for (int q = 0; q < 6; ++q) o.D[q] = D[(size_t)q * F.ntotal];
 }
 
-// smoother update of one node from t = K u at the node and its operands
+template <typename T, int EPI>
+__device__ __forceinline__ void load_node_ops(const PairView<T>& F, const SmoothArgs<T>& S, const T* __restrict__ u,
+                                              bool need_dir, int n, NodeOps<T>& o) {
+#pragma unroll
+  for (int c = 0; c < 3; ++c) o.r[c] = S.r_in[3 * n + c];
+  if constexpr (EPI == kStep) load_step_ops(F, S, u, need_dir, n, o);
+}
+
+// direction and iterate of one node from its new residual
 template <typename T>
-__device__ __forceinline__ void node_update(const SmoothArgs<T>& S, T a1, T a2, int n, const T (&t)[3],
-                                            const NodeOps<T>& o) {
-  T r[3];
-#pragma unroll
-  for (int c = 0; c < 3; ++c) r[c] = o.r[c] - t[c];
-  if (S.r_out) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) S.r_out[3 * n + c] = r[c];
-  }
-  if (!S.updates()) return;
+__device__ __forceinline__ void node_step(const SmoothArgs<T>& S, T a1, T a2, int n, const T (&r)[3], const NodeOps<T>& o) {
   T z[3];
   z[0] = o.D[0] * r[0] + o.D[3] * r[1] + o.D[4] * r[2];
   z[1] = o.D[3] * r[0] + o.D[1] * r[1] + o.D[5] * r[2];
@@ -189,20 +187,35 @@ __device__ __forceinline__ void node_update(const SmoothArgs<T>& S, T a1, T a2, 
 #pragma unroll
     for (int c = 0; c < 3; ++c) S.d_out[3 * n + c] = dn[c];
   }
-  if (S.x_out) {
+  if (!S.x_out && !S.x_out64) return;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) S.x_out[3 * n + c] = o.x[c] + dn[c];
-  }
-  if (S.x_out64) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) S.x_out64[3 * n + c] = double(o.x[c] + dn[c]);
+  for (int c = 0; c < 3; ++c) {
+    T x = o.x[c];
+    if (S.x_add) x += o.xa[c];
+    if (S.x_lag) x += o.d[c];
+    x += dn[c];
+    if (S.x_out) S.x_out[3 * n + c] = x;
+    if (S.x_out64) S.x_out64[3 * n + c] = double(x);
   }
 }
 
-// the Chebyshev coefficients of the step (a residual-only step carries no parameters)
+// update of one node from t = K u at the node and its operands
+template <typename T, int EPI>
+__device__ __forceinline__ void node_update(const SmoothArgs<T>& S, T a1, T a2, int n, const T (&t)[3], const NodeOps<T>& o) {
+  T r[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) r[c] = o.r[c] - t[c];
+  if (EPI == kResidual || S.r_out) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) S.r_out[3 * n + c] = r[c];
+  }
+  if constexpr (EPI == kStep) node_step(S, a1, a2, n, r, o);
+}
+
+// the Chebyshev coefficients of the step
 template <typename T>
 __device__ __forceinline__ void pair_coef(const SmoothArgs<T>& S, T& a1, T& a2) {
-  if (S.lp && S.updates()) {
+  if (S.lp) {
     a1 = S.k < 0 ? T(0) : T(S.lp->a1[S.k]);
     a2 = S.k < 0 ? T(S.lp->c_init) : T(S.lp->a2[S.k]);
   }
@@ -211,7 +224,7 @@ __device__ __forceinline__ void pair_coef(const SmoothArgs<T>& S, T& a1, T& a2) 
 // One node of the row list by a group of eight lanes, one cell each: the cell's force at its corner by the element operator
 // (the modal form of the tiles, back-transformed for that corner alone), summed over the group with the node's penalties
 // and extra entries.  Rows past the end: the group idles along.
-template <typename T, int MODE, bool CUBE, bool SMOOTH>
+template <typename T, int MODE, bool CUBE, int EPI>
 __device__ __forceinline__ void finish_row(const PairView<T>& F, const T* __restrict__ u, T* __restrict__ y,
                                            const SmoothArgs<T>& S, T a1, T a2, int row) {
   constexpr int W = MatWidth<MODE>::value;
@@ -221,8 +234,8 @@ __device__ __forceinline__ void finish_row(const PairView<T>& F, const T* __rest
   const int n = R.node[rc], code = R.cell[8 * rc + q];
   const int4 ex = R.ex[rc];
   NodeOps<T> o;
-  if constexpr (SMOOTH) {
-    if (live && q == 0) load_node_ops(F, S, u, a1 != T(0), n, o);
+  if constexpr (EPI != kProduct) {
+    if (live && q == 0) load_node_ops<T, EPI>(F, S, u, a1 != T(0) || S.x_lag, n, o);
   }
   T t[3] = {T(0), T(0), T(0)};
   if (q < 3) t[q == 2 ? 2 : q] = F.kd[3 * n + q] * u[3 * n + q];
@@ -283,8 +296,8 @@ __device__ __forceinline__ void finish_row(const PairView<T>& F, const T* __rest
 #pragma unroll
     for (int e = 1; e < 8; e <<= 1) t[c] += __shfl_xor_sync(0xffffffffu, t[c], e);
   if (!live || q != 0) return;
-  if constexpr (SMOOTH) {
-    node_update(S, a1, a2, n, t, o);
+  if constexpr (EPI != kProduct) {
+    node_update<T, EPI>(S, a1, a2, n, t, o);
   } else {
 #pragma unroll
     for (int c = 0; c < 3; ++c) y[3 * n + c] = t[c];
@@ -296,8 +309,8 @@ constexpr size_t pair_smem_bytes() {
   return 4 * sizeof(V2<T>) * 3 * WY * 32 + sizeof(T) * kMaxMatIds * (CUBE ? 2 : MatWidth<MODE>::value);
 }
 
-template <typename T, int MODE, bool CUBE, int WY, bool SMOOTH>
-__global__ void __launch_bounds__(32 * WY, FEB_PAIR_MINB)
+template <typename T, int MODE, bool CUBE, int WY, int EPI>
+__global__ void __launch_bounds__(32 * WY, 1)
 k_fine_pair(PairView<T> F, const T* __restrict__ u, T* __restrict__ y, SmoothArgs<T> S, const int* __restrict__ skip,
             int zchunk, int nbx, int nby) {
   if (skip && *skip) return;
@@ -306,8 +319,8 @@ k_fine_pair(PairView<T> F, const T* __restrict__ u, T* __restrict__ y, SmoothArg
   constexpr int OY = 2 * WY - 2;
   constexpr int MW = CUBE ? 2 : W;
   constexpr int kRowGroups = 4 * WY;
-  // FP32 smoothing loads the epilogue operands one step ahead; FP64 (no register room) loads them in finish()
-  constexpr bool PREF = SMOOTH && std::is_same<T, float>::value;
+  // FP32 loads the epilogue operands one step ahead; FP64 (no register room) loads them in finish()
+  constexpr bool PREF = EPI != kProduct && std::is_same<T, float>::value;
   using V = P2<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   // forward: (sum, diff) x-edge of the lower row per component; backward: (mean, diff) x-edge force of the
@@ -317,7 +330,7 @@ k_fine_pair(PairView<T> F, const T* __restrict__ u, T* __restrict__ y, SmoothArg
   T (*sMat)[MW] = reinterpret_cast<T (*)[MW]>(smem_raw + 4 * sizeof(V2<T>) * 3 * WY * 32);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   T a1 = T(0), a2 = T(0);
-  if constexpr (SMOOTH) pair_coef(S, a1, a2);
+  if constexpr (EPI == kStep) pair_coef(S, a1, a2);
   for (int q = threadIdx.x; q < kMaxMatIds; q += blockDim.x) {
     if constexpr (CUBE) {
       sMat[q][0] = q < F.nmat ? T(F.mtab[W * q] * F.h / 16.0) : T(0);
@@ -342,7 +355,7 @@ k_fine_pair(PairView<T> F, const T* __restrict__ u, T* __restrict__ y, SmoothArg
   const int n0base = in0 ? i + F.nxn * r0 : 0, n1base = in1 ? i + F.nxn * r1 : 0;
   const int cpl = F.nxn * F.mp;
   const int cbase = (xin && m < F.mp) ? i + F.nxn * m : -1;
-  const bool need_dir = SMOOTH && a1 != T(0);
+  [[maybe_unused]] const bool need_dir = a1 != T(0) || S.x_lag;
   // geometry of the general path: this thread's x width and its two rows' y widths
   V ga(T(1)), gb(T(1)), gia(T(1)), gib(T(1));
   if constexpr (!CUBE) {
@@ -423,12 +436,12 @@ k_fine_pair(PairView<T> F, const T* __restrict__ u, T* __restrict__ y, SmoothArg
       for (int c = 0; c < 3; ++c) t1[c] += F.kd[3 * n1 + c] * u[3 * n1 + c];
     }
     if constexpr (PREF) {
-      if (f0) node_update(S, a1, a2, n0, t0, o0);
-      if (f1) node_update(S, a1, a2, n1, t1, o1);
-    } else if constexpr (SMOOTH) {
+      if (f0) node_update<T, EPI>(S, a1, a2, n0, t0, o0);
+      if (f1) node_update<T, EPI>(S, a1, a2, n1, t1, o1);
+    } else if constexpr (EPI != kProduct) {
       NodeOps<T> o;
-      if (f0) { load_node_ops(F, S, u, need_dir, n0, o); node_update(S, a1, a2, n0, t0, o); }
-      if (f1) { load_node_ops(F, S, u, need_dir, n1, o); node_update(S, a1, a2, n1, t1, o); }
+      if (f0) { load_node_ops<T, EPI>(F, S, u, need_dir, n0, o); node_update<T, EPI>(S, a1, a2, n0, t0, o); }
+      if (f1) { load_node_ops<T, EPI>(F, S, u, need_dir, n1, o); node_update<T, EPI>(S, a1, a2, n1, t1, o); }
     } else {
       if (f0) {
 #pragma unroll
@@ -451,8 +464,8 @@ k_fine_pair(PairView<T> F, const T* __restrict__ u, T* __restrict__ y, SmoothArg
   auto prefetch = [&](int kk, NodeOps<T>& o0, NodeOps<T>& o1) {
     if constexpr (PREF) {
       if (kk >= K0 && kk < K1) {
-        if (own0) load_node_ops(F, S, u, need_dir, n0base + plane * kk, o0);
-        if (own1) load_node_ops(F, S, u, need_dir, n1base + plane * kk, o1);
+        if (own0) load_node_ops<T, EPI>(F, S, u, need_dir, n0base + plane * kk, o0);
+        if (own1) load_node_ops<T, EPI>(F, S, u, need_dir, n1base + plane * kk, o1);
       }
     }
   };
@@ -463,7 +476,7 @@ k_fine_pair(PairView<T> F, const T* __restrict__ u, T* __restrict__ y, SmoothArg
     load_plane(K0 + 1, vb);
     ca = load_cells(K0 - 1);
     for (int row0 = blockIdx.x * kRowGroups; row0 < F.rows.n; row0 += gridDim.x * kRowGroups)
-      finish_row<T, MODE, CUBE, SMOOTH>(F, u, y, S, a1, a2, row0 + (int)(threadIdx.x >> 3));
+      finish_row<T, MODE, CUBE, EPI>(F, u, y, S, a1, a2, row0 + (int)(threadIdx.x >> 3));
     edge(v0, E);
     put_edge(slot(K0 - 1), E);
     __syncthreads();
@@ -575,56 +588,82 @@ k_fine_pair(PairView<T> F, const T* __restrict__ u, T* __restrict__ y, SmoothArg
   }
 }
 
-template <typename T, int MODE, bool CUBE, int WY, bool SMOOTH>
+template <typename T, int MODE, bool CUBE, int WY, int EPI>
 int launch_pair_kernel(const PairView<T>& F, const T* u, T* y, const SmoothArgs<T>& A, const int* skip, int zc,
                        cudaStream_t s) {
   constexpr int OY = 2 * WY - 2;
   const int nbx = div_up(F.nxn, kXOwn), nby = div_up(F.nyn, OY), nbz = div_up(F.nzn, zc);
   const int64_t blocks = (int64_t)nbx * nby * nbz;
   constexpr size_t smem = pair_smem_bytes<T, MODE, CUBE, WY>();
-  auto kern = k_fine_pair<T, MODE, CUBE, WY, SMOOTH>;
+  auto kern = k_fine_pair<T, MODE, CUBE, WY, EPI>;
   FEB_TRY(set_dyn_smem((const void*)kern, (int)smem));
   kern<<<(unsigned)blocks, 32 * WY, smem, s>>>(F, u, y, A, skip, zc, nbx, nby);
   note_launch();
   return FEB_OK;
 }
 
-template <typename T, int MODE, bool CUBE, int WY, bool SMOOTH>
+template <typename T, int MODE, bool CUBE, int WY, int EPI>
 int prepare_pair_kernel() {
   constexpr size_t smem = pair_smem_bytes<T, MODE, CUBE, WY>();
-  return set_dyn_smem((const void*)k_fine_pair<T, MODE, CUBE, WY, SMOOTH>, (int)smem);
+  return set_dyn_smem((const void*)k_fine_pair<T, MODE, CUBE, WY, EPI>, (int)smem);
 }
 
 template <typename T, int MODE>
 int prepare_pair_precision(bool cube) {
   if constexpr (MODE == MAT_ISO_SRI && std::is_same<T, float>::value) {
-    if (cube) FEB_TRY((prepare_pair_kernel<T, MODE, true, 16, false>()));
+    if (cube) {
+      FEB_TRY((prepare_pair_kernel<T, MODE, true, 16, kProduct>()));
+      FEB_TRY((prepare_pair_kernel<T, MODE, true, 16, kResidual>()));
+    }
   }
   if constexpr (MODE == MAT_ISO_SRI) {
     if (cube) {
-      FEB_TRY((prepare_pair_kernel<T, MODE, true, 8, false>()));
-      FEB_TRY((prepare_pair_kernel<T, MODE, true, 8, true>()));
+      FEB_TRY((prepare_pair_kernel<T, MODE, true, 8, kProduct>()));
+      FEB_TRY((prepare_pair_kernel<T, MODE, true, 8, kResidual>()));
+      FEB_TRY((prepare_pair_kernel<T, MODE, true, 8, kStep>()));
     }
   }
-  FEB_TRY((prepare_pair_kernel<T, MODE, false, 8, false>()));
-  FEB_TRY((prepare_pair_kernel<T, MODE, false, 8, true>()));
+  FEB_TRY((prepare_pair_kernel<T, MODE, false, 8, kProduct>()));
+  FEB_TRY((prepare_pair_kernel<T, MODE, false, 8, kResidual>()));
+  FEB_TRY((prepare_pair_kernel<T, MODE, false, 8, kStep>()));
   return FEB_OK;
 }
 
-template <typename T, int MODE, bool SMOOTH>
-int launch_pair_wy(const PairView<T>& F, const T* u, T* y, const SmoothArgs<T>& A, const int* skip, PairConfig cfg,
+template <typename T, int MODE, int EPI>
+int launch_pair_wy(const PairView<T>& F, const T* u, T* y, const SmoothArgs<T>& A, const int* skip, const PairConfig& cfg,
                    cudaStream_t s) {
-  if (SMOOTH) cfg.wy = 8;   // the smoothing variants need the register room of 8-warp CTAs
-  const int zc = std::max(1, SMOOTH ? cfg.zchunk_smooth : cfg.zchunk);
+  const int zc = std::max(1, EPI == kStep ? cfg.zchunk_smooth : cfg.zchunk);
   if constexpr (MODE == MAT_ISO_SRI) {
     if (F.cube) {
-      if constexpr (std::is_same<T, float>::value && !SMOOTH) {
-        if (cfg.wy == 16) return launch_pair_kernel<T, MODE, true, 16, SMOOTH>(F, u, y, A, skip, zc, s);
+      if constexpr (std::is_same<T, float>::value && EPI != kStep) {   // steps need the register room of 8-warp CTAs
+        if (cfg.wy == 16) return launch_pair_kernel<T, MODE, true, 16, EPI>(F, u, y, A, skip, zc, s);
       }
-      return launch_pair_kernel<T, MODE, true, 8, SMOOTH>(F, u, y, A, skip, zc, s);
+      return launch_pair_kernel<T, MODE, true, 8, EPI>(F, u, y, A, skip, zc, s);
     }
   }
-  return launch_pair_kernel<T, MODE, false, 8, SMOOTH>(F, u, y, A, skip, zc, s);
+  return launch_pair_kernel<T, MODE, false, 8, EPI>(F, u, y, A, skip, zc, s);
+}
+
+// Second half of a smoothing step that is split in two launches: the update of every node from its product.
+// Bound by memory (160 x 112 x 96 cells, FP32, direction only: 142 MB in 25.9 us).  The two halves take 37.7 + 25.9 us there
+// against 76.6 us fused, whose 8 warps with 230 registers hide little of the operands' latency; with the residual instead of
+// the product in the first half 46.5 + 19.0 us.  Where the vectors stay in L2 (96 x 64 x 48: 12.3 + 6 us) fused steps are no
+// slower (16.5 us), so the tuning times both.  Not faster than 82 us at the large size: update warps beside the product's in
+// one CTA (84 us), 16 warps with the operands loaded late and prefetched into L2 (80 us), two CTAs of 128 registers (84 us).
+template <typename T>
+__global__ void __launch_bounds__(256)
+k_pair_update(PairView<T> F, const T* __restrict__ u, const T* t_in, SmoothArgs<T> S, const int* __restrict__ skip) {
+  if (skip && *skip) return;
+  const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (n >= F.ntotal) return;
+  T a1 = T(0), a2 = T(0);
+  pair_coef(S, a1, a2);
+  NodeOps<T> o;
+  T t[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) t[c] = t_in[3 * n + c];
+  load_node_ops<T, kStep>(F, S, u, a1 != T(0) || S.x_lag, (int)n, o);
+  node_update<T, kStep>(S, a1, a2, (int)n, t, o);
 }
 
 // ------------------------------------------------------------------------------------------------ set-up
@@ -805,36 +844,40 @@ __global__ void k_cheb_first6(const T* __restrict__ b, const T* __restrict__ D, 
 template <typename T, int MODE>
 int launch_fine_pair(const PairView<T>& F, const T* u, T* y, const SmoothArgs<T>* S, const int* skip, PairConfig cfg,
                      cudaStream_t s) {
-  if (S) return launch_pair_wy<T, MODE, true>(F, u, y, *S, skip, cfg, s);
-  return launch_pair_wy<T, MODE, false>(F, u, y, SmoothArgs<T>{}, skip, cfg, s);
+  if (!S) return launch_pair_wy<T, MODE, kProduct>(F, u, y, SmoothArgs<T>{}, skip, cfg, s);
+  if (!S->updates()) return launch_pair_wy<T, MODE, kResidual>(F, u, y, *S, skip, cfg, s);
+  if (!cfg.split || !y) return launch_pair_wy<T, MODE, kStep>(F, u, y, *S, skip, cfg, s);
+  FEB_TRY((launch_pair_wy<T, MODE, kProduct>(F, u, y, SmoothArgs<T>{}, skip, cfg, s)));
+  k_pair_update<T><<<div_up(F.ntotal, 256), 256, 0, s>>>(F, u, y, *S, skip); note_launch();
+  return FEB_OK;
 }
 
-template <typename T, int MODE, bool CUBE, int WY, bool SMOOTH>
+template <typename T, int MODE, bool CUBE, int WY, int EPI>
 int pair_occupancy() {
   int nb = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_fine_pair<T, MODE, CUBE, WY, SMOOTH>, 32 * WY,
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_fine_pair<T, MODE, CUBE, WY, EPI>, 32 * WY,
                                                     pair_smem_bytes<T, MODE, CUBE, WY>()) != cudaSuccess)
     return 1;
   return std::max(nb, 1);
 }
 
-template <typename T, bool SMOOTH>
+template <typename T, int EPI>
 int pair_occupancy_mode(int mode, bool cube) {
-  if (mode == MAT_ISO_SRI && cube) return pair_occupancy<T, MAT_ISO_SRI, true, 8, SMOOTH>();
+  if (mode == MAT_ISO_SRI && cube) return pair_occupancy<T, MAT_ISO_SRI, true, 8, EPI>();
   switch (mode) {
-    case MAT_ISO_SRI: return pair_occupancy<T, MAT_ISO_SRI, false, 8, SMOOTH>();
-    case MAT_ISO_FULL: return pair_occupancy<T, MAT_ISO_FULL, false, 8, SMOOTH>();
-    default: return pair_occupancy<T, MAT_ORTHO, false, 8, SMOOTH>();
+    case MAT_ISO_SRI: return pair_occupancy<T, MAT_ISO_SRI, false, 8, EPI>();
+    case MAT_ISO_FULL: return pair_occupancy<T, MAT_ISO_FULL, false, 8, EPI>();
+    default: return pair_occupancy<T, MAT_ORTHO, false, 8, EPI>();
   }
 }
 
 template <typename T>
 int fine_pair_blocks_per_sm(int mode, bool cube, int wy, bool smooth) {
-  if (smooth) return pair_occupancy_mode<T, true>(mode, cube);
+  if (smooth) return pair_occupancy_mode<T, kStep>(mode, cube);
   if constexpr (std::is_same<T, float>::value) {
-    if (wy == 16 && mode == MAT_ISO_SRI && cube) return pair_occupancy<T, MAT_ISO_SRI, true, 16, false>();
+    if (wy == 16 && mode == MAT_ISO_SRI && cube) return pair_occupancy<T, MAT_ISO_SRI, true, 16, kProduct>();
   }
-  return pair_occupancy_mode<T, false>(mode, cube);
+  return pair_occupancy_mode<T, kProduct>(mode, cube);
 }
 template int fine_pair_blocks_per_sm<float>(int, bool, int, bool);
 template int fine_pair_blocks_per_sm<double>(int, bool, int, bool);

@@ -1216,12 +1216,26 @@ struct FebHandle {
     Level& C = L[1];
     T *r = vr<T>(V), *d = vd<T>(V), *e = ve<T>(V), *xs = vt<T>(V);
     const int deg = std::max(1, opt.cheb_degree);
+    // Directions join the iterate late: a step that writes no x leaves d' to later ones, which read it anyway (the product's
+    // input u, or the buffer that the new direction replaces).  The sums and their order are those of x += d' at every step.
+    const T* base = d;         // the iterate without the last `late` directions
+    int late = 0;
+    auto step = [&](const T* u, const T* r_in, T* r_out, T* d_out, int k, bool last, T* x_out, double* x_out64) {
+      SmoothArgs<T> A;
+      A.r_in = r_in; A.r_out = r_out; A.d_out = d_out; A.lp = lp; A.k = k;
+      if (last || late == 2 || base == e) {
+        A.x_in = base; A.x_lag = late >= 1; A.x_add = late == 2 ? e : nullptr;
+        A.x_out = x_out; A.x_out64 = x_out64;
+        base = x_out;
+        late = 0;
+      } else {
+        ++late;
+      }
+      pair_run<T>(u, x, &A, skip);   // x: where a split step leaves K u (the last one replaces it by the result)
+    };
     launch_cheb_first6<T>(b, dinv6<T>(), lp, d, deg == 1 ? xs : nullptr, ntotal, skip, s);
     for (int k = 1; k < deg; ++k) {
-      SmoothArgs<T> A;
-      A.r_in = (k == 1) ? b : r; A.r_out = r; A.x_in = (k == 1) ? d : xs; A.x_out = xs; A.d_out = e; A.lp = lp;
-      A.k = k - 1;
-      pair_run<T>(d, nullptr, &A, skip);
+      step(d, k == 1 ? b : r, r, e, k - 1, k == deg - 1, xs, nullptr);
       std::swap(d, e);
     }
     {
@@ -1233,20 +1247,12 @@ struct FebHandle {
                        kTermDotBufs * C.nterms);
     vcycle<T>(1, vb<T>(C), vx<T>(C), skip);
     launch_prolong_add<T>(V.P, V.nx, V.ny, V.nz, V.nnode, V.ntotal, orig_copy, V.used, vx<T>(C), xs, skip, s);
-    {
-      SmoothArgs<T> A;
-      A.r_in = b; A.r_out = deg > 1 ? r : nullptr; A.x_in = xs; A.d_out = deg > 1 ? d : nullptr;
-      if (deg == 1 && x64) A.x_out64 = x64; else A.x_out = x;
-      A.lp = lp; A.k = -1;
-      pair_run<T>(xs, nullptr, &A, skip);
-    }
-    for (int k = 1; k < deg; ++k) {
-      const bool last = (k == deg - 1);
-      SmoothArgs<T> A;
-      A.r_in = r; A.r_out = last ? nullptr : r; A.x_in = x; A.d_out = last ? nullptr : e; A.lp = lp;
-      if (last && x64) A.x_out64 = x64; else A.x_out = x;
-      A.k = k - 1;
-      pair_run<T>(d, nullptr, &A, skip);
+    base = xs;
+    for (int k = 0; k < deg; ++k) {     // e holds the direction before last, or nothing: the new one may replace it
+      const bool last = k == deg - 1;
+      const bool wide = last && x64;
+      step(k == 0 ? xs : d, k == 0 ? b : r, last ? nullptr : r, last ? nullptr : e, k - 1, last, wide ? nullptr : (last ? x : xs),
+           wide ? x64 : nullptr);
       std::swap(d, e);
     }
   }
@@ -1745,20 +1751,29 @@ int tune_pair(FebHandle* h, PairConfig* best, T* u, T* y, T* y2, T* y3) {
   slot.wy = best->wy;
   slot.zchunk = best->zchunk;
   SmoothArgs<T> A;
-  A.r_in = u; A.r_out = y; A.x_in = u; A.x_out = y2; A.d_out = y3;   // no parameters: a1 = a2 = 0, same traffic
+  A.r_in = u; A.r_out = y; A.x_lag = true; A.d_out = y2;   // no parameters: a1 = a2 = 0, traffic of a step that writes no x
   best_ms = 1e30f;
-  for (int zc : wave_chunks<T>(h, 8, true)) {
-    slot.zchunk_smooth = zc;
-    for (int w = 0; w < 2; ++w) h->pair_run<T>(u, nullptr, &A, nullptr);
+  auto time_step = [&](float* ms) {
+    for (int w = 0; w < 2; ++w) h->pair_run<T>(u, y3, &A, nullptr);
     FEB_TRY(h->tune_events());
     FEB_CUDA(cudaEventRecord(h->tev0, h->s));
-    for (int r = 0; r < 3; ++r) h->pair_run<T>(u, nullptr, &A, nullptr);
+    for (int r = 0; r < 3; ++r) h->pair_run<T>(u, y3, &A, nullptr);
     FEB_CUDA(cudaEventRecord(h->tev1, h->s));
     FEB_CUDA(cudaEventSynchronize(h->tev1));
+    FEB_CUDA(cudaEventElapsedTime(ms, h->tev0, h->tev1));
+    return (int)FEB_OK;
+  };
+  slot.split = best->split = false;
+  for (int zc : wave_chunks<T>(h, 8, true)) {
+    slot.zchunk_smooth = zc;
     float ms = 0.f;
-    FEB_CUDA(cudaEventElapsedTime(&ms, h->tev0, h->tev1));
+    FEB_TRY(time_step(&ms));
     if (ms < best_ms) { best_ms = ms; best->zchunk_smooth = zc; }
   }
+  slot.split = true;
+  float ms = 0.f;
+  FEB_TRY(time_step(&ms));
+  best->split = ms < best_ms;
   slot = *best;
   return FEB_OK;
 }
@@ -1788,13 +1803,13 @@ int autotune_ku(FebHandle* h) {
     }
   }
   if (h->tc_ok && env_tc() == 1) h->ku32 = KuConfig{16, 16, 1};
-  if (penv && *penv) {      // "wy,zchunk[,zchunk_smooth]"
-    int wy = 8, zc = 16, zs = 0;
-    const int got = std::sscanf(penv, "%d,%d,%d", &wy, &zc, &zs);
+  if (penv && *penv) {      // "wy,zchunk[,zchunk_smooth[,split]]"
+    int wy = 8, zc = 16, zs = 0, split = 0;
+    const int got = std::sscanf(penv, "%d,%d,%d,%d", &wy, &zc, &zs, &split);
     if (got >= 2) {
       if (got < 3) zs = zc;
-      h->pc32 = PairConfig{(wy == 16 && h->P32.cube) ? 16 : 8, zc, zs};
-      h->pc64 = PairConfig{8, zc, zs};
+      h->pc32 = PairConfig{(wy == 16 && h->P32.cube) ? 16 : 8, zc, zs, split != 0};
+      h->pc64 = PairConfig{8, zc, zs, split != 0};
       ppinned = true;
     }
   }

@@ -60,3 +60,30 @@ def test_rows_match_cell_kernel(monkeypatch, shape):
         (y64, y32), (c64, _) = out["1"], out["0"]
         assert np.abs(y64 - c64).max() <= 1e-12 * np.abs(c64).max(), name
         assert np.linalg.norm(y32 - c64) / np.linalg.norm(c64) < 2e-6, name
+
+
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-10), ("mixed", 2e-3)])
+def test_split_and_fused_steps_match_unfused(monkeypatch, precision, tol):
+    """One V-cycle with the smoothing steps fused into the product and split into product and update, for every pattern in
+    which directions join the iterate late (degrees 1 to 5), against the separate kernels of FEB_KU_PAIR=0.  A direction that
+    is lost or added twice is an error of the size of the result; FP32 rounding, amplified by soft modes, is far below 2e-3."""
+    import torch
+    monkeypatch.setenv("FEB_KU_TC", "0")
+    F = synth.hindfoot_problem(28, 21, 18, h=2.0, seed=4)
+    fn, fa = F["fixed"]
+    nr, cr, nc, cc, v = F["extra"].node_coo()
+    kw = dict(cn=F["cn"], orig=F["orig"], pen_node=fn, pen_k=np.repeat((fa * 1e6)[:, None], 3, 1),
+              extra_coo=(3 * nr + cr, 3 * nc + cc, v))
+    for degree in (1, 2, 3, 4, 5):
+        z, r = {}, None
+        for name, pair, cfg in (("unfused", "0", ""), ("fused", "1", "8,5,5,0"), ("split", "1", "8,5,5,1")):
+            monkeypatch.setenv("FEB_KU_PAIR", pair)
+            monkeypatch.setenv("FEB_PAIR_CONFIG", cfg)
+            with engine.Problem(F["grid"], _lib.MAT_ISO_SRI, np.concatenate([F["lam"], F["mu"]]), F["active"],
+                                precision=precision, options=dict(cheb_degree=degree), **kw) as P:
+                if r is None:
+                    used = P.used_mask()[0].cpu().numpy().astype(bool)
+                    r = (np.random.default_rng(degree).standard_normal((P.ntotal, 3)) * used[:, None]).ravel()
+                z[name] = P.precondition(torch.from_numpy(r).cuda()).cpu().numpy()
+        for name in ("fused", "split"):
+            assert np.linalg.norm(z[name] - z["unfused"]) <= tol * np.linalg.norm(z["unfused"]), (degree, name)
