@@ -58,23 +58,6 @@ __global__ void __launch_bounds__(256) k_symmetrize(double* __restrict__ M, int 
   }
 }
 
-// M = -S from the swept lower tiles, both triangles.
-__global__ void __launch_bounds__(256) k_mirror(double* __restrict__ M, int ld) {
-  const int ti = blockIdx.y, tj = blockIdx.x;
-  if (tj > ti) return;
-  __shared__ double B[SB][SLD];
-  const int c = threadIdx.x & 63, r0 = threadIdx.x >> 6;
-  for (int r = r0; r < SB; r += 4) {
-    double* p = M + (size_t)(ti * SB + r) * ld + tj * SB + c;
-    const double v = -*p;
-    *p = v;
-    B[r][c] = v;
-  }
-  if (ti == tj) return;
-  __syncthreads();
-  for (int r = r0; r < SB; r += 4) M[(size_t)(tj * SB + r) * ld + ti * SB + c] = B[c][r];
-}
-
 // Symmetric sweep of a 64 x 64 block held 4 x 4 per thread (rows 4 ty + u, columns 4 tx + v): step p turns
 // a_pp = d into -1/d, a_ip and a_pi into a_ip / d and a_ij into a_ij - a_ip a_pj / d; after all steps the block is
 // minus its inverse.  Row p travels through a double-buffered line of shared memory (its column is the same numbers by
@@ -313,52 +296,100 @@ k_sweep_update(double* __restrict__ M, int ld, int k, const double* __restrict__
           make_double2(s[u][v][0], s[u][v][1]);
 }
 
-// x = Minv b on the coarsest level in one launch: the first brows blocks take a row a warp, the remaining blocks zero
-// the entries of nodes outside the dense system (cmap < 0), a disjoint set.  A block gathers b through klist into
-// shared memory once, so that its warps stream their rows of Minv with 16-byte loads and nothing else.  Bound by
-// reading Minv.  2457 dofs: 28.8 us with the gather inside the row loop, 9 us from L2 and 17 us from memory now; two
-// or four rows a warp, deeper unrolling, smaller blocks and an L2 prefetch of the rows were no faster (up to 40 %
-// slower).
-constexpr int kSolveChunk = 4096;
-constexpr int kSolveThreads = 512;
-
+// x = -S b on the coarsest level in one launch, S the swept matrix (minus the inverse), of which the lower tiles are read:
+// block (ti, tj) multiplies its 64 x 64 tile with b_tj and, off the diagonal, its transpose with b_ti, and leaves the two
+// partial vectors in slots of its own; the last block to arrive at a block row adds the row's slots in their order.  The
+// blocks after the tiles zero the entries of nodes outside the dense system (cmap < 0), a disjoint set.  A block has its
+// tile on the way (eight 16-byte loads a thread) before it gathers the 128 values of b.
+// Bound by reading the tiles, and by gather and arrivals where those come from L2.  With all of S read, a row a warp:
+// 3510 dofs in a solve 21.7 -> 17.0 us, 2457 dofs between level-0 sweeps (from memory) 23.0 -> 14.0 us, alone and from L2
+// 9.4 -> 10.4 us.  Runs of tiles with a sum a run, the next tile on its way, were slower (13 us; 5265 dofs 45 against 32).
 template <typename T>
-__global__ void __launch_bounds__(kSolveThreads)
-k_dense_solve(const double* __restrict__ Minv, int nd, int ld, const int* __restrict__ klist,
-              const int* __restrict__ cmap, int64_t n, const T* __restrict__ b, T* __restrict__ x, int brows,
+__global__ void __launch_bounds__(256)
+k_dense_solve(const double* __restrict__ S, int nd, int ld, const int* __restrict__ klist, const int* __restrict__ cmap,
+              int64_t n, const T* __restrict__ b, T* __restrict__ x, int tiles, double* part, int* arrived,
               const int* __restrict__ skip) {
   if (skip && *skip) return;
-  if ((int)blockIdx.x < brows) {
-    __shared__ __align__(16) double bs[kSolveChunk];
-    const int lane = threadIdx.x & 31, row = blockIdx.x * (kSolveThreads / 32) + threadIdx.x / 32;
-    double a0 = 0.0, a1 = 0.0;
-    for (int c0 = 0; c0 < nd; c0 += kSolveChunk) {
-      const int len = min(kSolveChunk, ld - c0);      // a multiple of 64
-      if (c0) __syncthreads();
-#pragma unroll 8
-      for (int j = threadIdx.x; j < len; j += kSolveThreads) {
-        const int q = min(c0 + j, nd - 1);
-        const double v = double(b[3 * (int64_t)klist[q / 3] + q % 3]);
-        bs[j] = c0 + j < nd ? v : 0.0;
-      }
-      __syncthreads();
-      if (row < nd) {
-        const double2* m = reinterpret_cast<const double2*>(Minv + (size_t)row * ld + c0) + lane;
-        const double2* bb = reinterpret_cast<const double2*>(bs) + lane;
-#pragma unroll 8
-        for (int j = 0; j < len / 2; j += 32) {
-          const double2 w = m[j], v = bb[j];
-          a0 += w.x * v.x;
-          a1 += w.y * v.y;
-        }
-      }
-    }
-    const double s = warp_sum(a0 + a1);
-    if (lane == 0 && row < nd) x[3 * (int64_t)klist[row / 3] + row % 3] = T(s);
+  if ((int)blockIdx.x >= tiles) {
+    const int64_t e = (int64_t)(blockIdx.x - tiles) * blockDim.x + threadIdx.x;
+    if (e < 3 * n && cmap[e / 3] < 0) x[e] = T(0);
     return;
   }
-  const int64_t e = (int64_t)(blockIdx.x - brows) * blockDim.x + threadIdx.x;
-  if (e < 3 * n && cmap[e / 3] < 0) x[e] = T(0);
+  __shared__ double xb[2][SB];                   // b_ti, b_tj
+  __shared__ __align__(16) double col[8][SB];
+  __shared__ int last[2];
+  const int nt = ld / SB, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int ti = (int)((sqrtf(8.f * (float)blockIdx.x + 1.f) - 1.f) * 0.5f);
+  while (ti * (ti + 1) / 2 > (int)blockIdx.x) --ti;
+  while ((ti + 1) * (ti + 2) / 2 <= (int)blockIdx.x) ++ti;
+  const int tj = blockIdx.x - ti * (ti + 1) / 2;
+  double2 v[8];
+#pragma unroll
+  for (int r = 0; r < 8; ++r)
+    v[r] = reinterpret_cast<const double2*>(S + (size_t)(ti * SB + 8 * w + r) * ld + tj * SB)[lane];
+  if (threadIdx.x < 2 * SB) {
+    const int h = threadIdx.x / SB, q = (h ? tj : ti) * SB + threadIdx.x % SB, qc = min(q, nd - 1);
+    const double bq = double(b[3 * (int64_t)klist[qc / 3] + qc % 3]);
+    xb[h][threadIdx.x % SB] = q < nd ? bq : 0.0;
+  }
+  __syncthreads();
+  const double x0 = xb[1][2 * lane], x1 = xb[1][2 * lane + 1];
+  double p[8], c0 = 0.0, c1 = 0.0;
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    const double xr = xb[0][8 * w + r];
+    p[r] = v[r].x * x0 + v[r].y * x1;
+    c0 += v[r].x * xr;
+    c1 += v[r].y * xr;
+  }
+  reinterpret_cast<double2*>(col[w])[lane] = make_double2(c0, c1);
+  // sums over the lanes of eight rows at once: after the exchanges lane l holds row 4 (l >> 4 & 1) + 2 (l >> 3 & 1) + (l >> 2 & 1)
+#pragma unroll
+  for (int h = 4, m = 16; h >= 1; h >>= 1, m >>= 1) {
+    const bool up = lane & m;
+#pragma unroll
+    for (int r = 0; r < h; ++r) {
+      const double give = up ? p[r] : p[h + r], keep = up ? p[h + r] : p[r];
+      p[r] = keep + __shfl_xor_sync(0xffffffffu, give, m);
+    }
+  }
+  p[0] += __shfl_xor_sync(0xffffffffu, p[0], 2);
+  p[0] += __shfl_xor_sync(0xffffffffu, p[0], 1);
+  if ((lane & 3) == 0)
+    part[((size_t)ti * nt + tj) * SB + 8 * w + 4 * (lane >> 4) + 2 * ((lane >> 3) & 1) + ((lane >> 2) & 1)] = p[0];
+  __syncthreads();
+  if (ti != tj && threadIdx.x < SB) {
+    double c = 0.0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) c += col[q][threadIdx.x];
+    part[((size_t)tj * nt + ti) * SB + threadIdx.x] = c;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    const int row = threadIdx.x ? tj : ti;
+    const bool mine = threadIdx.x == 0 || ti != tj;
+    __threadfence();                             // the block's slots before its arrival, and the others' after the last one
+    const bool done = mine && atomicAdd(arrived + row, 1) == nt - 1;
+    if (done) arrived[row] = 0;                  // for the next launch
+    __threadfence();
+    last[threadIdx.x] = done;
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {
+    if (!last[h]) continue;
+    const int row = h ? tj : ti, r = threadIdx.x & (SB - 1), g = threadIdx.x / SB;
+    double a = 0.0;
+    const double* q = part + (size_t)row * nt * SB + r;
+#pragma unroll 8
+    for (int t = g; t < nt; t += 4) a += __ldcg(q + (size_t)t * SB);
+    __syncthreads();                             // col is read
+    col[g][r] = a;
+    __syncthreads();
+    const int d = row * SB + r;
+    if (g == 0 && d < nd)
+      x[3 * (int64_t)klist[d / 3] + d % 3] = T(-((col[0][r] + col[1][r]) + (col[2][r] + col[3][r])));
+  }
 }
 
 }  // namespace
@@ -396,7 +427,7 @@ void launch_dense_add_entries(int nent, const int* rdof, const int* cdof, const 
 
 int dense_ld(int nd) { return div_up(nd, SB) * SB; }
 
-// Two launches a step.  Measured: the inverse of 1848 / 2457 / 3510 / 5265 dofs; an update takes 72 us at 5265 dofs
+// Two launches a step.  1890 / 2457 / 3510 / 5265 dofs take 0.86 / 1.42 / 2.5 / 6.7 ms; an update takes 72 us at 5265 dofs
 // (25 TFLOP/s), and below about 3000 dofs the next pivot's chain of divisions (20 us) bounds it.  With 32-wide pivot
 // blocks over the whole matrix and five launches a step the inverse of 3510 dofs took 13.9 ms and that of 2457 6.3 ms.
 int launch_dense_invert(double* M, int nd, double* scratch, int* status, cudaStream_t s) {
@@ -412,24 +443,26 @@ int launch_dense_invert(double* M, int nd, double* scratch, int* status, cudaStr
     k_sweep_panel<<<dim3(nt, SB / 16), 256, 0, s>>>(M, ld, k, Dinv, CT, WT); note_launch();
     if (nt > 1) { k_sweep_update<<<nt * (nt - 1) / 2, 256, smem, s>>>(M, ld, k, CT, WT, Dinv, status); note_launch(); }
   }
-  k_mirror<<<dim3(nt, nt), 256, 0, s>>>(M, ld); note_launch();
   return FEB_OK;
 }
 
 size_t dense_scratch_doubles(int nd) { return (size_t)SB * SB + 2 * (size_t)SB * dense_ld(nd); }
 
+size_t dense_part_doubles(int nd) { const size_t nt = dense_ld(nd) / SB; return nt * nt * SB; }
+int dense_tiles(int nd) { return dense_ld(nd) / SB; }
+
 template <typename T>
-void launch_dense_solve(const double* Minv, int nd, const int* klist, const int* cmap, int64_t n, const T* b, T* x,
-                        const int* skip, cudaStream_t s) {
-  const int brows = div_up(nd, kSolveThreads / 32);
-  k_dense_solve<T><<<brows + div_up(3 * n, kSolveThreads), kSolveThreads, 0, s>>>(Minv, nd, dense_ld(nd), klist, cmap, n,
-                                                                                  b, x, brows, skip);
+void launch_dense_solve(const double* S, int nd, const int* klist, const int* cmap, int64_t n, const T* b, T* x, double* part,
+                        int* arrived, const int* skip, cudaStream_t s) {
+  const int nt = dense_tiles(nd), tiles = nt * (nt + 1) / 2;
+  k_dense_solve<T><<<tiles + div_up(3 * n, 256), 256, 0, s>>>(S, nd, dense_ld(nd), klist, cmap, n, b, x, tiles, part, arrived,
+                                                             skip);
   note_launch();
 }
 
-template void launch_dense_solve<float>(const double*, int, const int*, const int*, int64_t, const float*, float*,
-                                        const int*, cudaStream_t);
-template void launch_dense_solve<double>(const double*, int, const int*, const int*, int64_t, const double*, double*,
-                                         const int*, cudaStream_t);
+template void launch_dense_solve<float>(const double*, int, const int*, const int*, int64_t, const float*, float*, double*,
+                                        int*, const int*, cudaStream_t);
+template void launch_dense_solve<double>(const double*, int, const int*, const int*, int64_t, const double*, double*, double*,
+                                         int*, const int*, cudaStream_t);
 
 }  // namespace feb

@@ -944,7 +944,8 @@ struct FebHandle {
   int coarsest = 0;
   // dense coarsest level
   int nd = 0;
-  double *Minv = nullptr;
+  double *Minv = nullptr, *dense_part = nullptr;   // -inverse of the coarsest level (lower tiles), partial vectors of its products
+  int* dense_arrived = nullptr;
   int *klist = nullptr, *cmap = nullptr;
   // scalars
   LevelParams* lp = nullptr;
@@ -1265,7 +1266,7 @@ struct FebHandle {
     }
     if (l == coarsest) {
       Level& V = L[l];
-      launch_dense_solve<T>(Minv, nd, klist, cmap, V.ntotal, b, x, skip, s);
+      launch_dense_solve<T>(Minv, nd, klist, cmap, V.ntotal, b, x, dense_part, dense_arrived, skip, s);
       return;
     }
     Level& V = L[l];
@@ -2391,6 +2392,8 @@ int build_dense(FebHandle* h) {
   FEB_TRY(H.pool.upload(&H.klist, klist.data(), klist.size()));
   const int ld = dense_ld(H.nd);
   FEB_TRY(H.pool.zeros(&H.Minv, (size_t)ld * ld));
+  FEB_TRY(H.pool.alloc(&H.dense_part, dense_part_doubles(H.nd)));
+  FEB_TRY(H.pool.zeros(&H.dense_arrived, dense_tiles(H.nd)));
   int *dr = nullptr, *dc = nullptr;
   double* dv = nullptr;
   if (H.coarsest > 0 && V.sparse.size()) {
