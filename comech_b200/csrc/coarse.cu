@@ -491,16 +491,16 @@ __global__ void k_sym_pattern(const double* __restrict__ basis, double* __restri
 }
 
 __global__ void k_sym_tags(const double* __restrict__ S64, int cnx, int cny, int cnz,
-                           const uint16_t* __restrict__ cellpair, int fnxn, int mp, const double* __restrict__ mtab,
+                           const uint32_t* __restrict__ cellpair, int fnxn, int mp, const double* __restrict__ mtab,
                            const double* __restrict__ pat, uint8_t* __restrict__ tag) {
   const int64_t n = (int64_t)cnx * cny * cnz;
   const int64_t J = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (J >= n) return;
   const int jx = int(J % cnx), jy = int((J / cnx) % cny), jz = int(J / ((int64_t)cnx * cny));
   const int64_t np = sym_np(cnx, cny, cnz), P = jx + (int64_t)sym_nxp(cnx) * (jy + (int64_t)cny * jz);
-  // fine cell (2 jx, 2 jy, 2 jz): row 2 jy is the upper byte of row pair m = jy
+  // fine cell (2 jx, 2 jy, 2 jz): row 2 jy is the upper half of row pair m = jy
   uint32_t id = 0;
-  if (jy < mp) id = (cellpair[2 * jx + (int64_t)fnxn * (jy + (int64_t)mp * (2 * jz))] >> 8) & 0x7fu;
+  if (jy < mp) id = (cellpair[2 * jx + (int64_t)fnxn * (jy + (int64_t)mp * (2 * jz))] >> 16) & 0x7fu;
   uint8_t t = 0;
   if (id > 0) {
     const double lam = mtab[2 * id], mu = mtab[2 * id + 1];
@@ -1131,7 +1131,7 @@ template int launch_galerkin_direct<MAT_ISO_FULL>(const double*, int, int, doubl
 void launch_sym_pattern(const double* basis, double* pat, cudaStream_t s) {
   k_sym_pattern<<<1, 256, 0, s>>>(basis, pat); note_launch();
 }
-void launch_sym_tags(const double* S64, int cnx, int cny, int cnz, const uint16_t* cellpair, int fnxn, int mp,
+void launch_sym_tags(const double* S64, int cnx, int cny, int cnz, const uint32_t* cellpair, int fnxn, int mp,
                      const double* mtab, const double* pat, uint8_t* tag, cudaStream_t s) {
   const int64_t n = (int64_t)cnx * cny * cnz;
   k_sym_tags<<<div_up(n, kThreads), kThreads, 0, s>>>(S64, cnx, cny, cnz, cellpair, fnxn, mp, mtab, pat, tag);

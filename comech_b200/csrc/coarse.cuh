@@ -153,7 +153,7 @@ void launch_sym_pattern(const double* basis, double* pat, cudaStream_t s);
 // Tags of the compressed level-1 stencil: node J gets the material id of fine cell (2 jx, 2 jy, 2 jz) (read
 // from the paired kernel's cell-pair words) when its stored FP64 half stencil S64 (row-padded) equals
 // lam pat[0] + mu pat[1] to 1e-12 (relative), else 0.
-void launch_sym_tags(const double* S64, int cnx, int cny, int cnz, const uint16_t* cellpair, int fnxn, int mp,
+void launch_sym_tags(const double* S64, int cnx, int cny, int cnz, const uint32_t* cellpair, int fnxn, int mp,
                      const double* mtab, const double* pat, uint8_t* tag, cudaStream_t s);
 
 // Fold diagonal penalties / local extra entries of level 0 into the level-1 stencil.

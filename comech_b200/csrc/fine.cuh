@@ -68,7 +68,7 @@ struct PairView {
   int nxn, nyn, nzn;         // grid nodes per axis
   int mp;                    // row pairs per (x, z) column: nyn / 2 + 1 (rows 2m-1, 2m)
   int64_t nnode, ntotal;     // grid nodes; grid nodes + split copies
-  const uint16_t* cellpair;  // [nzn][mp][nxn]: per row byte bits 0-6 material id, bit 7 node is special
+  const uint32_t* cellpair;  // [nzn][mp][nxn]: per row 16 bits: material id (7), node has a penalty, node is in the row list
   const double* mtab;        // [kMaxMatIds][W] material values of the ids (FP64)
   int nmat;                  // ids in use are < nmat
   bool cube;                 // equal cubic cells of edge h, SRI model: reduced modal core
@@ -76,7 +76,6 @@ struct PairView {
   const T* dx; const T* dy; const T* dz;      // cell widths per axis (general core)
   const T* idx; const T* idy; const T* idz;
   const T* kd;               // penalty diagonal, 3 per node (read at flagged nodes)
-  const uint8_t* rowflag;    // node is in the row list (read at flagged nodes)
   PairRows<T> rows;
   const T* dinv6;            // symmetric block-Jacobi inverse [6][ntotal]: 00 11 22 01 02 12
 };
@@ -133,7 +132,7 @@ void launch_rows(const FineView<double>& F, const int* node, int nrow, const int
                  const uint8_t* ids, int* cell, int4* ex, cudaStream_t s);
 template <int W>
 void launch_pack_pairs(int nx, int ny, int nz, int mp, const uint8_t* ids, const uint8_t* flag, const double* mat_s,
-                       const double* vals, uint16_t* cellpair, int* status, cudaStream_t s);
+                       const double* vals, uint32_t* cellpair, int* status, cudaStream_t s);
 template <typename T>
 void launch_dinv6(const double* D9, int64_t n, T* out, cudaStream_t s);
 template <typename T>

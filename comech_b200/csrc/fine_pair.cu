@@ -32,6 +32,7 @@ namespace feb {
 namespace {
 
 constexpr int kXOwn = 30;
+constexpr uint32_t kPenalty = 0x80u, kListed = 0x100u;   // node flags of a cell-pair word
 // cell codes of the row list: an irregular cell's index, a regular cell's material id as kRegularCell - id, or none
 constexpr int kNoCell = -1, kRegularCell = -1;
 #ifndef FEB_PAIR_UNROLL
@@ -374,7 +375,7 @@ k_fine_pair(PairView<T> F, const T* __restrict__ u, T* __restrict__ y, SmoothArg
     for (int c = 0; c < 3; ++c) v[c] = V((kin && in0) ? p0[c] : T(0), (kin && in1) ? p1[c] : T(0));
   };
   auto load_cells = [&](int k) -> uint32_t {
-    return (cbase >= 0 && k >= 0 && k < F.nzn) ? (uint32_t)F.cellpair[cbase + cpl * k] : 0u;
+    return (cbase >= 0 && k >= 0 && k < F.nzn) ? F.cellpair[cbase + cpl * k] : 0u;
   };
   auto slot = [](int p) { return (p + 2) & 1; };
   // x-edge of a plane: E[c][0] = v + v(+x), E[c][1] = v(+x) - v
@@ -424,14 +425,12 @@ k_fine_pair(PairView<T> F, const T* __restrict__ u, T* __restrict__ y, SmoothArg
     if (kk < K0 || kk >= K1) return;
     const int n0 = n0base + plane * kk, n1 = n1base + plane * kk;
     T t0[3] = {out[0].lo(), out[1].lo(), out[2].lo()}, t1[3] = {out[0].hi(), out[1].hi(), out[2].hi()};
-    bool f0 = own0, f1 = own1;   // the node is finished here
-    if (own0 && (flags & 0x80u)) {
-      f0 = !F.rowflag[n0];
+    const bool f0 = own0 && !(flags & kListed), f1 = own1 && !(flags & kListed << 16);   // the node is finished here
+    if (own0 && (flags & kPenalty)) {
 #pragma unroll
       for (int c = 0; c < 3; ++c) t0[c] += F.kd[3 * n0 + c] * u[3 * n0 + c];
     }
-    if (own1 && (flags & 0x8000u)) {
-      f1 = !F.rowflag[n1];
+    if (own1 && (flags & kPenalty << 16)) {
 #pragma unroll
       for (int c = 0; c < 3; ++c) t1[c] += F.kd[3 * n1 + c] * u[3 * n1 + c];
     }
@@ -517,7 +516,7 @@ k_fine_pair(PairView<T> F, const T* __restrict__ u, T* __restrict__ y, SmoothArg
     }
     // (d) element core of the two cells (i, r0, k), (i, r1, k)
     V FX[8], FY[8], FZ[8];
-    const int id0 = (lane < 31) ? int(cin & 0x7fu) : 0, id1 = (lane < 31) ? int((cin >> 8) & 0x7fu) : 0;
+    const int id0 = (lane < 31) ? int(cin & 0x7fu) : 0, id1 = (lane < 31) ? int((cin >> 16) & 0x7fu) : 0;
     if constexpr (CUBE) {
       const V L16(sMat[id0][0], sMat[id1][0]), M48(sMat[id0][1], sMat[id1][1]);
       cube_sri_core<T>(X, Y, Z, L16, M48, FX, FY, FZ);
@@ -769,21 +768,21 @@ __global__ void k_rows(FineView<double> F, const int* __restrict__ node, int nro
   ex[row] = x;
 }
 
-// node flags: grid nodes that receive a sparse contribution (penalty, extra entry, irregular cell corner)
+// grid nodes with a penalty (flag[n]) and grid nodes of the row list: extra entries, irregular cell corners (flag[nnode + n])
 __global__ void k_flag_nodes(const int* __restrict__ pen_node, int npen, const int* __restrict__ irr_nodes, int nirr,
                              const int* __restrict__ row_dof, int nrow, int64_t nnode, uint8_t* __restrict__ flag) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e < npen && pen_node[e] < nnode) flag[pen_node[e]] = 1;
-  if (e < 8 * nirr && irr_nodes[e] < nnode) flag[irr_nodes[e]] = 1;
-  if (e < nrow && row_dof[e] / 3 < nnode) flag[row_dof[e] / 3] = 1;
+  if (e < 8 * nirr && irr_nodes[e] < nnode) flag[nnode + irr_nodes[e]] = 1;
+  if (e < nrow && row_dof[e] / 3 < nnode) flag[nnode + row_dof[e] / 3] = 1;
 }
 
-// cell-pair words [nzn][mp][nxn]: byte h (h = 0, 1) describes row j = 2m - 1 + h: bits 0-6 the material id
-// of cell (i, j, k) (0 when the cell does not exist or is not regular), bit 7 the flag of node (i, j, k)
+// cell-pair words [nzn][mp][nxn]: half h (h = 0, 1) describes row j = 2m - 1 + h: bits 0-6 the material id
+// of cell (i, j, k) (0 when the cell does not exist or is not regular), then the flags of node (i, j, k)
 template <int W>
 __global__ void k_pack_pairs(int nx, int ny, int nz, int mp, const uint8_t* __restrict__ ids,
                              const uint8_t* __restrict__ flag, const double* __restrict__ mat_s,
-                             const double* __restrict__ vals, uint16_t* __restrict__ cellpair, int* __restrict__ status) {
+                             const double* __restrict__ vals, uint32_t* __restrict__ cellpair, int* __restrict__ status) {
   const int nxn = nx + 1, nyn = ny + 1, nzn = nz + 1;
   const int64_t total = (int64_t)nxn * mp * nzn;
   const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -793,20 +792,22 @@ __global__ void k_pack_pairs(int nx, int ny, int nz, int mp, const uint8_t* __re
   for (int hh = 0; hh < 2; ++hh) {
     const int j = 2 * m - 1 + hh;
     if (j < 0 || j >= nyn) continue;
-    uint32_t byte = 0;
+    uint32_t half = 0;
     if (i < nx && j < ny && k < nz) {
       const int64_t c = i + (int64_t)nx * (j + (int64_t)ny * k);
       const int id = ids[c];
-      byte = (uint32_t)id;
+      half = (uint32_t)id;
       bool same = true;
 #pragma unroll
       for (int q = 0; q < W; ++q) same &= (vals[W * id + q] == mat_s[W * c + q]);
       if (!same) atomicOr(status, 2);
     }
-    if (flag[i + (int64_t)nxn * (j + (int64_t)nyn * k)]) byte |= 0x80u;
-    word |= byte << (8 * hh);
+    const int64_t n = i + (int64_t)nxn * (j + (int64_t)nyn * k);
+    if (flag[(int64_t)nxn * nyn * nzn + n]) half |= kListed;
+    else if (flag[n]) half |= kPenalty;
+    word |= half << (16 * hh);
   }
-  cellpair[e] = (uint16_t)word;
+  cellpair[e] = word;
 }
 
 // symmetric block-Jacobi inverse [6][n] (00 11 22 01 02 12) from the SoA [9][n] inverse
@@ -913,7 +914,7 @@ void launch_flag_nodes(const int* pen_node, int npen, const int* irr_nodes, int 
 }
 template <int W>
 void launch_pack_pairs(int nx, int ny, int nz, int mp, const uint8_t* ids, const uint8_t* flag, const double* mat_s,
-                       const double* vals, uint16_t* cellpair, int* status, cudaStream_t s) {
+                       const double* vals, uint32_t* cellpair, int* status, cudaStream_t s) {
   const int64_t total = (int64_t)(nx + 1) * mp * (nz + 1);
   k_pack_pairs<W><<<div_up(total, kThreads), kThreads, 0, s>>>(nx, ny, nz, mp, ids, flag, mat_s, vals, cellpair, status);
   note_launch();
@@ -953,9 +954,9 @@ INST(double, MAT_ISO_SRI) INST(double, MAT_ISO_FULL) INST(double, MAT_ORTHO)
 template void launch_mat_ids<2>(const double*, int64_t, unsigned long long*, double*, uint8_t*, int*, cudaStream_t);
 template void launch_mat_ids<6>(const double*, int64_t, unsigned long long*, double*, uint8_t*, int*, cudaStream_t);
 template void launch_pack_pairs<2>(int, int, int, int, const uint8_t*, const uint8_t*, const double*, const double*,
-                                   uint16_t*, int*, cudaStream_t);
+                                   uint32_t*, int*, cudaStream_t);
 template void launch_pack_pairs<6>(int, int, int, int, const uint8_t*, const uint8_t*, const double*, const double*,
-                                   uint16_t*, int*, cudaStream_t);
+                                   uint32_t*, int*, cudaStream_t);
 template void launch_dinv6<float>(const double*, int64_t, float*, cudaStream_t);
 template void launch_dinv6<double>(const double*, int64_t, double*, cudaStream_t);
 template void launch_cheb_first6<float>(const float*, const float*, const LevelParams*, float*, float*, int64_t,

@@ -1873,7 +1873,6 @@ int setup_rows(FebHandle* h, const uint8_t* ids) {
   launch_convert<double, float>(kd64, kd32, (int64_t)n3, nullptr, H.s);
   FEB_CUDA(cudaGetLastError());
   H.P64.kd = kd64; H.P32.kd = kd32;
-  H.P64.rowflag = H.P32.rowflag = flag;
   H.P64.rows = PairRows<double>{};
   H.P32.rows = PairRows<float>{};
   // room for every node that may be flagged
@@ -1903,6 +1902,7 @@ int setup_rows(FebHandle* h, const uint8_t* ids) {
   }
   H.pool.free(cmap);
   H.pool.free(start);
+  H.pool.free(flag);
   return FEB_OK;
 }
 
@@ -1922,11 +1922,11 @@ int setup_pair(FebHandle* h, const double* mat_s64) {
   double* vals = nullptr;
   uint8_t *ids = nullptr, *flag = nullptr;
   int* status = nullptr;
-  uint16_t* cellpair = nullptr;
+  uint32_t* cellpair = nullptr;
   FEB_TRY(H.pool.zeros(&keys, kMaxMatIds));
   FEB_TRY(H.pool.zeros(&vals, (size_t)W * kMaxMatIds));
   FEB_TRY(H.pool.alloc(&ids, ncell));
-  FEB_TRY(H.pool.zeros(&flag, H.nnode));
+  FEB_TRY(H.pool.zeros(&flag, 2 * H.nnode));
   FEB_TRY(H.pool.zeros(&status, 1));
   FEB_TRY(H.pool.alloc(&cellpair, (size_t)nxn * mp * nzn));
   launch_mat_ids<W>(mat_s64, ncell, keys, vals, ids, status, H.s);
