@@ -47,15 +47,16 @@ void launch_fine_apply(const FineView<T>& F, const T* u, T* y, const int* skip, 
 // fused in the epilogue.
 constexpr int kMaxMatIds = 128;   // ids 1..127; 0 = no regular cell
 
-// Nodes finished from their cells one by one: node[r], the codes of its up to 8 cells (cell[8 r + q]: the cell of which the node
-// is corner q), its penalties (kd) and its extra entries (dof columns; those of component c are ex[r][c] .. ex[r][c + 1]).
+// Nodes finished from their cells one by one: node[r], its up to 8 cells (cell[8 r + q]: code of the cell of which the node is
+// corner q; corner[2 (8 r + q)] and the next: that cell's nodes), its penalties (kd) and its extra entries (dof columns; those
+// of component c are ex[r][c] .. ex[r][c + 1]).
 template <typename T>
 struct PairRows {
   int n = 0;
   const int* node = nullptr;
   const int* cell = nullptr;
+  const int4* corner = nullptr;
   const int* irr_cell = nullptr;
-  const int* irr_nodes = nullptr;
   const T* irr_mat = nullptr;
   const int4* ex = nullptr;
   const int* ecol = nullptr;
@@ -129,7 +130,7 @@ void launch_flag_nodes(const int* pen_node, int npen, const int* irr_nodes, int 
 void launch_row_flags(const FineView<double>& F, uint8_t* flag, int* cmap, int* start, cudaStream_t s);
 void launch_pen_diag(const int* node, const double* k, int n, double* kd, cudaStream_t s);
 void launch_rows(const FineView<double>& F, const int* node, int nrow, const int* orig_copy, const int* cmap, const int* start,
-                 const uint8_t* ids, int* cell, int4* ex, cudaStream_t s);
+                 const uint8_t* ids, int* cell, int4* corner, int4* ex, cudaStream_t s);
 template <int W>
 void launch_pack_pairs(int nx, int ny, int nz, int mp, const uint8_t* ids, const uint8_t* flag, const double* mat_s,
                        const double* vals, uint32_t* cellpair, int* status, cudaStream_t s);

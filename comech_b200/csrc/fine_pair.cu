@@ -222,18 +222,28 @@ __device__ __forceinline__ void pair_coef(const SmoothArgs<T>& S, T& a1, T& a2) 
   }
 }
 
+// What lane q of a row's group reads of the row list itself.
+struct RowFetch {
+  int n, code;
+  int4 ex, lo, hi;
+};
+
+template <typename T>
+__device__ __forceinline__ RowFetch fetch_row(const PairRows<T>& R, int row) {
+  const int q = threadIdx.x & 7, rc = min(row, R.n - 1);
+  return {R.node[rc], R.cell[8 * rc + q], R.ex[rc], R.corner[2 * (8 * rc + q)], R.corner[2 * (8 * rc + q) + 1]};
+}
+
 // One node of the row list by a group of eight lanes, one cell each: the cell's force at its corner by the element operator
 // (the modal form of the tiles, back-transformed for that corner alone), summed over the group with the node's penalties
 // and extra entries.  Rows past the end: the group idles along.
 template <typename T, int MODE, bool CUBE, int EPI>
 __device__ __forceinline__ void finish_row(const PairView<T>& F, const T* __restrict__ u, T* __restrict__ y,
-                                           const SmoothArgs<T>& S, T a1, T a2, int row) {
+                                           const SmoothArgs<T>& S, T a1, T a2, const RowFetch& f, bool live) {
   constexpr int W = MatWidth<MODE>::value;
   const PairRows<T>& R = F.rows;
-  const int q = threadIdx.x & 7, rc = min(row, R.n - 1);
-  const bool live = row < R.n;
-  const int n = R.node[rc], code = R.cell[8 * rc + q];
-  const int4 ex = R.ex[rc];
+  const int q = threadIdx.x & 7, n = f.n, code = f.code;
+  const int4 ex = f.ex;
   NodeOps<T> o;
   if constexpr (EPI != kProduct) {
     if (live && q == 0) load_node_ops<T, EPI>(F, S, u, a1 != T(0) || S.x_lag, n, o);
@@ -247,23 +257,18 @@ __device__ __forceinline__ void finish_row(const PairView<T>& F, const T* __rest
     else t[2] += x;
   }
   if (code != kNoCell) {
-    int id[8];
+    const int id[8] = {f.lo.x, f.lo.y, f.lo.z, f.lo.w, f.hi.x, f.hi.y, f.hi.z, f.hi.w};
     T m[W];
     int cell = 0;                                // x-fastest cell index, for the widths of the general geometry
     if (code >= 0) {
-      const int4 lo = reinterpret_cast<const int4*>(R.irr_nodes)[2 * code], hi = reinterpret_cast<const int4*>(R.irr_nodes)[2 * code + 1];
-      id[0] = lo.x; id[1] = lo.y; id[2] = lo.z; id[3] = lo.w; id[4] = hi.x; id[5] = hi.y; id[6] = hi.z; id[7] = hi.w;
 #pragma unroll
       for (int p = 0; p < W; ++p) m[p] = R.irr_mat[(size_t)W * code + p];
       if constexpr (!CUBE) cell = R.irr_cell[code];
-    } else {                                     // a regular cell around grid node n
-      const int n0 = n - (q & 1) - F.nxn * (((q >> 1) & 1) + F.nyn * (q >> 2));
-#pragma unroll
-      for (int l = 0; l < 8; ++l) id[l] = n0 + (l & 1) + F.nxn * (((l >> 1) & 1) + F.nyn * (l >> 2));
+    } else {                                     // a regular cell: its first corner is grid node id[0]
 #pragma unroll
       for (int p = 0; p < W; ++p) m[p] = T(F.mtab[W * (kRegularCell - code) + p]);
       if constexpr (!CUBE) {
-        const int i = n0 % F.nxn, j = (n0 / F.nxn) % F.nyn, k = n0 / (F.nxn * F.nyn);
+        const int i = id[0] % F.nxn, j = (id[0] / F.nxn) % F.nyn, k = id[0] / (F.nxn * F.nyn);
         cell = i + F.nx * (j + F.ny * k);
       }
     }
@@ -470,12 +475,21 @@ k_fine_pair(PairView<T> F, const T* __restrict__ u, T* __restrict__ y, SmoothArg
   };
   {   // prologue: face of plane K0-1; the CTA's share of the row list while its planes are on their way
     V v0[3], E[3][2];
+    const int nrow = F.rows.n, group = threadIdx.x >> 3;
+    int row0 = blockIdx.x * kRowGroups;
+    RowFetch rf;
+    if (row0 < nrow) rf = fetch_row(F.rows, row0 + group);
     load_plane(K0 - 1, v0);
     load_plane(K0, va);
     load_plane(K0 + 1, vb);
     ca = load_cells(K0 - 1);
-    for (int row0 = blockIdx.x * kRowGroups; row0 < F.rows.n; row0 += gridDim.x * kRowGroups)
-      finish_row<T, MODE, CUBE, EPI>(F, u, y, S, a1, a2, row0 + (int)(threadIdx.x >> 3));
+    while (row0 < nrow) {                        // the next rows are fetched while these are finished
+      const RowFetch f = rf;
+      const int row = row0 + group;
+      row0 += gridDim.x * kRowGroups;
+      if (row0 < nrow) rf = fetch_row(F.rows, row0 + group);
+      finish_row<T, MODE, CUBE, EPI>(F, u, y, S, a1, a2, f, row < nrow);
+    }
     edge(v0, E);
     put_edge(slot(K0 - 1), E);
     __syncthreads();
@@ -738,7 +752,7 @@ __global__ void k_pen_diag(const int* __restrict__ node, const double* __restric
 // and the bounds of the extra entries of the node's dofs (consecutive CSR rows, some may be missing).
 __global__ void k_rows(FineView<double> F, const int* __restrict__ node, int nrow, const int* __restrict__ orig_copy,
                        const int* __restrict__ cmap, const int* __restrict__ start, const uint8_t* __restrict__ ids,
-                       int* __restrict__ cell, int4* __restrict__ ex) {
+                       int* __restrict__ cell, int4* __restrict__ corner, int4* __restrict__ ex) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int row = t >> 3, q = t & 7;
   if (row >= nrow) return;
@@ -753,6 +767,15 @@ __global__ void k_rows(FineView<double> F, const int* __restrict__ node, int nro
     else if (ids[c] && n < F.nnode) code = kRegularCell - (int)ids[c];
   }
   cell[8 * row + q] = code;
+  int id[8];
+#pragma unroll
+  for (int l = 0; l < 8; ++l) {
+    if (code >= 0) id[l] = F.irr_nodes[8 * (int64_t)code + l];
+    else if (code != kNoCell) id[l] = i + (l & 1) + F.nxn * (j + ((l >> 1) & 1) + F.nyn * (k + (l >> 2)));
+    else id[l] = n;
+  }
+  corner[2 * (8 * row + q)] = make_int4(id[0], id[1], id[2], id[3]);
+  corner[2 * (8 * row + q) + 1] = make_int4(id[4], id[5], id[6], id[7]);
   if (q) return;
   int4 x = make_int4(0, 0, 0, 0);
   int e = start[n];
@@ -931,8 +954,8 @@ void launch_pen_diag(const int* node, const double* k, int n, double* kd, cudaSt
   if (n > 0) { k_pen_diag<<<div_up(n, kThreads), kThreads, 0, s>>>(node, k, n, kd); note_launch(); }
 }
 void launch_rows(const FineView<double>& F, const int* node, int nrow, const int* orig_copy, const int* cmap, const int* start,
-                 const uint8_t* ids, int* cell, int4* ex, cudaStream_t s) {
-  k_rows<<<div_up(8 * (int64_t)nrow, kThreads), kThreads, 0, s>>>(F, node, nrow, orig_copy, cmap, start, ids, cell, ex);
+                 const uint8_t* ids, int* cell, int4* corner, int4* ex, cudaStream_t s) {
+  k_rows<<<div_up(8 * (int64_t)nrow, kThreads), kThreads, 0, s>>>(F, node, nrow, orig_copy, cmap, start, ids, cell, corner, ex);
   note_launch();
 }
 template <typename T>

@@ -1879,7 +1879,7 @@ int setup_rows(FebHandle* h, const uint8_t* ids) {
   const int64_t cap = std::min<int64_t>(H.ntotal, 8 * (int64_t)F.nirr + F.nrow + (H.ntotal - H.nnode));
   if (cap > 0) {
     int *node = nullptr, *cnt = nullptr, *cell = nullptr;
-    int4* ex = nullptr;
+    int4 *ex = nullptr, *corner = nullptr;
     uint8_t* tmp = nullptr;
     size_t tb = 0;
     thrust::counting_iterator<int> it(0);
@@ -1892,11 +1892,12 @@ int setup_rows(FebHandle* h, const uint8_t* ids) {
     FEB_CUDA(cudaMemcpyAsync(&n, cnt, sizeof(int), cudaMemcpyDeviceToHost, H.s));
     FEB_CUDA(cudaStreamSynchronize(H.s));
     FEB_TRY(H.pool.alloc(&cell, 8 * (size_t)n));
+    FEB_TRY(H.pool.alloc(&corner, 16 * (size_t)n));
     FEB_TRY(H.pool.alloc(&ex, n));
-    launch_rows(F, node, n, H.orig_copy, cmap, start, ids, cell, ex, H.s);
+    launch_rows(F, node, n, H.orig_copy, cmap, start, ids, cell, corner, ex, H.s);
     FEB_CUDA(cudaGetLastError());
-    H.P64.rows = PairRows<double>{n, node, cell, F.irr_cell, F.irr_nodes, F.irr_mat, ex, F.col, F.val};
-    H.P32.rows = PairRows<float>{n, node, cell, F.irr_cell, F.irr_nodes, H.F32.irr_mat, ex, H.F32.col, H.F32.val};
+    H.P64.rows = PairRows<double>{n, node, cell, corner, F.irr_cell, F.irr_mat, ex, F.col, F.val};
+    H.P32.rows = PairRows<float>{n, node, cell, corner, F.irr_cell, H.F32.irr_mat, ex, H.F32.col, H.F32.val};
     H.pool.free(tmp);
     H.pool.free(cnt);
   }
