@@ -1322,13 +1322,13 @@ struct FebHandle {
     }
   }
 
-  // One CG iteration (SciPy order: z = M r, beta, p, q = A p, alpha, x, r, convergence).  loop: the body of a device-side
+  // One CG iteration (SciPy order: z = M r, beta, p, q = A p, alpha, x, r, convergence).  loop.on: the body of a device-side
   // while loop, which runs an iteration of a finished CG only when the start was already converged; the kernels that
   // write neither x, r nor the state then need no look at `done`, a dependent load at the head of every one of them.
   template <typename T>
-  void cg_body(CgState* S, T* x_, T* r_, T* z_, T* p_, T* q_, bool loop) {
+  void cg_body(CgState* S, T* x_, T* r_, T* z_, T* p_, T* q_, LoopCondition loop) {
     const int* done = &S->done;
-    const int* skip = loop ? nullptr : done;
+    const int* skip = loop.on ? nullptr : done;
     const int64_t n = 3 * ntotal;
     // the mixed precision's FP32 copy of r is written by the x/r update (and by cg_start before the loop)
     const bool mixed = std::is_same<T, double>::value && opt.precision != FEB_PREC_FP64;
@@ -1337,7 +1337,7 @@ struct FebHandle {
     launch_update_p<T>(z_, p_, S, n, skip, s);
     apply<T>(0, p_, q_, skip);
     launch_dot_finalize<T, T>(FIN_ALPHA, p_, q_, n, partials, ctr, S, done, s);
-    launch_update_xr_conv<T>(p_, q_, x_, r_, mixed ? rf : nullptr, S, n, partials, ctr, done, s);
+    launch_update_xr_conv<T>(p_, q_, x_, r_, mixed ? rf : nullptr, S, n, partials, ctr, loop, done, s);
   }
 
   // one CG iteration captured as a graph; with use_graphs == 2 the iteration is the body of a device-side
@@ -1362,17 +1362,16 @@ struct FebHandle {
       FEB_CUDA(cudaGraphAddNode(&node, g, nullptr, 0, &cp));
       cudaGraph_t body = cp.conditional.phGraph_out[0];
       FEB_CUDA(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-      if (inner) cg_body<float>(S, xf, rf, zf, pf, qf, true);
-      else cg_body<double>(S, x, r, z, p, q, true);
-      launch_set_condition(cond, S, s);
+      if (inner) cg_body<float>(S, xf, rf, zf, pf, qf, LoopCondition{true, cond});
+      else cg_body<double>(S, x, r, z, p, q, LoopCondition{true, cond});
       FEB_CUDA(cudaStreamEndCapture(s, &body));
       size_t nn = 0;
       FEB_CUDA(cudaGraphGetNodes(body, nullptr, &nn));
       *nodes = (int)nn;
     } else {
       FEB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-      if (inner) cg_body<float>(S, xf, rf, zf, pf, qf, false);
-      else cg_body<double>(S, x, r, z, p, q, false);
+      if (inner) cg_body<float>(S, xf, rf, zf, pf, qf, {});
+      else cg_body<double>(S, x, r, z, p, q, {});
       FEB_CUDA(cudaStreamEndCapture(s, &g));
       size_t nn = 0;
       FEB_CUDA(cudaGraphGetNodes(g, nullptr, &nn));
@@ -1416,8 +1415,8 @@ struct FebHandle {
           launches += *nn;
           note_launch(*nn);
         } else {
-          if (inner) cg_body<float>(S, xf, rf, zf, pf, qf, false);
-          else cg_body<double>(S, x, r, z, p, q, false);
+          if (inner) cg_body<float>(S, xf, rf, zf, pf, qf, {});
+          else cg_body<double>(S, x, r, z, p, q, {});
         }
       }
     }
@@ -2763,8 +2762,7 @@ int add_batch_instance(FebHandle& H, cudaGraph_t G, const double* f_in, const do
   FEB_CUDA(cudaGraphAddNode(&ncond, G, &npre, 1, &cp));
   cudaGraph_t body = cp.conditional.phGraph_out[0];
   FEB_CUDA(cudaStreamBeginCaptureToGraph(H.s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-  H.cg_body<double>(H.st, H.x, H.r, H.z, H.p, H.q, true);
-  launch_set_condition(cond, H.st, H.s);
+  H.cg_body<double>(H.st, H.x, H.r, H.z, H.p, H.q, LoopCondition{true, cond});
   FEB_CUDA(cudaStreamEndCapture(H.s, &body));
   // finish
   cudaGraph_t post = nullptr;

@@ -24,35 +24,50 @@ k_dot_partial(const Ta* __restrict__ a, const Tb* __restrict__ b, int64_t n, dou
   if (threadIdx.x == 0) partials[blockIdx.x] = s;
 }
 
+// What the CG's scalar steps read of the state.  A reduction's kernel loads it at its start, so that the step at its end does
+// not wait for it.
+struct CgScalars {
+  double rz, rz_old, thr2;
+  int it, maxiter;
+};
+__device__ __forceinline__ CgScalars load_scalars(const CgState* st) {
+  return {st->rz, st->rz_old, st->thr2, st->it, st->maxiter};
+}
+
 // The scalar step of a reduction's caller, given the reduction's value s (thread 0 only).
-__device__ void finalize_step(int kind, double s, CgState* st, LevelParams* lp, int deg) {
+__device__ __forceinline__ void cg_step(int kind, double s, const CgScalars& c, CgState* st) {
   switch (kind) {
     case FIN_RZ:
       st->rz = s;
-      st->beta = (st->it == 0) ? 0.0 : s / st->rz_old;
+      st->beta = (c.it == 0) ? 0.0 : s / c.rz_old;
       break;
     case FIN_ALPHA:
       st->pq = s;
       if (!(s > 0.0) || !isfinite(s)) {
         st->status = isfinite(s) ? FEB_ERR_BREAKDOWN : FEB_ERR_NAN;
         st->done = 1;
-        st->flag = st->maxiter;
+        st->flag = c.maxiter;
       } else {
-        st->alpha = st->rz / s;
+        st->alpha = c.rz / s;
       }
       break;
     case FIN_CONV:
       st->rr = s;
-      st->rz_old = st->rz;
-      st->it += 1;
+      st->rz_old = c.rz;
+      st->it = c.it + 1;
       if (!isfinite(s)) {
-        st->status = FEB_ERR_NAN; st->done = 1; st->flag = st->maxiter;
-      } else if (s < st->thr2) {
+        st->status = FEB_ERR_NAN; st->done = 1; st->flag = c.maxiter;
+      } else if (s < c.thr2) {
         st->done = 1; st->flag = 0;
-      } else if (st->it >= st->maxiter) {
-        st->done = 1; st->flag = st->maxiter;
+      } else if (c.it + 1 >= c.maxiter) {
+        st->done = 1; st->flag = c.maxiter;
       }
       break;
+  }
+}
+
+__device__ void finalize_step(int kind, double s, CgState* st, LevelParams* lp, int deg) {
+  switch (kind) {
     case FIN_INIT:
       st->rr = s;
       if (!isfinite(s)) { st->status = FEB_ERR_NAN; st->done = 1; st->flag = st->maxiter; }
@@ -101,24 +116,25 @@ k_finalize(int kind, const double* __restrict__ partials, int np, CgState* st, L
   if (threadIdx.x == 0) finalize_step(kind, s, st, lp, deg);
 }
 
-// Last-block finalisation of a grid reduction: every block has stored its partial; the block that arrives
-// last (counted on `ctr`, after a fence that publishes the partial) sums all partials in the same fixed order
-// as k_finalize, runs the scalar step and re-arms the counter.  Block-uniform; no block waits for another.
-__device__ __forceinline__ void last_block_finalize(int kind, double* partials, unsigned int* ctr, CgState* st) {
+// Last-block sum of a grid reduction: thread 0 of every block stores the block's partial s; the block that arrives last
+// (counted on `ctr`, between thread 0's fences) sums all partials in a fixed order into t and re-arms the counter.
+// Block-uniform; no block waits for another.  True in thread 0 of that block.
+__device__ __forceinline__ bool last_block_sum(double s, double* partials, unsigned int* ctr, double& t) {
   __shared__ bool last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(ctr, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  double s = 0.0;
-  for (int i = threadIdx.x; i < (int)gridDim.x; i += kThreads) s += ((volatile double*)partials)[i];
-  s = block_sum(s);
   if (threadIdx.x == 0) {
-    finalize_step(kind, s, st, nullptr, 0);
-    *ctr = 0u;
+    partials[blockIdx.x] = s;
+    __threadfence();
+    last = atomicAdd(ctr, 1u) == gridDim.x - 1;
+    __threadfence();
   }
+  __syncthreads();
+  if (!last) return false;
+  t = 0.0;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += kThreads) t += __ldcg(partials + i);
+  t = block_sum(t);
+  if (threadIdx.x != 0) return false;
+  *ctr = 0u;
+  return true;
 }
 
 // dot product with the caller's scalar step in the last block (FIN_RZ, FIN_ALPHA)
@@ -127,6 +143,7 @@ __global__ void __launch_bounds__(kThreads)
 k_dot_finalize(int kind, const Ta* __restrict__ a, const Tb* __restrict__ b, int64_t n, double* partials,
                unsigned int* ctr, CgState* st, const int* __restrict__ skip) {
   if (skip && *skip) return;
+  const CgScalars c = load_scalars(st);
   double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
   const int64_t stride = (int64_t)gridDim.x * kThreads;
   int64_t i = blockIdx.x * (int64_t)kThreads + threadIdx.x;
@@ -137,9 +154,8 @@ k_dot_finalize(int kind, const Ta* __restrict__ a, const Tb* __restrict__ b, int
     s3 += double(a[i + 3 * stride]) * double(b[i + 3 * stride]);
   }
   for (; i < n; i += stride) s0 += double(a[i]) * double(b[i]);
-  double s = block_sum((s0 + s1) + (s2 + s3));
-  if (threadIdx.x == 0) partials[blockIdx.x] = s;
-  last_block_finalize(kind, partials, ctr, st);
+  double t;
+  if (last_block_sum(block_sum((s0 + s1) + (s2 + s3)), partials, ctr, t)) cg_step(kind, t, c, st);
 }
 
 template <typename T>
@@ -151,15 +167,20 @@ __global__ void k_update_p(const T* __restrict__ z, T* __restrict__ p, const CgS
     p[i] = z[i] + beta * p[i];
 }
 
-// x += alpha p, r -= alpha q, partial ||r||^2; rf (optional) receives r in FP32 for the next FP32 V-cycle;
-// with ctr the last block runs the convergence step (FIN_CONV) itself
+// x += alpha p, r -= alpha q, ||r||^2 and the convergence step (FIN_CONV); rf (optional) receives r in FP32 for the next
+// FP32 V-cycle.  loop.on: the iteration is the body of a device-side while loop, and this kernel, its last, sets the loop's
+// condition (a launch of one thread for it took 2 us).
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 k_update_xr(const T* __restrict__ p, const T* __restrict__ q, T* __restrict__ x, T* __restrict__ r,
-            float* __restrict__ rf, CgState* st, int64_t n, double* partials, unsigned int* ctr,
+            float* __restrict__ rf, CgState* st, int64_t n, double* partials, unsigned int* ctr, LoopCondition loop,
             const int* __restrict__ skip) {
-  if (skip && *skip) return;
+  if (skip && *skip) {
+    if (loop.on && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(loop.handle, 0u);
+    return;
+  }
   const T alpha = T(st->alpha);
+  const CgScalars c = load_scalars(st);
   double s0 = 0.0, s1 = 0.0;
   const int64_t stride = (int64_t)gridDim.x * kThreads;
   int64_t i = blockIdx.x * (int64_t)kThreads + threadIdx.x;
@@ -180,9 +201,11 @@ k_update_xr(const T* __restrict__ p, const T* __restrict__ q, T* __restrict__ x,
     if (rf) rf[i] = float(ri);
     s0 += double(ri) * double(ri);
   }
-  double s = block_sum(s0 + s1);
-  if (threadIdx.x == 0) partials[blockIdx.x] = s;
-  if (ctr) last_block_finalize(FIN_CONV, partials, ctr, st);
+  double t;
+  if (last_block_sum(block_sum(s0 + s1), partials, ctr, t)) {
+    cg_step(FIN_CONV, t, c, st);
+    if (loop.on) cudaGraphSetConditional(loop.handle, st->done ? 0u : 1u);
+  }
 }
 
 template <typename T>
@@ -303,24 +326,13 @@ k_bj_apply_norm(const T* __restrict__ D, const T* __restrict__ v, T* __restrict_
     s += double(z0) * double(z0) + double(z1) * double(z1) + double(z2) * double(z2);
   }
   s = block_sum(s);
-  if (threadIdx.x == 0) partials[blockIdx.x] = s;
-  if (!ctr) return;
-  __shared__ bool last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(ctr, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  double t = 0.0;
-  for (int i = threadIdx.x; i < (int)gridDim.x; i += kThreads) t += ((volatile double*)partials)[i];
-  t = block_sum(t);
-  if (threadIdx.x == 0) {
+  double t;
+  if (!ctr) {
+    if (threadIdx.x == 0) partials[blockIdx.x] = s;
+  } else if (last_block_sum(s, partials, ctr, t)) {
     finalize_step(FIN_POWER, t, nullptr, fin, deg);
-    *ctr = 0u;
   }
 }
-
 
 template <typename Ts, typename Td>
 __global__ void k_convert(const Ts* __restrict__ a, Td* __restrict__ b, int64_t n, const int* __restrict__ skip) {
@@ -358,17 +370,13 @@ __global__ void k_mask_vector(double* __restrict__ v, const uint8_t* __restrict_
   if (!used[i / 3]) v[i] = fill;
 }
 
-__global__ void k_set_condition(cudaGraphConditionalHandle h, const CgState* __restrict__ st) {
-  cudaGraphSetConditional(h, st->done ? 0u : 1u);
-}
+// blocks of a self-finishing reduction: an element a thread, kRedBlocks at most.  Fewer blocks with several elements a thread
+// were slower on small vectors (24 thousand values: 6.2 us with four, 5.6 us with all kRedBlocks).
+inline int red_grid(int64_t n) { return (int)std::min<int64_t>(kRedBlocks, div_up(n, kThreads)); }
 
 inline int grid_for(int64_t n) { return int(std::min<int64_t>((n + kThreads - 1) / kThreads, 8 * kSmCount)); }
 
 }  // namespace
-
-void launch_set_condition(cudaGraphConditionalHandle h, const CgState* st, cudaStream_t s) {
-  k_set_condition<<<1, 1, 0, s>>>(h, st); note_launch();
-}
 
 template <typename Ta, typename Tb>
 void launch_dot_partial(const Ta* a, const Tb* b, int64_t n, double* partials, const int* skip, cudaStream_t s) {
@@ -386,22 +394,15 @@ void launch_update_p(const T* z, T* p, const CgState* st, int64_t n, const int* 
 }
 
 template <typename T>
-void launch_update_xr(const T* p, const T* q, T* x, T* r, const CgState* st, int64_t n, double* partials,
-                      const int* skip, cudaStream_t s) {
-  k_update_xr<T><<<kRedBlocks, kThreads, 0, s>>>(p, q, x, r, nullptr, const_cast<CgState*>(st), n, partials, nullptr,
-                                                 skip); note_launch();
-}
-
-template <typename T>
 void launch_update_xr_conv(const T* p, const T* q, T* x, T* r, float* rf, CgState* st, int64_t n, double* partials,
-                           unsigned int* ctr, const int* skip, cudaStream_t s) {
-  k_update_xr<T><<<kRedBlocks, kThreads, 0, s>>>(p, q, x, r, rf, st, n, partials, ctr, skip); note_launch();
+                           unsigned int* ctr, LoopCondition loop, const int* skip, cudaStream_t s) {
+  k_update_xr<T><<<red_grid(n), kThreads, 0, s>>>(p, q, x, r, rf, st, n, partials, ctr, loop, skip); note_launch();
 }
 
 template <typename Ta, typename Tb>
 void launch_dot_finalize(int kind, const Ta* a, const Tb* b, int64_t n, double* partials, unsigned int* ctr,
                          CgState* st, const int* skip, cudaStream_t s) {
-  k_dot_finalize<Ta, Tb><<<kRedBlocks, kThreads, 0, s>>>(kind, a, b, n, partials, ctr, st, skip); note_launch();
+  k_dot_finalize<Ta, Tb><<<red_grid(n), kThreads, 0, s>>>(kind, a, b, n, partials, ctr, st, skip); note_launch();
 }
 
 template <typename T>
@@ -441,7 +442,7 @@ void launch_random_start(T* x, const uint8_t* mask, int64_t nn, uint64_t seed, c
 template <typename T>
 void launch_bj_apply_norm(const T* Dinv, const T* v, T* y, int64_t nn, double* partials, cudaStream_t s,
                           const LevelParams* scale, LevelParams* fin, unsigned int* ctr, int deg) {
-  k_bj_apply_norm<T><<<kRedBlocks, kThreads, 0, s>>>(Dinv, v, y, nn, partials, scale, fin, ctr, deg); note_launch();
+  k_bj_apply_norm<T><<<ctr ? red_grid(nn) : kRedBlocks, kThreads, 0, s>>>(Dinv, v, y, nn, partials, scale, fin, ctr, deg); note_launch();
 }
 
 template void launch_random_start<float>(float*, const uint8_t*, int64_t, uint64_t, cudaStream_t);
@@ -476,8 +477,6 @@ void launch_mask_vector(double* v, const uint8_t* used, int64_t nn, double fill,
 
 #define INST_T(T)                                                                                              \
   template void launch_update_p<T>(const T*, T*, const CgState*, int64_t, const int*, cudaStream_t);          \
-  template void launch_update_xr<T>(const T*, const T*, T*, T*, const CgState*, int64_t, double*, const int*,   \
-                                    cudaStream_t);                                                             \
   template void launch_cheb_first<T>(const T*, T*, T*, T*, const T*, const LevelParams*, int64_t, const int*,   \
                                      cudaStream_t, const TermAcc<T>&);                                         \
   template void launch_cheb_init<T>(const T*, const T*, T*, T*, T*, const T*, const LevelParams*, int64_t,      \
@@ -497,9 +496,9 @@ template void launch_dot_partial<float, float>(const float*, const float*, int64
                                                cudaStream_t);
 template void launch_convert<double, float>(const double*, float*, int64_t, const int*, cudaStream_t);
 template void launch_update_xr_conv<double>(const double*, const double*, double*, double*, float*, CgState*, int64_t,
-                                            double*, unsigned int*, const int*, cudaStream_t);
+                                            double*, unsigned int*, LoopCondition, const int*, cudaStream_t);
 template void launch_update_xr_conv<float>(const float*, const float*, float*, float*, float*, CgState*, int64_t,
-                                           double*, unsigned int*, const int*, cudaStream_t);
+                                           double*, unsigned int*, LoopCondition, const int*, cudaStream_t);
 template void launch_dot_finalize<double, double>(int, const double*, const double*, int64_t, double*, unsigned int*,
                                                   CgState*, const int*, cudaStream_t);
 template void launch_dot_finalize<float, float>(int, const float*, const float*, int64_t, double*, unsigned int*,

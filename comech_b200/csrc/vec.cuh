@@ -63,8 +63,11 @@ struct LevelParams {
   double a1[8], a2[8];       // Chebyshev step k: d = a1[k] d + a2[k] M r
 };
 
-// sets the while-loop condition of a conditional graph node: continue while the CG is not done
-void launch_set_condition(cudaGraphConditionalHandle h, const CgState* st, cudaStream_t s);
+// the condition of the device-side while loop whose body an iteration is (on), or none
+struct LoopCondition {
+  bool on = false;
+  cudaGraphConditionalHandle handle{};
+};
 
 template <typename Ta, typename Tb>
 void launch_dot_partial(const Ta* a, const Tb* b, int64_t n, double* partials, const int* skip, cudaStream_t s);
@@ -77,14 +80,12 @@ void launch_finalize(int kind, const double* partials, CgState* st, LevelParams*
 
 template <typename T>
 void launch_update_p(const T* z, T* p, const CgState* st, int64_t n, const int* skip, cudaStream_t s);
-template <typename T>
-void launch_update_xr(const T* p, const T* q, T* x, T* r, const CgState* st, int64_t n, double* partials,
-                      const int* skip, cudaStream_t s);
-// the CG's x/r update with the convergence step (FIN_CONV) in its last block; rf (optional) receives r in
-// FP32.  ctr: a zeroed counter, re-armed by the kernel, used by one reduction at a time on the stream.
+// the CG's x/r update with the convergence step (FIN_CONV) in its last block, which also sets the loop's condition (continue
+// while the CG is not done); rf (optional) receives r in FP32.  ctr: a zeroed counter, re-armed by the kernel, used by one
+// reduction at a time on the stream.
 template <typename T>
 void launch_update_xr_conv(const T* p, const T* q, T* x, T* r, float* rf, CgState* st, int64_t n, double* partials,
-                           unsigned int* ctr, const int* skip, cudaStream_t s);
+                           unsigned int* ctr, LoopCondition loop, const int* skip, cudaStream_t s);
 // a.b with the step `kind` (FIN_RZ, FIN_ALPHA) in the last block
 template <typename Ta, typename Tb>
 void launch_dot_finalize(int kind, const Ta* a, const Tb* b, int64_t n, double* partials, unsigned int* ctr,
