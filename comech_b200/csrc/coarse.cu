@@ -69,201 +69,120 @@ __global__ void k_csr_add(int nrow, const int* __restrict__ row_dof, const int* 
   atomic_add(y + row_dof[e], s);
 }
 
-template <typename T>
-__device__ __forceinline__ void restrict_grid_at(const TransferDev& P, int jx, int jy, int jz, int fnx, int fny, const T* rf,
-                                                 T& s0, T& s1, T& s2) {
+// Coarse node J's fan along one axis: fine nodes f - 1, f, f + 1 around its own with their weights; weight 0 and index f
+// where there is none.
+template <bool EVEN>
+__device__ __forceinline__ void axis_fan3(const AxisDev& A, int J, int (&I)[3], double (&w)[3]) {
+  const int f = EVEN ? 2 * J : A.cidx[J];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const int i = f + a - 1;
+    const bool in = i >= 0 && i < A.nf;
+    w[a] = EVEN ? (in ? (a == 1 ? 1.0 : 0.5) : 0.0) : A.fan[3 * J + a];
+    I[a] = in ? i : f;
+  }
+}
+
+// r_c = P^T r_f, a thread a coarse node (EVEN: weights 1 and 1/2, no tables).  All 81 loads of a node's 27 fine neighbours
+// are independent of one another and of any branch; with loops over the neighbours that exist the loads went out a few at a
+// time.  Split copies that restrict into the node (cp_ptr; grid weights, ascending copy order) are gathered by the same
+// thread.  Bound by latency on small levels.  Mean over the levels, before and after: 24x18x16 7.7 -> 5.5 us (FP32),
+// 160x112x96 7.0 -> 5.9 us (FP32), 64x45x38 (odd, FP64) 10.0 + 4.9 (copies by atomics) -> 5.5 us.
+template <typename T, bool EVEN>
+__global__ void __launch_bounds__(128)
+k_restrict(TransferDev P, const T* __restrict__ rf, T* __restrict__ rc, const int* __restrict__ skip, T* __restrict__ zero,
+           int nzero, int64_t fnnode) {
+  if (skip && *skip) return;
+  if (nzero && blockIdx.x == 0)
+    for (int e = threadIdx.x; e < nzero; e += blockDim.x) zero[e] = T(0);
+  const int cnx = P.ax[0].nc, cny = P.ax[1].nc, cnz = P.ax[2].nc, fnx = P.ax[0].nf, fny = P.ax[1].nf;
+  const int J = blockIdx.x * 128 + threadIdx.x;
+  if (J >= cnx * cny * cnz) return;
+  int cb = 0, ce = 0;
+  if (P.cp_ptr) { cb = P.cp_ptr[J]; ce = P.cp_ptr[J + 1]; }
   int Ix[3], Iy[3], Iz[3];
   double wx[3], wy[3], wz[3];
-  int nxs = axis_fan(P.ax[0], jx, Ix, wx), nys = axis_fan(P.ax[1], jy, Iy, wy), nzs = axis_fan(P.ax[2], jz, Iz, wz);
-  s0 = s1 = s2 = T(0);
-  for (int c = 0; c < nzs; ++c)
-    for (int b = 0; b < nys; ++b)
-      for (int a = 0; a < nxs; ++a) {
-        int64_t f = Ix[a] + (int64_t)fnx * (Iy[b] + (int64_t)fny * Iz[c]);
-        T w = T(wx[a] * wy[b] * wz[c]);
-        s0 += w * rf[3 * f]; s1 += w * rf[3 * f + 1]; s2 += w * rf[3 * f + 2];
+  axis_fan3<EVEN>(P.ax[0], J % cnx, Ix, wx);
+  axis_fan3<EVEN>(P.ax[1], (J / cnx) % cny, Iy, wy);
+  axis_fan3<EVEN>(P.ax[2], J / (cnx * cny), Iz, wz);
+  T s0 = T(0), s1 = T(0), s2 = T(0);
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const T* r = rf + 3 * ((int64_t)Ix[a] + (int64_t)fnx * (Iy[b] + (int64_t)fny * Iz[c]));
+        const T w = T(wx[a] * wy[b] * wz[c]);
+        s0 += w * r[0]; s1 += w * r[1]; s2 += w * r[2];
       }
+  for (int e = cb; e < ce; ++e) {
+    const int64_t f = fnnode + P.cp_copy[e];
+    const T w = T(P.cp_w[e]);
+    s0 += w * rf[3 * f]; s1 += w * rf[3 * f + 1]; s2 += w * rf[3 * f + 2];
+  }
+  rc[3 * J] = s0; rc[3 * J + 1] = s1; rc[3 * J + 2] = s2;
 }
 
-template <typename T>
-__global__ void k_restrict_grid(TransferDev P, int fnx, int fny, const T* __restrict__ rf, T* __restrict__ rc,
-                                const int* __restrict__ skip, T* __restrict__ zero, int nzero) {
-  if (skip && *skip) return;
-  if (nzero && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0)
-    for (int e = threadIdx.x; e < nzero; e += blockDim.x) zero[e] = T(0);
+// Interpolated coarse value at fine grid position (pi, pj, pk): up to 8 coarse nodes, weight 0 where there are fewer.
+template <typename T, bool EVEN>
+__device__ __forceinline__ void prolong_at(const TransferDev& P, int pi, int pj, int pk, const T* xc, T& s0, T& s1, T& s2) {
+  int J[3][2];
+  double w[3][2];
+  const int p[3] = {pi, pj, pk};
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const AxisDev& A = P.ax[d];
+    if constexpr (EVEN) {
+      J[d][0] = p[d] >> 1; J[d][1] = (p[d] + 1) >> 1;
+      w[d][0] = (p[d] & 1) ? 0.5 : 1.0; w[d][1] = (p[d] & 1) ? 0.5 : 0.0;
+    } else {
+      J[d][0] = A.ca[p[d]]; J[d][1] = A.cb[p[d]];
+      w[d][0] = A.wa[p[d]]; w[d][1] = J[d][1] != J[d][0] ? A.wb[p[d]] : 0.0;
+    }
+  }
   const int cnx = P.ax[0].nc, cny = P.ax[1].nc;
-  const int jx = blockIdx.x * blockDim.x + threadIdx.x, jy = blockIdx.y, jz = blockIdx.z;
-  if (jx >= cnx) return;
-  const int64_t J = jx + (int64_t)cnx * (jy + (int64_t)cny * jz);
-  T s0, s1, s2;
-  restrict_grid_at(P, jx, jy, jz, fnx, fny, rf, s0, s1, s2);
-  rc[3 * J] = s0; rc[3 * J + 1] = s1; rc[3 * J + 2] = s2;
-}
-
-// r_c = P^T r_f for even coarsening: coarse node J gathers fine nodes 2 J + a, a in {-1, 0, 1} per axis, with
-// weight 1 (a = 0) or 1/2 (a = +-1)
-template <typename T>
-__device__ __forceinline__ void restrict_even_at(int jx, int jy, int jz, int fnx, int fny, int fnz, const T* rf, T& s0, T& s1,
-                                                 T& s2) {
   s0 = s1 = s2 = T(0);
 #pragma unroll
-  for (int c = -1; c <= 1; ++c) {
-    const int fk = 2 * jz + c;
-    if (fk < 0 || fk >= fnz) continue;
+  for (int c = 0; c < 2; ++c)
 #pragma unroll
-    for (int b = -1; b <= 1; ++b) {
-      const int fj = 2 * jy + b;
-      if (fj < 0 || fj >= fny) continue;
+    for (int b = 0; b < 2; ++b)
 #pragma unroll
-      for (int a = -1; a <= 1; ++a) {
-        const int fi = 2 * jx + a;
-        if (fi < 0 || fi >= fnx) continue;
-        const T w = T((a ? 0.5 : 1.0) * (b ? 0.5 : 1.0) * (c ? 0.5 : 1.0));
-        const int64_t f = fi + (int64_t)fnx * (fj + (int64_t)fny * fk);
-        s0 += w * rf[3 * f]; s1 += w * rf[3 * f + 1]; s2 += w * rf[3 * f + 2];
-      }
-    }
-  }
-}
-
-template <typename T>
-__global__ void k_restrict_even(int cnx, int cny, int fnx, int fny, int fnz, const T* __restrict__ rf,
-                                T* __restrict__ rc, const int* __restrict__ skip, T* __restrict__ zero, int nzero,
-                                const int* __restrict__ cp_ptr, const int* __restrict__ cp_copy,
-                                const double* __restrict__ cp_w, int64_t fnnode) {
-  if (skip && *skip) return;
-  if (nzero && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0)
-    for (int e = threadIdx.x; e < nzero; e += blockDim.x) zero[e] = T(0);
-  const int jx = blockIdx.x * blockDim.x + threadIdx.x, jy = blockIdx.y, jz = blockIdx.z;
-  if (jx >= cnx) return;
-  T s0, s1, s2;
-  restrict_even_at(jx, jy, jz, fnx, fny, fnz, rf, s0, s1, s2);
-  const int64_t J = jx + (int64_t)cnx * (jy + (int64_t)cny * jz);
-  if (cp_ptr) {   // split copies restricting into J, in ascending copy order
-    for (int e = cp_ptr[J]; e < cp_ptr[J + 1]; ++e) {
-      const int64_t f = fnnode + cp_copy[e];
-      const T w = T(cp_w[e]);
-      s0 += w * rf[3 * f]; s1 += w * rf[3 * f + 1]; s2 += w * rf[3 * f + 2];
-    }
-  }
-  rc[3 * J] = s0; rc[3 * J + 1] = s1; rc[3 * J + 2] = s2;
-}
-
-// x_f += P x_c on used fine nodes for even coarsening: per axis an even fine node takes its coarse node, an odd
-// one the mean of its two neighbours
-// even coarsening: the interpolated coarse value at fine grid position (pi, pj, pk)
-template <typename T>
-__device__ __forceinline__ void even_interp(int cnx, int cny, int pi, int pj, int pk, const T* xc,
-                                            T& s0, T& s1, T& s2) {
-  const int ni = (pi & 1) + 1, nj = (pj & 1) + 1, nk = (pk & 1) + 1;
-  const T wi = T(ni == 2 ? 0.5 : 1.0), wj = T(nj == 2 ? 0.5 : 1.0), wk = T(nk == 2 ? 0.5 : 1.0);
-  s0 = 0; s1 = 0; s2 = 0;
-  for (int c = 0; c < nk; ++c)
-    for (int b = 0; b < nj; ++b)
-      for (int a = 0; a < ni; ++a) {
-        const int64_t K = (pi >> 1) + a + (int64_t)cnx * ((pj >> 1) + b + (int64_t)cny * ((pk >> 1) + c));
-        const T w = wi * wj * wk;
-        s0 += w * xc[3 * K]; s1 += w * xc[3 * K + 1]; s2 += w * xc[3 * K + 2];
+      for (int a = 0; a < 2; ++a) {
+        const T* x = xc + 3 * ((int64_t)J[0][a] + (int64_t)cnx * (J[1][b] + (int64_t)cny * J[2][c]));
+        const T v = T(w[0][a] * w[1][b] * w[2][c]);
+        s0 += v * x[0]; s1 += v * x[1]; s2 += v * x[2];
       }
 }
 
-// x_f += P x_c for even coarsening; grid (x blocks of 64, fny, fnz + extra): the z layers past fnz take the
-// split copies (ids fnnode .. fnnode + ncopy), which receive their grid position's value
-template <typename T>
-__global__ void k_prolong_even(int cnx, int cny, int fnx, int fny, int fnz, const uint8_t* __restrict__ used,
-                               const T* __restrict__ xc, T* __restrict__ xf, const int* __restrict__ skip,
-                               TermAcc<T> acc, int64_t fnnode, int64_t ncopy, const int* __restrict__ orig_copy) {
+// x_f += P x_c on the used fine nodes, a thread each, and the split copies (which take their grid position's value) after them.
+// All loads are independent of branches, as in the restriction.  Mean over the levels, before and after: 24x18x16 4.3 -> 2.7 us
+// (FP32), 160x112x96 11.1 -> 9.4 us (FP32), 64x45x38 (odd, FP64) 6.0 + 4.8 (copies) -> 3.5 us.  A thread per 2 x 2 x 2 fine
+// nodes, which shares the coarse loads, took 12.4 us at the largest.
+template <typename T, bool EVEN>
+__global__ void __launch_bounds__(128)
+k_prolong(TransferDev P, const uint8_t* __restrict__ used, const T* __restrict__ xc, T* __restrict__ xf,
+          const int* __restrict__ skip, TermAcc<T> acc, int64_t ncopy, const int* __restrict__ orig_copy) {
   if (skip && *skip) return;
-  if ((int)blockIdx.z >= fnz) {
-    const int64_t c = ((int64_t)(blockIdx.z - fnz) * gridDim.y + blockIdx.y) * ((int64_t)gridDim.x * blockDim.x) +
-                      blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int fnx = P.ax[0].nf, fny = P.ax[1].nf, fnz = P.ax[2].nf, grid = fnx * fny * fnz, e = blockIdx.x * 128 + threadIdx.x;
+  if (e >= grid) {
+    const int c = e - grid;
     if (c >= ncopy) return;
     const int o = orig_copy[c];
-    const int pi = o % fnx, pj = (o / fnx) % fny, pk = o / (fnx * fny);
     T s0, s1, s2;
-    even_interp(cnx, cny, pi, pj, pk, xc, s0, s1, s2);
-    const int64_t n = fnnode + c;
-    xf[3 * n] += s0; xf[3 * n + 1] += s1; xf[3 * n + 2] += s2;
+    prolong_at<T, EVEN>(P, o % fnx, (o / fnx) % fny, o / (fnx * fny), xc, s0, s1, s2);
+    T* x = xf + 3 * ((int64_t)fnx * fny * fnz + c);
+    x[0] += s0; x[1] += s1; x[2] += s2;
     return;
   }
-  const int pi = blockIdx.x * blockDim.x + threadIdx.x, pj = blockIdx.y, pk = blockIdx.z;
-  if (pi >= fnx) return;
-  const int64_t n = pi + (int64_t)fnx * (pj + (int64_t)fny * pk);
-  if (!used[n]) return;
+  const bool on = used[e];
   T s0, s1, s2;
-  even_interp(cnx, cny, pi, pj, pk, xc, s0, s1, s2);
-  xf[3 * n] += s0; xf[3 * n + 1] += s1; xf[3 * n + 2] += s2;
-  term_acc(acc, n, s0, s1, s2);
-}
-
-template <typename T>
-__global__ void k_restrict_copies(TransferDev P, int fnx, int fny, int64_t fnnode, int64_t fntotal,
-                                  const int* __restrict__ orig_copy, const T* __restrict__ rf, T* __restrict__ rc,
-                                  const int* __restrict__ skip) {
-  if (skip && *skip) return;
-  int64_t e = fnnode + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (e >= fntotal) return;
-  const int o = orig_copy[e - fnnode];
-  const int pi = o % fnx, pj = (o / fnx) % fny, pk = o / (fnx * fny);
-  int Jx[2], Jy[2], Jz[2];
-  double wx[2], wy[2], wz[2];
-  int nxs = axis_support(P.ax[0], pi, Jx, wx), nys = axis_support(P.ax[1], pj, Jy, wy),
-      nzs = axis_support(P.ax[2], pk, Jz, wz);
-  const int cnx = P.ax[0].nc, cny = P.ax[1].nc;
-  for (int c = 0; c < nzs; ++c)
-    for (int b = 0; b < nys; ++b)
-      for (int a = 0; a < nxs; ++a) {
-        int64_t K = Jx[a] + (int64_t)cnx * (Jy[b] + (int64_t)cny * Jz[c]);
-        T w = T(wx[a] * wy[b] * wz[c]);
-        for (int q = 0; q < 3; ++q) atomic_add(rc + 3 * K + q, w * rf[3 * e + q]);
-      }
-}
-
-template <typename T>
-__device__ __forceinline__ void prolong_at(const TransferDev& P, int pi, int pj, int pk, const T* xc,
-                                           T& s0, T& s1, T& s2) {
-  int Jx[2], Jy[2], Jz[2];
-  double wx[2], wy[2], wz[2];
-  int nxs = axis_support(P.ax[0], pi, Jx, wx), nys = axis_support(P.ax[1], pj, Jy, wy),
-      nzs = axis_support(P.ax[2], pk, Jz, wz);
-  const int cnx = P.ax[0].nc, cny = P.ax[1].nc;
-  s0 = s1 = s2 = T(0);
-  for (int c = 0; c < nzs; ++c)
-    for (int b = 0; b < nys; ++b)
-      for (int a = 0; a < nxs; ++a) {
-        int64_t K = Jx[a] + (int64_t)cnx * (Jy[b] + (int64_t)cny * Jz[c]);
-        T w = T(wx[a] * wy[b] * wz[c]);
-        s0 += w * xc[3 * K]; s1 += w * xc[3 * K + 1]; s2 += w * xc[3 * K + 2];
-      }
-}
-
-template <typename T>
-__global__ void k_prolong_grid(TransferDev P, int fnx, int fny, const uint8_t* __restrict__ used,
-                               const T* __restrict__ xc, T* __restrict__ xf, const int* __restrict__ skip,
-                               TermAcc<T> acc) {
-  if (skip && *skip) return;
-  const int pi = blockIdx.x * blockDim.x + threadIdx.x, pj = blockIdx.y, pk = blockIdx.z;
-  if (pi >= fnx) return;
-  const int64_t n = pi + (int64_t)fnx * (pj + (int64_t)fny * pk);
-  if (!used[n]) return;
-  T s0, s1, s2;
-  prolong_at(P, pi, pj, pk, xc, s0, s1, s2);
-  xf[3 * n] += s0; xf[3 * n + 1] += s1; xf[3 * n + 2] += s2;
-  term_acc(acc, n, s0, s1, s2);
-}
-
-template <typename T>
-__global__ void k_prolong_copies(TransferDev P, int fnx, int fny, int64_t fnnode, int64_t fntotal,
-                                 const int* __restrict__ orig_copy, const T* __restrict__ xc, T* __restrict__ xf,
-                                 const int* __restrict__ skip) {
-  if (skip && *skip) return;
-  int64_t n = fnnode + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (n >= fntotal) return;
-  const int o = orig_copy[n - fnnode];
-  const int pi = o % fnx, pj = (o / fnx) % fny, pk = o / (fnx * fny);
-  T s0, s1, s2;
-  prolong_at(P, pi, pj, pk, xc, s0, s1, s2);
-  xf[3 * n] += s0; xf[3 * n + 1] += s1; xf[3 * n + 2] += s2;
+  prolong_at<T, EVEN>(P, e % fnx, (e / fnx) % fny, e / (fnx * fny), xc, s0, s1, s2);
+  T* x = xf + 3 * (int64_t)e;
+  const T x0 = x[0], x1 = x[1], x2 = x[2];
+  if (!on) return;
+  x[0] = x0 + s0; x[1] = x1 + s1; x[2] = x2 + s2;
+  term_acc(acc, e, s0, s1, s2);
 }
 
 __global__ void k_kept_mask(TransferDev P, const uint8_t* __restrict__ used_f, uint8_t* __restrict__ kept_c) {
@@ -1058,41 +977,23 @@ void launch_csr_add(int nrow, const int* row_dof, const int* row_ptr, const int*
 }
 
 template <typename T>
-void launch_restrict(const TransferDev& P, int fnx, int fny, int fnz, int64_t fnnode, int64_t fntotal,
-                     const int* orig_copy, const T* rf, T* rc, const int* skip, cudaStream_t s, T* zero, int nzero) {
+void launch_restrict(const TransferDev& P, int64_t fnnode, const T* rf, T* rc, const int* skip, cudaStream_t s, T* zero,
+                     int nzero) {
   if (!zero) nzero = 0;
-  if (P.even) {
-    k_restrict_even<T><<<dim3(div_up(P.ax[0].nc, 64), P.ax[1].nc, P.ax[2].nc), 64, 0, s>>>(
-        P.ax[0].nc, P.ax[1].nc, fnx, fny, fnz, rf, rc, skip, zero, nzero, P.cp_ptr, P.cp_copy, P.cp_w, fnnode);
-    note_launch();
-    if (P.cp_ptr) return;   // the copies were gathered
-  } else {
-    k_restrict_grid<T><<<dim3(div_up(P.ax[0].nc, 64), P.ax[1].nc, P.ax[2].nc), 64, 0, s>>>(P, fnx, fny, rf, rc, skip,
-                                                                                         zero, nzero); note_launch();
-  }
-  if (fntotal > fnnode)
-    k_restrict_copies<T><<<div_up(fntotal - fnnode, kThreads), kThreads, 0, s>>>(P, fnx, fny, fnnode, fntotal,
-                                                                                 orig_copy, rf, rc, skip); note_launch();
-  (void)fnz;
+  const int g = div_up((int64_t)P.ax[0].nc * P.ax[1].nc * P.ax[2].nc, 128);
+  if (P.even) k_restrict<T, true><<<g, 128, 0, s>>>(P, rf, rc, skip, zero, nzero, fnnode);
+  else k_restrict<T, false><<<g, 128, 0, s>>>(P, rf, rc, skip, zero, nzero, fnnode);
+  note_launch();
 }
 
 template <typename T>
-void launch_prolong_add(const TransferDev& P, int fnx, int fny, int fnz, int64_t fnnode, int64_t fntotal,
-                        const int* orig_copy, const uint8_t* used, const T* xc, T* xf, const int* skip,
-                        cudaStream_t s, const TermAcc<T>& acc) {
-  if (P.even) {   // the copies ride in extra z layers of the same launch
-    const int64_t ncopy = fntotal - fnnode, layer = (int64_t)div_up(fnx, 64) * 64 * fny;
-    const int extra = (int)((ncopy + layer - 1) / layer);
-    k_prolong_even<T><<<dim3(div_up(fnx, 64), fny, fnz + extra), 64, 0, s>>>(
-        P.ax[0].nc, P.ax[1].nc, fnx, fny, fnz, used, xc, xf, skip, acc, fnnode, ncopy, orig_copy); note_launch();
-    return;
-  } else {
-    k_prolong_grid<T><<<dim3(div_up(fnx, 64), fny, fnz), 64, 0, s>>>(P, fnx, fny, used, xc, xf, skip, acc); note_launch();
-  }
-  if (fntotal > fnnode) {
-    k_prolong_copies<T><<<div_up(fntotal - fnnode, kThreads), kThreads, 0, s>>>(P, fnx, fny, fnnode, fntotal,
-                                                                               orig_copy, xc, xf, skip); note_launch();
-  }
+void launch_prolong_add(const TransferDev& P, int64_t fnnode, int64_t fntotal, const int* orig_copy, const uint8_t* used,
+                        const T* xc, T* xf, const int* skip, cudaStream_t s, const TermAcc<T>& acc) {
+  const int64_t ncopy = fntotal - fnnode;
+  const int g = div_up(fntotal, 128);
+  if (P.even) k_prolong<T, true><<<g, 128, 0, s>>>(P, used, xc, xf, skip, acc, ncopy, orig_copy);
+  else k_prolong<T, false><<<g, 128, 0, s>>>(P, used, xc, xf, skip, acc, ncopy, orig_copy);
+  note_launch();
 }
 
 void launch_kept_mask(const TransferDev& P, const uint8_t* used_f, uint8_t* kept_c, cudaStream_t s) {
@@ -1175,16 +1076,13 @@ template void launch_csr_add<float>(int, const int*, const int*, const int*, con
                                     const int*, cudaStream_t);
 template void launch_csr_add<double>(int, const int*, const int*, const int*, const double*, const double*, double*,
                                      const int*, cudaStream_t);
-template void launch_restrict<float>(const TransferDev&, int, int, int, int64_t, int64_t, const int*, const float*,
-                                     float*, const int*, cudaStream_t, float*, int);
-template void launch_restrict<double>(const TransferDev&, int, int, int, int64_t, int64_t, const int*, const double*,
-                                      double*, const int*, cudaStream_t, double*, int);
-template void launch_prolong_add<float>(const TransferDev&, int, int, int, int64_t, int64_t, const int*,
-                                        const uint8_t*, const float*, float*, const int*, cudaStream_t,
-                                        const TermAcc<float>&);
-template void launch_prolong_add<double>(const TransferDev&, int, int, int, int64_t, int64_t, const int*,
-                                         const uint8_t*, const double*, double*, const int*, cudaStream_t,
-                                         const TermAcc<double>&);
+template void launch_restrict<float>(const TransferDev&, int64_t, const float*, float*, const int*, cudaStream_t, float*, int);
+template void launch_restrict<double>(const TransferDev&, int64_t, const double*, double*, const int*, cudaStream_t, double*,
+                                      int);
+template void launch_prolong_add<float>(const TransferDev&, int64_t, int64_t, const int*, const uint8_t*, const float*, float*,
+                                        const int*, cudaStream_t, const TermAcc<float>&);
+template void launch_prolong_add<double>(const TransferDev&, int64_t, int64_t, const int*, const uint8_t*, const double*,
+                                         double*, const int*, cudaStream_t, const TermAcc<double>&);
 template void launch_galerkin_cells<MAT_ISO_SRI>(const FineView<double>&, const double*, const TransferDev&, double*,
                                                  double*, int, int, int, cudaStream_t);
 template void launch_galerkin_cells<MAT_ISO_FULL>(const FineView<double>&, const double*, const TransferDev&, double*,

@@ -15,6 +15,7 @@ struct AxisDev {
   const int* ca; const int* cb;    // per fine node: coarse neighbours a <= b (a == b for coincident nodes)
   const double* wa; const double* wb;
   const int* cidx;                 // per coarse node: fine node index
+  const double* fan;               // per coarse node: weights of the fine nodes cidx - 1, cidx, cidx + 1 (0: none)
   const int* iv_first;             // per coarse interval [J, J+1]: first fine cell
   const int* iv_count;             //   and number of fine cells (1 or 2)
 };
@@ -23,8 +24,8 @@ struct TransferDev {
   AxisDev ax[3];
   int even = 0;   // 1: every axis coarsens 2 n - 1 -> n nodes with weights 1 and 1/2 (uniform spacing, even cell
                   // counts); the transfers then index directly instead of reading the axis tables
-  // even coarsening of a level with split copies: per coarse node J the copies that restrict into it,
-  // entries cp_ptr[J] .. cp_ptr[J+1] of (copy index, weight), so that the restriction gathers them (no atomics)
+  // level with split copies: per coarse node J the copies that restrict into it, entries cp_ptr[J] .. cp_ptr[J+1] of
+  // (copy index, weight), so that the restriction gathers them (no atomics)
   const int* cp_ptr = nullptr;
   const int* cp_copy = nullptr;
   const double* cp_w = nullptr;
@@ -114,19 +115,17 @@ template <typename T>
 void launch_csr_add(int nrow, const int* row_dof, const int* row_ptr, const int* col, const T* val, const T* u, T* y,
                     const int* skip, cudaStream_t s);
 
-// r_c = P^T r_f.  Fine level given by its grid dims; copies (ids >= nnode) are folded through `orig`.
+// r_c = P^T r_f, split copies (ids from fnnode on) included.
 // zero[0 .. nzero): cleared by the same launch (the coarse level's term-dot buffers of this V-cycle).
 template <typename T>
-void launch_restrict(const TransferDev& P, int fnx, int fny, int fnz, int64_t fnnode, int64_t fntotal,
-                     const int* orig_copy, const T* rf, T* rc, const int* skip, cudaStream_t s, T* zero = nullptr,
+void launch_restrict(const TransferDev& P, int64_t fnnode, const T* rf, T* rc, const int* skip, cudaStream_t s, T* zero = nullptr,
                      int nzero = 0);
 
 // x_f += P x_c on used fine nodes (copies take their grid node's value).
 // acc: the term dots of the added P x_c (the fine level's iterate changes by it) are accumulated
 template <typename T>
-void launch_prolong_add(const TransferDev& P, int fnx, int fny, int fnz, int64_t fnnode, int64_t fntotal,
-                        const int* orig_copy, const uint8_t* used, const T* xc, T* xf, const int* skip,
-                        cudaStream_t s, const TermAcc<T>& acc = TermAcc<T>());
+void launch_prolong_add(const TransferDev& P, int64_t fnnode, int64_t fntotal, const int* orig_copy, const uint8_t* used,
+                        const T* xc, T* xf, const int* skip, cudaStream_t s, const TermAcc<T>& acc = TermAcc<T>());
 
 // One axis pass of the separable Galerkin product P^T A P of a [243][n] stencil: axis d of the input grid
 // (inx, iny, inz) coarsened by ax to the output grid (onx, ony, onz).

@@ -1244,10 +1244,10 @@ struct FebHandle {
       A.r_in = (deg == 1) ? b : r; A.r_out = r;
       pair_run<T>(d, nullptr, &A, skip);
     }
-    launch_restrict<T>(V.P, V.nx, V.ny, V.nz, V.nnode, V.ntotal, orig_copy, r, vb<T>(C), skip, s, tdb<T>(C),
+    launch_restrict<T>(V.P, V.nnode, r, vb<T>(C), skip, s, tdb<T>(C),
                        kTermDotBufs * C.nterms);
     vcycle<T>(1, vb<T>(C), vx<T>(C), skip);
-    launch_prolong_add<T>(V.P, V.nx, V.ny, V.nz, V.nnode, V.ntotal, orig_copy, V.used, vx<T>(C), xs, skip, s);
+    launch_prolong_add<T>(V.P, V.nnode, V.ntotal, orig_copy, V.used, vx<T>(C), xs, skip, s);
     base = xs;
     for (int k = 0; k < deg; ++k) {     // e holds the direction before last, or nothing: the new one may replace it
       const bool last = k == deg - 1;
@@ -1280,10 +1280,10 @@ struct FebHandle {
       apply<T>(l, x, t, skip);
       launch_residual<T>(b, t, r, 3 * V.ntotal, skip, s);
     }
-    launch_restrict<T>(V.P, V.nx, V.ny, V.nz, V.nnode, V.ntotal, orig_copy, r, vb<T>(C), skip, s, tdb<T>(C),
+    launch_restrict<T>(V.P, V.nnode, r, vb<T>(C), skip, s, tdb<T>(C),
                        kTermDotBufs * C.nterms);
     vcycle<T>(l + 1, vb<T>(C), vx<T>(C), skip);
-    launch_prolong_add<T>(V.P, V.nx, V.ny, V.nz, V.nnode, V.ntotal, orig_copy, V.used, vx<T>(C), x, skip, s,
+    launch_prolong_add<T>(V.P, V.nnode, V.ntotal, orig_copy, V.used, vx<T>(C), x, skip, s,
                           term_acc<T>(V, nullptr, tdx));
     smooth<T>(l, b, x, false, skip);
   }
@@ -1541,14 +1541,25 @@ int upload_transfer(Pool& pool, Level& V) {
     double *wa, *wb;
     FEB_TRY(pool.upload(&ca, A.ca.data(), A.ca.size()));
     FEB_TRY(pool.upload(&cb, A.cb.data(), A.cb.size()));
-    FEB_TRY(pool.upload(&wa, A.wa.data(), A.wa.size()));
+    // wa, then per coarse node the weights of the fine nodes around its own
+    std::vector<double> waf(A.wa);
+    for (int J = 0; J < A.nc; ++J)
+      for (int i = A.cidx[J] - 1; i <= A.cidx[J] + 1; ++i) {
+        double w = 0.0;
+        if (i >= 0 && i < A.nf) {
+          if (A.ca[i] == J) w += A.wa[i];
+          if (A.cb[i] == J) w += A.wb[i];
+        }
+        waf.push_back(w);
+      }
+    FEB_TRY(pool.upload(&wa, waf.data(), waf.size()));
     FEB_TRY(pool.upload(&wb, A.wb.data(), A.wb.size()));
     FEB_TRY(pool.upload(&cidx, A.cidx.data(), A.cidx.size()));
     std::vector<int> f(A.iv_first), c(A.iv_count);
     if (f.empty()) { f.push_back(0); c.push_back(0); }
     FEB_TRY(pool.upload(&ivf, f.data(), f.size()));
     FEB_TRY(pool.upload(&ivc, c.data(), c.size()));
-    D.ca = ca; D.cb = cb; D.wa = wa; D.wb = wb; D.cidx = cidx; D.iv_first = ivf; D.iv_count = ivc;
+    D.ca = ca; D.cb = cb; D.wa = wa; D.wb = wb; D.cidx = cidx; D.fan = wa + A.wa.size(); D.iv_first = ivf; D.iv_count = ivc;
   }
   // even coarsening on every axis: 2 nc - 1 fine nodes, odd fine nodes halfway between their coarse neighbours
   bool even = true;
@@ -1565,20 +1576,28 @@ int upload_transfer(Pool& pool, Level& V) {
   return FEB_OK;
 }
 
-// the split copies' restriction as a gather per coarse node (even coarsening): copy c sits at fine grid
-// position orig_copy[c] and restricts with the weights of that position
+// the split copies' restriction as a gather per coarse node: copy c sits at fine grid position orig_copy[c] and restricts
+// with the weights of that position
 int upload_copy_gather(Pool& pool, Level& V, const std::vector<int64_t>& orig_copy) {
-  if (!V.P.even || orig_copy.empty()) return FEB_OK;
+  if (orig_copy.empty()) return FEB_OK;
   const int fnx = V.nx, fny = V.ny, cnx = V.ax[0].nc, cny = V.ax[1].nc, cnz = V.ax[2].nc;
   const int64_t nc = (int64_t)cnx * cny * cnz;
   std::vector<int> cnt(nc + 1, 0);
   auto each = [&](int64_t o, auto&& f) {
-    const int pi = int(o % fnx), pj = int((o / fnx) % fny), pk = int(o / ((int64_t)fnx * fny));
-    const int ni = (pi & 1) + 1, nj = (pj & 1) + 1, nk = (pk & 1) + 1;
-    const double w = (ni == 2 ? 0.5 : 1.0) * (nj == 2 ? 0.5 : 1.0) * (nk == 2 ? 0.5 : 1.0);
-    for (int c = 0; c < nk; ++c)
-      for (int b = 0; b < nj; ++b)
-        for (int a = 0; a < ni; ++a) f((pi >> 1) + a + (int64_t)cnx * ((pj >> 1) + b + (int64_t)cny * ((pk >> 1) + c)), w);
+    const int p[3] = {int(o % fnx), int((o / fnx) % fny), int(o / ((int64_t)fnx * fny))};
+    int n[3], J[3][2];
+    double w[3][2];
+    for (int d = 0; d < 3; ++d) {       // the coarse nodes with a weight, as in the device code
+      const AxisHost& A = V.ax[d];
+      const int i = p[d];
+      n[d] = 0;
+      if (A.wa[i] != 0.0) { J[d][n[d]] = A.ca[i]; w[d][n[d]++] = V.P.even ? (i % 2 ? 0.5 : 1.0) : A.wa[i]; }
+      if (A.cb[i] != A.ca[i] && A.wb[i] != 0.0) { J[d][n[d]] = A.cb[i]; w[d][n[d]++] = V.P.even ? 0.5 : A.wb[i]; }
+    }
+    for (int c = 0; c < n[2]; ++c)
+      for (int b = 0; b < n[1]; ++b)
+        for (int a = 0; a < n[0]; ++a)
+          f(J[0][a] + (int64_t)cnx * (J[1][b] + (int64_t)cny * J[2][c]), w[0][a] * w[1][b] * w[2][c]);
   };
   for (size_t c = 0; c < orig_copy.size(); ++c) each(orig_copy[c], [&](int64_t J, double) { cnt[J + 1]++; });
   for (int64_t J = 0; J < nc; ++J) cnt[J + 1] += cnt[J];
