@@ -176,13 +176,14 @@ k_prolong(TransferDev P, const uint8_t* __restrict__ used, const T* __restrict__
     return;
   }
   const bool on = used[e];
+  const TermBounds tb = term_bounds(acc, e);
   T s0, s1, s2;
   prolong_at<T, EVEN>(P, e % fnx, (e / fnx) % fny, e / (fnx * fny), xc, s0, s1, s2);
   T* x = xf + 3 * (int64_t)e;
   const T x0 = x[0], x1 = x[1], x2 = x[2];
   if (!on) return;
   x[0] = x0 + s0; x[1] = x1 + s1; x[2] = x2 + s2;
-  term_acc(acc, e, s0, s1, s2);
+  term_acc(acc, tb, s0, s1, s2);
 }
 
 __global__ void k_kept_mask(TransferDev P, const uint8_t* __restrict__ used_f, uint8_t* __restrict__ kept_c) {
@@ -708,19 +709,31 @@ __device__ __forceinline__ void sym_slot(const SymView<T>& L, const T* u, int n,
   sym_acc<T, Q>(v, a0, a1, a2);
 }
 
+// Bounds of a node's entries that the stencil cannot hold and of its rank-1 terms.
+struct SymExtra {
+  int beg = 0, end = 0;
+  TermBounds terms;
+};
+
 // One 32-node tile of the product: node n (lane's, clamped to the row; pn its padded position) and the share of warp w of 4
 // of its sum, without the epilogue.  CMP: the level carries the compressed single-material blocks (tags; patterns sp, sm in
 // shared memory); without them the pattern code is not compiled into the kernel at all.  Offsets within the stencil planes
 // are 32-bit (126 x the padded node count < 2^31 is checked at launch).  H (with CT, FP32): the stored blocks are read
 // from the 16-bit copy Sh and the slot sums scaled by hscale before the entries and terms are added.
 template <typename T, bool CMP, bool CT, bool H>
-__device__ __forceinline__ void sym_product(const SymView<T>& L, const T* u, int n, int pn, int ic, int j, int k, bool valid,
+__device__ __forceinline__ void sym_product(const SymView<T>& L, const T* u, int n, int pn, int ic, int j, int k, bool valid, SymExtra& ex,
                                             int lane, int w, const T* sp, const T* sm, T& a0, T& a1, T& a2) {
   const int nx = L.nx, ny = L.ny, nz = L.nz;
   const int nxp = L.nxp, NP = (int)L.np;          // row-padded stencil planes
   int tn = 0;
   if constexpr (CMP) tn = L.tag[n];
   a0 = a1 = a2 = T(0);
+  // FP64 loads them half-way through the blocks.  The 16-bit variant does not, and is held to 48 registers: with 56, a large
+  // level loses the tenth resident CTA (160 x 112 x 96, level 2: 8.8 against 7.8 us).
+  auto bounds = [&]() {
+    if (L.node_ptr && valid) { ex.beg = L.node_ptr[n]; ex.end = L.node_ptr[n + 1]; }
+    if (L.tn_ptr && valid) { ex.terms.p = L.tn_ptr[n]; ex.terms.pe = L.tn_ptr[n + 1]; }
+  };
   if constexpr (CT) {
     // the 14 slots over the 4 warps (warp-uniform switch): 0 4 8 12 | 1 5 9 13 | 2 6 10 | 3 7 11
 #define FEB_SLOT(Q) sym_slot<T, CMP, H, Q>(L, u, n, pn, ic, j, k, tn, sp, sm, a0, a1, a2)
@@ -731,6 +744,7 @@ __device__ __forceinline__ void sym_product(const SymView<T>& L, const T* u, int
       default: FEB_SLOT(3); FEB_SLOT(7); FEB_SLOT(11); break;
     }
 #undef FEB_SLOT
+    bounds();
     if constexpr (H) {
       const T sc = T(*L.hscale);
       a0 *= sc; a1 *= sc; a2 *= sc;
@@ -740,6 +754,7 @@ __device__ __forceinline__ void sym_product(const SymView<T>& L, const T* u, int
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
       const int q = w + 4 * t;
+      if (t == 2) bounds();
       if (q > 13) break;                                     // warp-uniform (t == 3, w >= 2)
       const int o = 13 + q;
       const int dx = o % 3 - 1, dy = (o / 3) % 3 - 1, dz = o / 9 - 1;
@@ -776,13 +791,11 @@ __device__ __forceinline__ void sym_product(const SymView<T>& L, const T* u, int
     }
   }
   if (L.node_ptr) {
-    int beg = 0, end = 0;
-    if (valid) { beg = L.node_ptr[n]; end = L.node_ptr[n + 1]; }
-    unsigned todo = __ballot_sync(0xffffffffu, end > beg) & (0x11111111u << w);
+    unsigned todo = __ballot_sync(0xffffffffu, ex.end > ex.beg) & (0x11111111u << w);
     while (todo) {
       const int src = __ffs(todo) - 1;
       todo &= todo - 1;
-      const int b0 = __shfl_sync(0xffffffffu, beg, src), b1 = __shfl_sync(0xffffffffu, end, src);
+      const int b0 = __shfl_sync(0xffffffffu, ex.beg, src), b1 = __shfl_sync(0xffffffffu, ex.end, src);
       T s0 = 0, s1 = 0, s2 = 0;
       for (int e = b0 + lane; e < b1; e += 32) {
         const T v = L.ent_v[e] * u[L.ent_col[e]];
@@ -795,14 +808,21 @@ __device__ __forceinline__ void sym_product(const SymView<T>& L, const T* u, int
       if (lane == src) { a0 += s0; a1 += s1; a2 += s2; }
     }
   }
-  if (L.tn_ptr && valid) {   // rank-1 terms: the term's dot lam_t v_t.u comes from k_term_dots; the node's
-                             // pairs are split over the 4 warps
-    const int pe = L.tn_ptr[n + 1];
-    for (int p = L.tn_ptr[n] + w; p < pe; p += 4) {
-      const T dot = L.tdot[L.tn_term[p]];
-      a0 += dot * L.tn_coef[3 * p];
-      a1 += dot * L.tn_coef[3 * p + 1];
-      a2 += dot * L.tn_coef[3 * p + 2];
+  // rank-1 terms: the term's dot lam_t v_t.u comes from k_term_dots or the writer of u; the node's pairs are split over the 4
+  // warps, and four pairs' loads go out together
+  for (int p = ex.terms.p + w; p < ex.terms.pe; p += 16) {
+    int q[4];
+    T dot[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) q[t] = min(p + 4 * t, ex.terms.pe - 1);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) dot[t] = L.tdot[L.tn_term[q[t]]];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      if (p + 4 * t >= ex.terms.pe) break;
+      a0 += dot[t] * L.tn_coef[3 * q[t]];
+      a1 += dot[t] * L.tn_coef[3 * q[t] + 1];
+      a2 += dot[t] * L.tn_coef[3 * q[t] + 2];
     }
   }
 }
@@ -829,7 +849,7 @@ struct SymOps {
 // Finishes component c of node n from the four warps' partial sums red[w][component][lane].
 template <typename T, int EPI>
 __device__ __forceinline__ void sym_finish(const SymOps<T, EPI>& o, const T (*red)[3][32], int lane, int n, int c, T* y, T* r,
-                                           T* d_out, T* x_out, const LevelParams* lp, int kstep, const TermAcc<T>& acc) {
+                                           T* d_out, T* x_out, const LevelParams* lp, int kstep, const TermAcc<T>& acc, const TermBounds& tb) {
   auto sum = [&](int q) { return red[0][q][lane] + red[1][q][lane] + red[2][q][lane] + red[3][q][lane]; };
   if constexpr (EPI == EPI_APPLY) {
     y[3 * n + c] = sum(c);
@@ -849,12 +869,12 @@ __device__ __forceinline__ void sym_finish(const SymOps<T, EPI>& o, const T (*re
     r[3 * n + c] = c == 0 ? r0 : (c == 1 ? r1 : r2);
     d_out[3 * n + c] = e;
     x_out[3 * n + c] = x;
-    term_acc1(acc, n, c, e);
+    term_acc1(acc, tb, c, e);
   }
 }
 
 template <typename T, int EPI, bool CMP, bool CT, bool H>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, H ? 10 : 1)   // 16-bit blocks: 48 registers, so that ten CTAs hide the blocks' latency
 k_sym(SymView<T> L, const T* __restrict__ u, T* __restrict__ y, const T* __restrict__ b, const T* r_in, T* r,
       T* __restrict__ d_out, const T* x_in, T* x_out, const LevelParams* __restrict__ lp, int kstep,
       const int* __restrict__ skip, TermAcc<T> acc) {
@@ -873,15 +893,16 @@ k_sym(SymView<T> L, const T* __restrict__ u, T* __restrict__ y, const T* __restr
   const bool valid = i < L.nx;
   const int ic = valid ? i : L.nx - 1;
   const int n = ic + L.nx * (j + L.ny * k), pn = ic + L.nxp * (j + L.ny * k);
+  SymExtra ex;
   T a0, a1, a2;
-  sym_product<T, CMP, CT, H>(L, u, n, pn, ic, j, k, valid, lane, w, CMP ? &spat[0][0] : nullptr, CMP ? &smat[0][0] : nullptr,
+  sym_product<T, CMP, CT, H>(L, u, n, pn, ic, j, k, valid, ex, lane, w, CMP ? &spat[0][0] : nullptr, CMP ? &smat[0][0] : nullptr,
                              a0, a1, a2);
   red[w][0][lane] = a0; red[w][1][lane] = a1; red[w][2][lane] = a2;
   // epilogue operands, read before the barrier (r is rewritten after it)
   SymOps<T, EPI> o;
   if (w < 3 && valid) o.load(L, n, w, u, b, r_in, x_in);
   __syncthreads();
-  if (w < 3 && valid) sym_finish<T, EPI>(o, red, lane, n, w, y, r, d_out, x_out, lp, kstep, acc);
+  if (w < 3 && valid) sym_finish<T, EPI>(o, red, lane, n, w, y, r, d_out, x_out, lp, kstep, acc, acc.tn_ptr ? ex.terms : TermBounds{});
 }
 
 }  // namespace

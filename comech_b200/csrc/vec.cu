@@ -223,6 +223,7 @@ __global__ void k_cheb_first(const T* __restrict__ b, T* __restrict__ r, T* __re
   if (skip && *skip) return;
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= nn) return;
+  const TermBounds tb = term_bounds(acc, i);
   const T c = T(lp->c_init);
   T r0 = b[3 * i], r1 = b[3 * i + 1], r2 = b[3 * i + 2], z0, z1, z2;
   bj(D, nn, i, r0, r1, r2, z0, z1, z2);
@@ -230,7 +231,7 @@ __global__ void k_cheb_first(const T* __restrict__ b, T* __restrict__ r, T* __re
   z0 *= c; z1 *= c; z2 *= c;
   d[3 * i] = z0; d[3 * i + 1] = z1; d[3 * i + 2] = z2;
   x[3 * i] = z0; x[3 * i + 1] = z1; x[3 * i + 2] = z2;
-  term_acc(acc, i, z0, z1, z2);
+  term_acc(acc, tb, z0, z1, z2);
 }
 
 template <typename T>
@@ -272,13 +273,14 @@ __global__ void k_cheb_from_r(const T* __restrict__ r, T* __restrict__ d, T* __r
   if (skip && *skip) return;
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= nn) return;
+  const TermBounds tb = term_bounds(acc, i);
   const T c = T(lp->c_init);
   T z0, z1, z2;
   bj(D, nn, i, r[3 * i], r[3 * i + 1], r[3 * i + 2], z0, z1, z2);
   z0 *= c; z1 *= c; z2 *= c;
   d[3 * i] = z0; d[3 * i + 1] = z1; d[3 * i + 2] = z2;
   x[3 * i] += z0; x[3 * i + 1] += z1; x[3 * i + 2] += z2;
-  term_acc(acc, i, z0, z1, z2);
+  term_acc(acc, tb, z0, z1, z2);
 }
 
 template <typename T>

@@ -30,28 +30,47 @@ struct TermAcc {
   T* dot_b = nullptr;
 };
 
+// bounds of a node's (node, term) pairs: loaded at a kernel's start, long before the delta is known
+struct TermBounds {
+  int p = 0, pe = 0;
+};
 template <typename T>
-__device__ __forceinline__ void term_acc(const TermAcc<T>& A, int64_t n, T v0, T v1, T v2) {
-  if (!A.tn_ptr) return;
-  const int pe = A.tn_ptr[n + 1];
-  for (int p = A.tn_ptr[n]; p < pe; ++p) {
-    const int t = A.tn_term[p];
-    const T c = A.t_lam[t] * (A.tn_coef[3 * p] * v0 + A.tn_coef[3 * p + 1] * v1 + A.tn_coef[3 * p + 2] * v2);
-    if (A.dot_a) atomicAdd(A.dot_a + t, c);
-    if (A.dot_b) atomicAdd(A.dot_b + t, c);
+__device__ __forceinline__ TermBounds term_bounds(const TermAcc<T>& A, int64_t n) {
+  TermBounds b;
+  if (A.tn_ptr) { b.p = A.tn_ptr[n]; b.pe = A.tn_ptr[n + 1]; }
+  return b;
+}
+// Pairs four at a time, so that their loads go out together: the atomics between them would keep one pair's loads behind the
+// pair before.  value(pair) is v_t . delta.
+template <typename T, typename F>
+__device__ __forceinline__ void term_add(const TermAcc<T>& A, const TermBounds& b, F value) {
+  for (int p = b.p; p < b.pe; p += 4) {
+    int t[4];
+    T c[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int pq = min(p + q, b.pe - 1);
+      t[q] = A.tn_term[pq];
+      c[q] = value(pq);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) c[q] *= A.t_lam[t[q]];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (p + q >= b.pe) break;
+      if (A.dot_a) atomicAdd(A.dot_a + t[q], c[q]);
+      if (A.dot_b) atomicAdd(A.dot_b + t[q], c[q]);
+    }
   }
+}
+template <typename T>
+__device__ __forceinline__ void term_acc(const TermAcc<T>& A, const TermBounds& b, T v0, T v1, T v2) {
+  term_add(A, b, [&](int p) { return A.tn_coef[3 * p] * v0 + A.tn_coef[3 * p + 1] * v1 + A.tn_coef[3 * p + 2] * v2; });
 }
 // one component `comp` of the node's delta (a kernel whose threads own single components)
 template <typename T>
-__device__ __forceinline__ void term_acc1(const TermAcc<T>& A, int64_t n, int comp, T v) {
-  if (!A.tn_ptr) return;
-  const int pe = A.tn_ptr[n + 1];
-  for (int p = A.tn_ptr[n]; p < pe; ++p) {
-    const int t = A.tn_term[p];
-    const T c = A.t_lam[t] * A.tn_coef[3 * p + comp] * v;
-    if (A.dot_a) atomicAdd(A.dot_a + t, c);
-    if (A.dot_b) atomicAdd(A.dot_b + t, c);
-  }
+__device__ __forceinline__ void term_acc1(const TermAcc<T>& A, const TermBounds& b, int comp, T v) {
+  term_add(A, b, [&](int p) { return A.tn_coef[3 * p + comp] * v; });
 }
 
 // Per-level smoother parameters written by the power iteration.
