@@ -306,25 +306,21 @@ def timed_steps(fn, steps, flush, dist=None, clocks=None, per_step=None):
     return ms, out
 
 
-def special_nodes(P, g):
-    """Grid nodes of the level-0 operator that receive a sparse contribution (ground springs, extra entries,
-    corners of cells touching split copies) plus the split copies: the nodes that go through the accumulator."""
+def irregular_cells(P, g):
+    """Number of active cells of the level-0 operator that touch split copies."""
     cells = np.flatnonzero(P["active"])
-    irr = cells[(P["cn"][cells] != g.cell_nodes[cells]).any(1)]
-    nr = P["extra"].node_coo()[0]
-    nodes = np.unique(np.concatenate([np.asarray(P["fixed"][0]), P["cn"][irr].ravel(), nr]))
-    return int(np.count_nonzero(nodes < g.nnode)) + (len(P["orig"]) - g.nnode), len(irr)
+    return int((P["cn"][cells] != g.cell_nodes[cells]).any(1).sum())
 
 
 def ku_roofline(P, d, lib, engine, _lib, pk, pk_kind):
-    """The level-0 operator (sparse pass + paired-row kernel) timed on a rotating set of operand buffers
+    """The level-0 operator (paired-row kernel with its row list) timed on a rotating set of operand buffers
     larger than L2, with its algorithmic bytes."""
     import ctypes as C
     import torch
     g = P["grid"]
     ntotal = len(P["orig"])
     nact = int(P["active"].sum())
-    n_spec, n_irr = special_nodes(P, g)
+    n_irr = irregular_cells(P, g)
     n_pen = len(P["fixed"][0])
     n_extra = P["extra"].node_coo()[4].size
     npair = (g.nx + 1) * ((g.ny + 1) // 2 + 1) * (g.nz + 1)
@@ -341,11 +337,9 @@ def ku_roofline(P, d, lib, engine, _lib, pk, pk_kind):
             ms = C.c_float()
             for nrep in (2 * nbuf, 20 * nbuf):
                 _lib.check(lib.feb_benchmark_apply_set(pr.h, 0 if sv == 8 else 1, nbuf, up, yp, nrep, C.byref(ms)))
-            # u, y; cell-pair words (2 bytes per pair of node rows); the sparse part: irregular cells (8 node ids +
-            # 2 material values), penalties (node + 3 values), extra entries (column + value), and the
-            # accumulator of the special nodes (atomic adds, then read and cleared by the owners)
-            alg = (6 * ntotal * sv + 2 * npair + n_irr * (32 + 2 * sv) + n_pen * (4 + 3 * sv) + n_extra * (8 + sv)
-                   + n_spec * 3 * sv * 3)
+            # u, y; cell-pair words (4 bytes per pair of node rows); the sparse part: irregular cells (8 node ids +
+            # 2 material values), penalties (node + 3 values), extra entries (column + value)
+            alg = 6 * ntotal * sv + 4 * npair + n_irr * (32 + 2 * sv) + n_pen * (4 + 3 * sv) + n_extra * (8 + sv)
             roof[name] = dict(ms=ms.value, bytes=alg, gbs=alg / (ms.value * 1e-3) / 1e9, nbuf=nbuf)
             del us, ys
     finally:
@@ -367,8 +361,7 @@ def ku_roofline(P, d, lib, engine, _lib, pk, pk_kind):
         # d read; r and x read and written; d' written; the 6-value symmetric block-Jacobi inverse; the K.u's
         # cell-pair words and sparse part as above
         sv = 4
-        alg_s = (24 * ntotal * sv + 2 * npair + n_irr * (32 + 2 * sv) + n_pen * (4 + 3 * sv) + n_extra * (8 + sv)
-                 + n_spec * 3 * sv * 3)
+        alg_s = 24 * ntotal * sv + 4 * npair + n_irr * (32 + 2 * sv) + n_pen * (4 + 3 * sv) + n_extra * (8 + sv)
         sm = dict(ms=ms.value, bytes=alg_s, gbs=alg_s / (ms.value * 1e-3) / 1e9, nbuf=nbuf)
         del sets
     finally:
@@ -376,7 +369,7 @@ def ku_roofline(P, d, lib, engine, _lib, pk, pk_kind):
     r32 = roof["fp32"]
     return {"bound": "hbm", "achieved": round(sm["gbs"], 1), "peak": pk, "unit": "GB/s",
             "frac": round(sm["gbs"] / pk, 4), "traffic": ku_traffic(SMOOTH_PROFILE),
-            "kernel": "level-0 smoother step FP32 (k_fine_sparse + k_fine_pair with the fused Chebyshev update), the "
+            "kernel": "level-0 smoother step FP32 (k_fine_pair with the Chebyshev update, fused or as k_pair_update), the "
                       "solve's largest share of device time; operands rotated over "
                       f"{sm['nbuf']} buffer sets (> L2)",
             "peak_kind": pk_kind, "ms_per_launch": round(sm["ms"], 4), "algorithmic_bytes": sm["bytes"],

@@ -3,8 +3,9 @@
 // Work split of one launch (a product y = K u, or one Chebyshev / residual step of the smoother):
 //   * tile CTAs compute the regular cells matrix-free.  A grid node whose 8 cells are all handled here (the bulk) is
 //     finished in registers: its product is stored, or the smoother update of that node runs on the spot (r -= K d,
-//     z = Dinv r, d' = a1 d + a2 z, x += d').  On large grids the update is a launch of its own (k_pair_update).  A node flagged "special" with a penalty spring adds its diagonal first; one
-//     that cells touching split copies or extra entries reach is left out (its row flag is set).
+//     z = Dinv r, d' = a1 d + a2 z, x += d').  On large grids the update is a launch of its own (k_pair_update).  A node
+//     with a penalty spring adds its diagonal first; one that cells touching split copies or extra entries reach is left
+//     out (the flags of the cell-pair words).
 //   * those nodes and the split copies (PairRows) are finished by groups of eight lanes, one cell each, spread over all
 //     CTAs: each does its few while its first planes are on their way.  There are not many (1 % of the nodes of a
 //     160 x 112 x 96 foot).  As a kernel of its own ahead of the tiles, summing cells with atomics into a vector that the
@@ -19,8 +20,8 @@
 // (forward) and below (backward), z in registers along the march.  On cubic cells with the SRI isotropic
 // model (the engine's voxel model, rb/splitfe.py:58-69) the modal core collapses to 27 pair operations
 // with 5 per-cell constants (see cube_sri_core); other materials and rectilinear grids run the general
-// modal core.  Cell materials are 7-bit ids into a table held in shared memory: one 16-bit load gives
-// the two cells of a thread's rows plus the "special" flags of its two nodes.
+// modal core.  Cell materials are 7-bit ids into a table held in shared memory: one 32-bit load gives
+// the two cells of a thread's rows plus the flags of its two nodes.
 #include <algorithm>
 
 #include "fine.cuh"

@@ -1927,7 +1927,7 @@ int setup_rows(FebHandle* h, const uint8_t* ids) {
 
 // Paired-row level-0 operator (fine_pair.cu): material ids of the regular cells (FEB_KU_PAIR=0 keeps the
 // per-cell kernels), flags of the grid nodes that receive sparse contributions, the cell-pair words, the
-// sparse accumulators and the symmetric level-0 block-Jacobi inverse.  Leaves pair_ok false when more than
+// row list and the symmetric level-0 block-Jacobi inverse.  Leaves pair_ok false when more than
 // kMaxMatIds - 1 distinct materials occur (or on a hash collision).
 template <int W>
 int setup_pair(FebHandle* h, const double* mat_s64) {
