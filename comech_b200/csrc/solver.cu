@@ -1232,7 +1232,8 @@ struct FebHandle {
       } else {
         ++late;
       }
-      pair_run<T>(u, x, &A, skip);   // x: where a split step leaves K u (the last one replaces it by the result)
+      // x: where a split step leaves K u (the last one replaces it by the result); a call in place keeps its b there
+      pair_run<T>(u, x == b ? nullptr : x, &A, skip);
     };
     launch_cheb_first6<T>(b, dinv6<T>(), lp, d, deg == 1 ? xs : nullptr, ntotal, skip, s);
     for (int k = 1; k < deg; ++k) {

@@ -85,5 +85,9 @@ def test_split_and_fused_steps_match_unfused(monkeypatch, precision, tol):
                     used = P.used_mask()[0].cpu().numpy().astype(bool)
                     r = (np.random.default_rng(degree).standard_normal((P.ntotal, 3)) * used[:, None]).ravel()
                 z[name] = P.precondition(torch.from_numpy(r).cuda()).cpu().numpy()
-        for name in ("fused", "split"):
+                if name != "unfused":                    # the same with the result in r's place
+                    p = torch.from_numpy(r).cuda()
+                    _lib.check(_lib.load().feb_precondition(P.h, p.data_ptr(), p.data_ptr()))
+                    z[name + ", in place"] = p.cpu().numpy()
+        for name in set(z) - {"unfused"}:
             assert np.linalg.norm(z[name] - z["unfused"]) <= tol * np.linalg.norm(z["unfused"]), (degree, name)
