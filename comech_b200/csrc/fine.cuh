@@ -123,8 +123,7 @@ int fine_pair_tiles_xy(int nxn, int nyn, int wy);
 template <int W>
 void launch_mat_ids(const double* mat_s, int64_t ncell, unsigned long long* keys, double* vals, uint8_t* ids,
                     int* status, cudaStream_t s);
-void launch_flag_nodes(const int* pen_node, int npen, const int* irr_nodes, int nirr, const int* row_dof, int nrow,
-                       int64_t nnode, uint8_t* flag, cudaStream_t s);
+void launch_flag_nodes(const FineView<double>& F, const int* orig_copy, uint8_t* flag, int* status, cudaStream_t s);
 // set-up of the row list: flags of its nodes (with the irregular cell of every cell and the first CSR row of every node's extra
 // entries, both preset to -1), the penalty diagonal, the rows (ids: material id of every regular cell)
 void launch_row_flags(const FineView<double>& F, uint8_t* flag, int* cmap, int* start, cudaStream_t s);

@@ -690,7 +690,7 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z) {   // splitmix64 finalise
 // Material id of every regular cell: open addressing over ids 1..kMaxMatIds-1 keyed by a 64-bit hash of the
 // cell's W FP64 values.  The first thread to claim a slot writes its values; k_pack_pairs then checks every
 // cell against the table (a hash collision or a full table sets the status word and the operator keeps the
-// per-cell kernel).
+// per-cell kernels).
 template <int W>
 __global__ void k_mat_ids(const double* __restrict__ mat_s, int64_t ncell, unsigned long long* __restrict__ keys,
                           double* __restrict__ vals, uint8_t* __restrict__ ids, int* __restrict__ status) {
@@ -792,13 +792,20 @@ __global__ void k_rows(FineView<double> F, const int* __restrict__ node, int nro
   ex[row] = x;
 }
 
-// grid nodes with a penalty (flag[n]) and grid nodes of the row list: extra entries, irregular cell corners (flag[nnode + n])
-__global__ void k_flag_nodes(const int* __restrict__ pen_node, int npen, const int* __restrict__ irr_nodes, int nirr,
-                             const int* __restrict__ row_dof, int nrow, int64_t nnode, uint8_t* __restrict__ flag) {
+// grid nodes with a penalty (flag[n]) and grid nodes of the row list: extra entries, irregular cell corners (flag[nnode + n]).
+// Connectivity in which a corner is neither the grid node there nor a copy of it sets the status word: a row finds the cells
+// of its node around the node's grid position (k_rows), so the list would lose that corner's force.
+__global__ void k_flag_nodes(FineView<double> F, const int* __restrict__ orig_copy, uint8_t* __restrict__ flag,
+                             int* __restrict__ status) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e < npen && pen_node[e] < nnode) flag[pen_node[e]] = 1;
-  if (e < 8 * nirr && irr_nodes[e] < nnode) flag[nnode + irr_nodes[e]] = 1;
-  if (e < nrow && row_dof[e] / 3 < nnode) flag[nnode + row_dof[e] / 3] = 1;
+  if (e < F.npen && F.pen_node[e] < F.nnode) flag[F.pen_node[e]] = 1;
+  if (e < 8 * F.nirr) {
+    const int n = F.irr_nodes[e], c = F.irr_cell[e >> 3], l = e & 7;
+    const int i = c % F.nx + (l & 1), j = (c / F.nx) % F.ny + ((l >> 1) & 1), k = c / (F.nx * F.ny) + (l >> 2);
+    if (n < F.nnode) flag[F.nnode + n] = 1;
+    if ((n < F.nnode ? n : orig_copy[n - F.nnode]) != i + F.nxn * (j + F.nyn * k)) atomicOr(status, 4);
+  }
+  if (e < F.nrow && F.row_dof[e] / 3 < F.nnode) flag[F.nnode + F.row_dof[e] / 3] = 1;
 }
 
 // cell-pair words [nzn][mp][nxn]: half h (h = 0, 1) describes row j = 2m - 1 + h: bits 0-6 the material id
@@ -928,11 +935,10 @@ void launch_mat_ids(const double* mat_s, int64_t ncell, unsigned long long* keys
                     int* status, cudaStream_t s) {
   k_mat_ids<W><<<div_up(ncell, kThreads), kThreads, 0, s>>>(mat_s, ncell, keys, vals, ids, status); note_launch();
 }
-void launch_flag_nodes(const int* pen_node, int npen, const int* irr_nodes, int nirr, const int* row_dof, int nrow,
-                       int64_t nnode, uint8_t* flag, cudaStream_t s) {
-  const int n = std::max(npen, std::max(8 * nirr, nrow));
+void launch_flag_nodes(const FineView<double>& F, const int* orig_copy, uint8_t* flag, int* status, cudaStream_t s) {
+  const int n = std::max(F.npen, std::max(8 * F.nirr, F.nrow));
   if (n > 0) {
-    k_flag_nodes<<<div_up(n, kThreads), kThreads, 0, s>>>(pen_node, npen, irr_nodes, nirr, row_dof, nrow, nnode, flag);
+    k_flag_nodes<<<div_up(n, kThreads), kThreads, 0, s>>>(F, orig_copy, flag, status);
     note_launch();
   }
 }

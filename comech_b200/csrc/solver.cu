@@ -1929,7 +1929,8 @@ int setup_rows(FebHandle* h, const uint8_t* ids) {
 // Paired-row level-0 operator (fine_pair.cu): material ids of the regular cells (FEB_KU_PAIR=0 keeps the
 // per-cell kernels), flags of the grid nodes that receive sparse contributions, the cell-pair words, the
 // row list and the symmetric level-0 block-Jacobi inverse.  Leaves pair_ok false when more than
-// kMaxMatIds - 1 distinct materials occur (or on a hash collision).
+// kMaxMatIds - 1 distinct materials occur (or on a hash collision), and for connectivity whose corners are not the grid
+// node there or a copy of it.
 template <int W>
 int setup_pair(FebHandle* h, const double* mat_s64) {
   FebHandle& H = *h;
@@ -1950,8 +1951,7 @@ int setup_pair(FebHandle* h, const double* mat_s64) {
   FEB_TRY(H.pool.zeros(&status, 1));
   FEB_TRY(H.pool.alloc(&cellpair, (size_t)nxn * mp * nzn));
   launch_mat_ids<W>(mat_s64, ncell, keys, vals, ids, status, H.s);
-  launch_flag_nodes(H.F64.pen_node, H.F64.npen, H.F64.irr_nodes, H.F64.nirr, H.F64.row_dof, H.F64.nrow, H.nnode, flag,
-                    H.s);
+  launch_flag_nodes(H.F64, H.orig_copy, flag, status, H.s);
   launch_pack_pairs<W>(H.nx, H.ny, H.nz, mp, ids, flag, mat_s64, vals, cellpair, status, H.s);
   FEB_CUDA(cudaGetLastError());
   int st = 0;

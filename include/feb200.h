@@ -61,7 +61,8 @@ typedef struct FebOperator {
   int32_t mat_mode;              /* FEB_MAT_* */
   const double* mat;             /* [dev] ISO: lam[ncell] followed by mu[ncell]; ORTHO: coeffs[ncell][6]; cell-id order */
   const uint8_t* active;         /* [dev] ncell flags */
-  const int64_t* cn;             /* [dev] ncell x 8 node ids (split connectivity), NULL = grid connectivity */
+  const int64_t* cn;             /* [dev] ncell x 8 node ids (split connectivity), NULL = grid connectivity; a corner that is
+                                    neither the grid node there nor a copy of it selects the per-cell level-0 kernels */
   int64_t nnode_total;           /* grid nodes + split copies */
   const int64_t* orig;           /* [dev] grid node of every node id (nnode_total), NULL when there are no copies */
   int64_t npen;                  /* diagonal penalties: kd[3 node + c] += k[3 i + c] */
