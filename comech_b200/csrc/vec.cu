@@ -158,13 +158,16 @@ k_dot_finalize(int kind, const Ta* __restrict__ a, const Tb* __restrict__ b, int
   if (last_block_sum(block_sum((s0 + s1) + (s2 + s3)), partials, ctr, t)) cg_step(kind, t, c, st);
 }
 
+// p = z + beta p, and z at a first iteration (beta 0), whose p may hold anything: a refused solve leaves NaN there
 template <typename T>
 __global__ void k_update_p(const T* __restrict__ z, T* __restrict__ p, const CgState* __restrict__ st, int64_t n,
                            const int* __restrict__ skip) {
   if (skip && *skip) return;
   const T beta = T(st->beta);
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    p[i] = z[i] + beta * p[i];
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const T zi = z[i], pi = p[i];
+    p[i] = beta == T(0) ? zi : zi + beta * pi;
+  }
 }
 
 // x += alpha p, r -= alpha q, ||r||^2 and the convergence step (FIN_CONV); rf (optional) receives r in FP32 for the next
