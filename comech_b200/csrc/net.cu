@@ -651,19 +651,25 @@ __global__ void __launch_bounds__(128) k_wgrad(const FebWgrad W, int64_t R, int 
 // columns hold all 27.  A CTA takes 32 x 32 channels and a range of rows (the launch fills the SMs), keeps the sums in
 // tensor memory and adds them with coalesced FP32 atomics at its end.
 //
-// The backward pass of 32 -> 32 on 96x64x48 (data, weight and bias gradients) takes 71 us; with mma.sync weight gradients and the
-// former data gradient it took 365 us.  Bound by the windows' rows, as the convolutions are.
+// The backward pass of 32 -> 32 on 96x64x48 (data, weight and bias gradients) takes 74 us, 31 of them here; with mma.sync weight
+// gradients and the former data gradient it took 365 us.  Bound by the windows' rows, as the convolutions are.
 //
-// Warps 0-2: one dz each of the final sums; warp 4: TMA; warp 5: MMAs.  For long z (a P window that leaves no room for two
-// slots) P is not shifted: nine Q windows a step, N = 32 (ndy = 1).
+// FP32 rounding grows with the rows that one accumulator takes in sequence, so the accumulators are read every `per_sum` steps
+// (wgrad3_plan) and the sums added in registers: nine warps, dz = warp mod 4 and dx (for ndy = 1: dx, dy) = warp div 4.  Against
+// one sum a CTA the 32 -> 32 gradient takes 31.1 instead of 29.1 us, 128 -> 128 on 24x16x12 15.5 instead of 14.2; the errors
+// against 64 bits are 1.1e-6 instead of 2.3e-6 and 1.2e-7 instead of 5.4e-7 (mma.sync, split in sums of the same lengths:
+// 2.0e-6 and 1.6e-7).
+//
+// Warp 3: TMA; warp 7: MMAs.  For long z (a P window that leaves no room for two slots) P is not shifted: nine Q windows a
+// step, N = 32 (ndy = 1).
 constexpr int kWgRows = 128;                     // rows (K) a step
 constexpr int kWgQ = kWgRows + 16;               // rows of a Q window: three more are read; slots stay 1 KB aligned
-constexpr int kWgTail = 8 * (4 + 4 + 1) + 16;
-constexpr int kWgThreads = 192;
+constexpr int kWgTail = 8 * (4 + 4 + 3) + 16;
+constexpr int kWgThreads = 384;
 
 struct Wgrad3Plan {
   int ndy, slots, boxes, box, stage;             // dy shifts of P a window, ring slots, P boxes a step and rows a box, slot bytes
-  int steps, per_cta;                            // row steps in all and a CTA
+  int steps, per_cta, per_sum;                   // row steps in all, a CTA, and a sum in the accumulators
 };
 
 inline Wgrad3Plan wgrad3_plan(const FebNetGrid& g, int64_t R, int tiles) {
@@ -681,6 +687,9 @@ inline Wgrad3Plan wgrad3_plan(const FebNetGrid& g, int64_t R, int tiles) {
   p.steps = div_up(R + (int64_t)(p.ndy - 1) * (g.nz + 2), kWgRows);
   const int splits = std::max(1, std::min(kSmCount / tiles, p.steps));
   p.per_cta = div_up(p.steps, splits);
+  // rows a sum, at most: fewer on small grids, whose gradients are sums of fewer
+  const int most = (R > 200000 ? 2048 : (R > 20000 ? 512 : 128)) / kWgRows;
+  p.per_sum = div_up(p.per_cta, div_up(p.per_cta, most));
   return p;
 }
 
@@ -689,13 +698,17 @@ k_wgrad3(const FebWgrad W, const __grid_constant__ CUtensorMap mapP, const __gri
   extern __shared__ __align__(1024) unsigned char smem[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + (size_t)L.slots * L.stage);
   uint64_t* empty = full + 4;
-  uint64_t* done = empty + 4;
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
+  uint64_t* done = empty + 4;                    // a sum is in the accumulators
+  uint64_t* freed = done + 1;                    // and has been read
+  uint64_t* drain = freed + 1;
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(drain + 1);
   volatile uint32_t* dead = tslot + 1;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     for (int s = 0; s < 4; ++s) { tc::mbar_init(full + s, 1); tc::mbar_init(empty + s, 1); }
     tc::mbar_init(done, 1);
+    tc::mbar_init(freed, 9);
+    tc::mbar_init(drain, 1);
     tc::mbar_fence_init();
     *dead = 0;
   }
@@ -709,7 +722,7 @@ k_wgrad3(const FebWgrad W, const __grid_constant__ CUtensorMap mapP, const __gri
   const uint32_t base = tc::smem_addr(smem);
   const uint32_t bytesP = (uint32_t)(L.boxes * L.box * kC3Row);
 
-  if (warp == 4) {                               // ---- producer
+  if (warp == 3) {                               // ---- producer
     if (lane == 0) {
       bool ok = true;
       RingPos at;
@@ -735,14 +748,19 @@ k_wgrad3(const FebWgrad W, const __grid_constant__ CUtensorMap mapP, const __gri
       }
     }
     __syncwarp();
-  } else if (warp == 5) {                        // ---- MMA issue
+  } else if (warp == 7) {                        // ---- MMA issue
     if (lane == 0) {
       const uint32_t idesc = tc::idesc_bf16(128, 32 * L.ndy) | tc::kIdescMnMajor;
       const uint32_t dcol = L.ndy == 3 ? 128 : 32;
       bool ok = true;
-      int acc = 0;
+      int acc = 0, in_sum = 0;
+      uint32_t sums = 0;
       RingPos at;
       for (int st = st0; st < st1; ++st, at.next(L.slots)) {
+        if (in_sum == 0 && sums > 0) {           // the sum before has been read
+          ok = tc::mbar_wait(tc::smem_addr(freed), (sums - 1) & 1) && !*dead;
+          if (!ok) break;
+        }
         ok = tc::mbar_wait(tc::smem_addr(full + at.slot), at.pass & 1);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -758,31 +776,59 @@ k_wgrad3(const FebWgrad W, const __grid_constant__ CUtensorMap mapP, const __gri
         }
         acc = 1;
         tc::commit(empty + at.slot);
+        if (++in_sum == L.per_sum || st + 1 == st1) {
+          tc::commit(done);
+          in_sum = acc = 0;
+          ++sums;
+        }
       }
-      if (ok) tc::commit(done);
-      else *dead = 1;
+      if (!ok) {                                 // the MMAs in flight end before the CTA frees its tensor memory
+        *dead = 1;
+        tc::commit(drain);
+        tc::mbar_wait(tc::smem_addr(drain), 0);
+      }
     }
     __syncwarp();
-  } else if (warp < 3) {                         // ---- sums of dz = warp - 1: lane b, columns a
-    bool ok = tc::mbar_wait(tc::smem_addr(done), 0) && !*dead;
-    ok = __all_sync(0xffffffffu, ok) != 0;
-    if (!ok) *dead = 1;
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll 1
-    for (int g = 0; g < 9; ++g) {                // (dx, dy)
-      float v[32];
-      // P's block i is shifted by i - 1 rows of z: it holds dy = 1 - i
-      const int col = L.ndy == 3 ? (g / 3) * 128 + (2 - g % 3) * 32 : g * 32;
-      if (ok) {
-        tc::tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)col, v);
+  } else if ((warp & 3) < 3) {                   // ---- sums of dz = (warp & 3) - 1, (dx, dy) = 3 (warp / 4) + 0 .. 2: lane b, columns a
+    const int dz = warp & 3, g0 = 3 * (warp >> 2);
+    const int nsum = (st1 - st0 + L.per_sum - 1) / L.per_sum;
+    float s[3][32];
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+      for (int a = 0; a < 32; ++a) s[j][a] = 0.f;
+    bool ok = true;
+    for (int q = 0; q < nsum && ok; ++q) {
+      ok = tc::mbar_wait(tc::smem_addr(done), (uint32_t)(q & 1)) && !*dead;
+      ok = __all_sync(0xffffffffu, ok) != 0;
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        float v[32];
+        // P's block i is shifted by i - 1 rows of z: it holds dy = 1 - i
+        const int col = L.ndy == 3 ? (g0 / 3) * 128 + (2 - j) * 32 : (g0 + j) * 32;
+        tc::tmem_ld32(tmem + ((uint32_t)(32 * dz) << 16) + (uint32_t)col, v);
         tc::wait_ld();
-      } else {                                   // a wait ran out: the gradient says so
 #pragma unroll
-        for (int a = 0; a < 32; ++a) v[a] = __int_as_float(0x7fffffff);
+        for (int a = 0; a < 32; ++a) s[j][a] += v[a];
       }
-      float* dw = W.dw + ((int64_t)(g * 3 + warp) * W.na + a0) * W.nb + b0 + lane;
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(freed);
+    }
+    if (!ok) {                                   // a wait ran out: the gradient says so
+      *dead = 1;
 #pragma unroll
-      for (int a = 0; a < 32; ++a) atomicAdd(dw + (int64_t)a * W.nb, v[a]);
+      for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int a = 0; a < 32; ++a) s[j][a] = __int_as_float(0x7fffffff);
+    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      float* dw = W.dw + ((int64_t)((g0 + j) * 3 + dz) * W.na + a0) * W.nb + b0 + lane;
+#pragma unroll
+      for (int a = 0; a < 32; ++a) atomicAdd(dw + (int64_t)a * W.nb, s[j][a]);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
