@@ -41,10 +41,15 @@ struct KuConfig {
 template <typename T, int MODE>
 void launch_fine_apply(const FineView<T>& F, const T* u, T* y, const int* skip, KuConfig cfg, cudaStream_t s);
 
+// Sparse part of the level-0 operator only (irregular cells, penalties, extra entries), added with atomics into acc (3 per
+// node).
+template <typename T, int MODE>
+void launch_fine_sparse_into(const FineView<T>& F, const T* u, T* acc, const int* skip, cudaStream_t s);
+
 // ------------------------------------------------------------------------------------------------ paired K.u
 // Operator of the paired-row kernel (fine_pair.cu): regular cells by 7-bit material ids, penalty springs as a diagonal,
-// the nodes that irregular cells or extra entries reach (and the split copies) as a list of rows, the smoother update
-// fused in the epilogue.
+// the nodes that irregular cells or extra entries reach (and the split copies) as a list of rows or, where these are many,
+// through accumulators; the smoother update fused in the epilogue.
 constexpr int kMaxMatIds = 128;   // ids 1..127; 0 = no regular cell
 
 // Nodes finished from their cells one by one: node[r], its up to 8 cells (cell[8 r + q]: code of the cell of which the node is
@@ -78,6 +83,7 @@ struct PairView {
   const T* idx; const T* idy; const T* idz;
   const T* kd;               // penalty diagonal, 3 per node (read at flagged nodes)
   PairRows<T> rows;
+  T* acc;                    // instead of kd and rows: sparse part of the product under way, 3 per node, zero between products
   const T* dinv6;            // symmetric block-Jacobi inverse [6][ntotal]: 00 11 22 01 02 12
 };
 
@@ -109,10 +115,11 @@ struct PairConfig {
   bool split = false;     // smoothing steps in two launches: product (its shape), update of all nodes
 };
 
-// y = K u (S null), the residual or the smoother step S; y takes K u of a step split in two launches (null: not split)
+// y = K u (S null), the residual or the smoother step S; y takes K u of a step split in two launches (null: not split).
+// Products that share F.acc have to follow one another.
 template <typename T, int MODE>
-int launch_fine_pair(const PairView<T>& F, const T* u, T* y, const SmoothArgs<T>* S, const int* skip, PairConfig cfg,
-                     cudaStream_t s);
+int launch_fine_pair(const PairView<T>& F, const FineView<T>& G, const T* u, T* y, const SmoothArgs<T>* S, const int* skip,
+                     PairConfig cfg, cudaStream_t s);
 // sets the shared-memory limits of every paired-kernel variant of this model on the current device (call
 // before any stream capture)
 int prepare_fine_pair(int mode, bool cube);

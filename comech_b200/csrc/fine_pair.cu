@@ -11,6 +11,9 @@
 //     160 x 112 x 96 foot).  As a kernel of its own ahead of the tiles, summing cells with atomics into a vector that the
 //     tiles added and cleared, this part took 5.3 / 6.2 / 9.2 us a product (24x18x16 / 96x64x48 / 160x112x96, FP32)
 //     however little there was to do; with assembled 3x3-block rows instead of cells it was bound by reading them.
+//   * where those nodes are many (rows_listed in solver.cu), that form is the faster one again: k_fine_sparse sums the cells,
+//     springs and entries into F.acc, the tiles add and clear it at the flagged nodes, and CTAs after the tiles do so for the
+//     split copies.
 //
 // Tiling: a warp holds 32 node columns (30 owned, one halo column on each side) of two neighbouring node
 // rows; a CTA of WY warps holds 2 WY rows (2 WY - 2 owned) and marches in z over `zchunk` node planes.
@@ -33,7 +36,7 @@ namespace feb {
 namespace {
 
 constexpr int kXOwn = 30;
-constexpr uint32_t kPenalty = 0x80u, kListed = 0x100u;   // node flags of a cell-pair word
+constexpr uint32_t kPenalty = 0x80u, kListed = 0x100u;   // node flags of a cell-pair word (kListed: reached by the sparse part)
 // cell codes of the row list: an irregular cell's index, a regular cell's material id as kRegularCell - id, or none
 constexpr int kNoCell = -1, kRegularCell = -1;
 #ifndef FEB_PAIR_UNROLL
@@ -214,6 +217,22 @@ __device__ __forceinline__ void node_update(const SmoothArgs<T>& S, T a1, T a2, 
   if constexpr (EPI == kStep) node_step(S, a1, a2, n, r, o);
 }
 
+// what a flagged node that is finished here adds: its sparse part from the accumulator (ACC; cleared for the next product), or
+// its penalties
+template <typename T, bool ACC>
+__device__ __forceinline__ void add_sparse(const PairView<T>& F, const T* __restrict__ u, int n, T (&t)[3]) {
+  if constexpr (ACC) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      t[c] += F.acc[3 * n + c];
+      F.acc[3 * n + c] = T(0);
+    }
+  } else {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) t[c] += F.kd[3 * n + c] * u[3 * n + c];
+  }
+}
+
 // the Chebyshev coefficients of the step
 template <typename T>
 __device__ __forceinline__ void pair_coef(const SmoothArgs<T>& S, T& a1, T& a2) {
@@ -316,10 +335,11 @@ constexpr size_t pair_smem_bytes() {
   return 4 * sizeof(V2<T>) * 3 * WY * 32 + sizeof(T) * kMaxMatIds * (CUBE ? 2 : MatWidth<MODE>::value);
 }
 
-template <typename T, int MODE, bool CUBE, int WY, int EPI>
+// ACC: the sparse part goes through accumulators (no row list; `tiles` CTAs, then those of the split copies)
+template <typename T, int MODE, bool CUBE, int WY, int EPI, bool ACC>
 __global__ void __launch_bounds__(32 * WY, 1)
 k_fine_pair(PairView<T> F, const T* __restrict__ u, T* __restrict__ y, SmoothArgs<T> S, const int* __restrict__ skip,
-            int zchunk, int nbx, int nby) {
+            int zchunk, int nbx, int nby, int tiles) {
   if (skip && *skip) return;
   constexpr int W = MatWidth<MODE>::value;
   constexpr bool HAS12 = (MODE != MAT_ISO_SRI);
@@ -338,6 +358,23 @@ k_fine_pair(PairView<T> F, const T* __restrict__ u, T* __restrict__ y, SmoothArg
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   T a1 = T(0), a2 = T(0);
   if constexpr (EPI == kStep) pair_coef(S, a1, a2);
+  if constexpr (ACC) {
+    if ((int)blockIdx.x >= tiles) {              // a split copy a thread
+      const int64_t n = F.nnode + ((int)blockIdx.x - tiles) * (int64_t)blockDim.x + threadIdx.x;
+      if (n >= F.ntotal) return;
+      T t[3] = {T(0), T(0), T(0)};
+      add_sparse<T, ACC>(F, u, (int)n, t);
+      if constexpr (EPI == kProduct) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) y[3 * n + c] = t[c];
+      } else {
+        NodeOps<T> o;
+        load_node_ops<T, EPI>(F, S, u, a1 != T(0) || S.x_lag, (int)n, o);
+        node_update<T, EPI>(S, a1, a2, (int)n, t, o);
+      }
+      return;
+    }
+  }
   for (int q = threadIdx.x; q < kMaxMatIds; q += blockDim.x) {
     if constexpr (CUBE) {
       sMat[q][0] = q < F.nmat ? T(F.mtab[W * q] * F.h / 16.0) : T(0);
@@ -431,15 +468,10 @@ k_fine_pair(PairView<T> F, const T* __restrict__ u, T* __restrict__ y, SmoothArg
     if (kk < K0 || kk >= K1) return;
     const int n0 = n0base + plane * kk, n1 = n1base + plane * kk;
     T t0[3] = {out[0].lo(), out[1].lo(), out[2].lo()}, t1[3] = {out[0].hi(), out[1].hi(), out[2].hi()};
-    const bool f0 = own0 && !(flags & kListed), f1 = own1 && !(flags & kListed << 16);   // the node is finished here
-    if (own0 && (flags & kPenalty)) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) t0[c] += F.kd[3 * n0 + c] * u[3 * n0 + c];
-    }
-    if (own1 && (flags & kPenalty << 16)) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) t1[c] += F.kd[3 * n1 + c] * u[3 * n1 + c];
-    }
+    constexpr uint32_t kAway = ACC ? 0u : kListed, kAdds = ACC ? kPenalty | kListed : kPenalty;
+    const bool f0 = own0 && !(flags & kAway), f1 = own1 && !(flags & kAway << 16);   // the node is finished here
+    if (own0 && (flags & kAdds)) add_sparse<T, ACC>(F, u, n0, t0);
+    if (own1 && (flags & kAdds << 16)) add_sparse<T, ACC>(F, u, n1, t1);
     if constexpr (PREF) {
       if (f0) node_update<T, EPI>(S, a1, a2, n0, t0, o0);
       if (f1) node_update<T, EPI>(S, a1, a2, n1, t1, o1);
@@ -476,20 +508,24 @@ k_fine_pair(PairView<T> F, const T* __restrict__ u, T* __restrict__ y, SmoothArg
   };
   {   // prologue: face of plane K0-1; the CTA's share of the row list while its planes are on their way
     V v0[3], E[3][2];
-    const int nrow = F.rows.n, group = threadIdx.x >> 3;
-    int row0 = blockIdx.x * kRowGroups;
-    RowFetch rf;
-    if (row0 < nrow) rf = fetch_row(F.rows, row0 + group);
+    [[maybe_unused]] const int nrow = ACC ? 0 : F.rows.n, group = threadIdx.x >> 3;
+    [[maybe_unused]] int row0 = blockIdx.x * kRowGroups;
+    [[maybe_unused]] RowFetch rf;
+    if constexpr (!ACC) {
+      if (row0 < nrow) rf = fetch_row(F.rows, row0 + group);
+    }
     load_plane(K0 - 1, v0);
     load_plane(K0, va);
     load_plane(K0 + 1, vb);
     ca = load_cells(K0 - 1);
-    while (row0 < nrow) {                        // the next rows are fetched while these are finished
-      const RowFetch f = rf;
-      const int row = row0 + group;
-      row0 += gridDim.x * kRowGroups;
-      if (row0 < nrow) rf = fetch_row(F.rows, row0 + group);
-      finish_row<T, MODE, CUBE, EPI>(F, u, y, S, a1, a2, f, row < nrow);
+    if constexpr (!ACC) {
+      while (row0 < nrow) {                      // the next rows are fetched while these are finished
+        const RowFetch f = rf;
+        const int row = row0 + group;
+        row0 += gridDim.x * kRowGroups;
+        if (row0 < nrow) rf = fetch_row(F.rows, row0 + group);
+        finish_row<T, MODE, CUBE, EPI>(F, u, y, S, a1, a2, f, row < nrow);
+      }
     }
     edge(v0, E);
     put_edge(slot(K0 - 1), E);
@@ -602,24 +638,32 @@ k_fine_pair(PairView<T> F, const T* __restrict__ u, T* __restrict__ y, SmoothArg
   }
 }
 
-template <typename T, int MODE, bool CUBE, int WY, int EPI>
-int launch_pair_kernel(const PairView<T>& F, const T* u, T* y, const SmoothArgs<T>& A, const int* skip, int zc,
-                       cudaStream_t s) {
+template <typename T, int MODE, bool CUBE, int WY, int EPI, bool ACC>
+int launch_pair_variant(const PairView<T>& F, const T* u, T* y, const SmoothArgs<T>& A, const int* skip, int zc,
+                        cudaStream_t s) {
   constexpr int OY = 2 * WY - 2;
   const int nbx = div_up(F.nxn, kXOwn), nby = div_up(F.nyn, OY), nbz = div_up(F.nzn, zc);
-  const int64_t blocks = (int64_t)nbx * nby * nbz;
+  const int64_t tiles = (int64_t)nbx * nby * nbz, copies = ACC ? div_up(F.ntotal - F.nnode, 32 * WY) : 0;
   constexpr size_t smem = pair_smem_bytes<T, MODE, CUBE, WY>();
-  auto kern = k_fine_pair<T, MODE, CUBE, WY, EPI>;
+  auto kern = k_fine_pair<T, MODE, CUBE, WY, EPI, ACC>;
   FEB_TRY(set_dyn_smem((const void*)kern, (int)smem));
-  kern<<<(unsigned)blocks, 32 * WY, smem, s>>>(F, u, y, A, skip, zc, nbx, nby);
+  kern<<<(unsigned)(tiles + copies), 32 * WY, smem, s>>>(F, u, y, A, skip, zc, nbx, nby, (int)tiles);
   note_launch();
   return FEB_OK;
 }
 
 template <typename T, int MODE, bool CUBE, int WY, int EPI>
+int launch_pair_kernel(const PairView<T>& F, const T* u, T* y, const SmoothArgs<T>& A, const int* skip, int zc,
+                       cudaStream_t s) {
+  return F.acc ? launch_pair_variant<T, MODE, CUBE, WY, EPI, true>(F, u, y, A, skip, zc, s)
+               : launch_pair_variant<T, MODE, CUBE, WY, EPI, false>(F, u, y, A, skip, zc, s);
+}
+
+template <typename T, int MODE, bool CUBE, int WY, int EPI>
 int prepare_pair_kernel() {
   constexpr size_t smem = pair_smem_bytes<T, MODE, CUBE, WY>();
-  return set_dyn_smem((const void*)k_fine_pair<T, MODE, CUBE, WY, EPI>, (int)smem);
+  FEB_TRY(set_dyn_smem((const void*)k_fine_pair<T, MODE, CUBE, WY, EPI, false>, (int)smem));
+  return set_dyn_smem((const void*)k_fine_pair<T, MODE, CUBE, WY, EPI, true>, (int)smem);
 }
 
 template <typename T, int MODE>
@@ -644,8 +688,9 @@ int prepare_pair_precision(bool cube) {
 }
 
 template <typename T, int MODE, int EPI>
-int launch_pair_wy(const PairView<T>& F, const T* u, T* y, const SmoothArgs<T>& A, const int* skip, const PairConfig& cfg,
-                   cudaStream_t s) {
+int launch_pair_wy(const PairView<T>& F, const FineView<T>& G, const T* u, T* y, const SmoothArgs<T>& A, const int* skip,
+                   const PairConfig& cfg, cudaStream_t s) {
+  if (F.acc) launch_fine_sparse_into<T, MODE>(G, u, F.acc, skip, s);
   const int zc = std::max(1, EPI == kStep ? cfg.zchunk_smooth : cfg.zchunk);
   if constexpr (MODE == MAT_ISO_SRI) {
     if (F.cube) {
@@ -874,12 +919,12 @@ __global__ void k_cheb_first6(const T* __restrict__ b, const T* __restrict__ D, 
 }  // namespace
 
 template <typename T, int MODE>
-int launch_fine_pair(const PairView<T>& F, const T* u, T* y, const SmoothArgs<T>* S, const int* skip, PairConfig cfg,
-                     cudaStream_t s) {
-  if (!S) return launch_pair_wy<T, MODE, kProduct>(F, u, y, SmoothArgs<T>{}, skip, cfg, s);
-  if (!S->updates()) return launch_pair_wy<T, MODE, kResidual>(F, u, y, *S, skip, cfg, s);
-  if (!cfg.split || !y) return launch_pair_wy<T, MODE, kStep>(F, u, y, *S, skip, cfg, s);
-  FEB_TRY((launch_pair_wy<T, MODE, kProduct>(F, u, y, SmoothArgs<T>{}, skip, cfg, s)));
+int launch_fine_pair(const PairView<T>& F, const FineView<T>& G, const T* u, T* y, const SmoothArgs<T>* S, const int* skip,
+                     PairConfig cfg, cudaStream_t s) {
+  if (!S) return launch_pair_wy<T, MODE, kProduct>(F, G, u, y, SmoothArgs<T>{}, skip, cfg, s);
+  if (!S->updates()) return launch_pair_wy<T, MODE, kResidual>(F, G, u, y, *S, skip, cfg, s);
+  if (!cfg.split || !y) return launch_pair_wy<T, MODE, kStep>(F, G, u, y, *S, skip, cfg, s);
+  FEB_TRY((launch_pair_wy<T, MODE, kProduct>(F, G, u, y, SmoothArgs<T>{}, skip, cfg, s)));
   k_pair_update<T><<<div_up(F.ntotal, 256), 256, 0, s>>>(F, u, y, *S, skip); note_launch();
   return FEB_OK;
 }
@@ -887,7 +932,7 @@ int launch_fine_pair(const PairView<T>& F, const T* u, T* y, const SmoothArgs<T>
 template <typename T, int MODE, bool CUBE, int WY, int EPI>
 int pair_occupancy() {
   int nb = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_fine_pair<T, MODE, CUBE, WY, EPI>, 32 * WY,
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_fine_pair<T, MODE, CUBE, WY, EPI, false>, 32 * WY,
                                                     pair_smem_bytes<T, MODE, CUBE, WY>()) != cudaSuccess)
     return 1;
   return std::max(nb, 1);
@@ -976,8 +1021,8 @@ void launch_cheb_first6(const T* b, const T* D6, const LevelParams* lp, T* d, T*
 }
 
 #define INST(T, M)                                                                                          \
-  template int launch_fine_pair<T, M>(const PairView<T>&, const T*, T*, const SmoothArgs<T>*, const int*, PairConfig, \
-                                      cudaStream_t);
+  template int launch_fine_pair<T, M>(const PairView<T>&, const FineView<T>&, const T*, T*, const SmoothArgs<T>*, const int*, \
+                                      PairConfig, cudaStream_t);
 INST(float, MAT_ISO_SRI) INST(float, MAT_ISO_FULL) INST(float, MAT_ORTHO)
 INST(double, MAT_ISO_SRI) INST(double, MAT_ISO_FULL) INST(double, MAT_ORTHO)
 #undef INST

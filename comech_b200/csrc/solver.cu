@@ -673,6 +673,7 @@ struct Csr {
   int *row_dof = nullptr, *row_ptr = nullptr, *col = nullptr;
   double* v64 = nullptr;
   float* v32 = nullptr;
+  int nent = 0, longest = 0;              // entries in all and of the longest row
 };
 
 int upload_csr(Pool& pool, const Entries& E, Csr& C) {
@@ -688,6 +689,8 @@ int upload_csr(Pool& pool, const Entries& E, Csr& C) {
   }
   rp.push_back((int)E.size());
   C.nrow = (int)rd.size();
+  C.nent = (int)E.size();
+  for (int i = 0; i < C.nrow; ++i) C.longest = std::max(C.longest, rp[i + 1] - rp[i]);
   if (C.nrow == 0) return FEB_OK;
   FEB_TRY(pool.upload(&C.row_dof, rd.data(), rd.size()));
   FEB_TRY(pool.upload(&C.row_ptr, rp.data(), rp.size()));
@@ -1038,6 +1041,13 @@ struct FebHandle {
     return coarse_fail ? coarse_error() : FEB_OK;
   }
 
+  // level-0 products through accumulators share these with the level-0 power iteration: a product on s waits (on the
+  // device) for that chain while it may still run
+  int wait_fine() {
+    if (pending && coarsest > 0 && P64.acc) FEB_CUDA(cudaStreamWaitEvent(s, aux_ev[0], 0));
+    return FEB_OK;
+  }
+
   // the rigid-mode coefficients' stream (set with the rigid groups) and its fork / join events
   cudaStream_t rs = nullptr;
   cudaEvent_t rs_fork = nullptr, rs_join = nullptr;
@@ -1082,9 +1092,9 @@ struct FebHandle {
   template <typename T>
   void pair_run(const T* u, T* y, const SmoothArgs<T>* S, const int* skip) {
     switch (mode) {
-      case MAT_ISO_SRI: launch_fine_pair<T, MAT_ISO_SRI>(pview<T>(), u, y, S, skip, pcfg<T>(), s); break;
-      case MAT_ISO_FULL: launch_fine_pair<T, MAT_ISO_FULL>(pview<T>(), u, y, S, skip, pcfg<T>(), s); break;
-      default: launch_fine_pair<T, MAT_ORTHO>(pview<T>(), u, y, S, skip, pcfg<T>(), s); break;
+      case MAT_ISO_SRI: launch_fine_pair<T, MAT_ISO_SRI>(pview<T>(), fine<T>(), u, y, S, skip, pcfg<T>(), s); break;
+      case MAT_ISO_FULL: launch_fine_pair<T, MAT_ISO_FULL>(pview<T>(), fine<T>(), u, y, S, skip, pcfg<T>(), s); break;
+      default: launch_fine_pair<T, MAT_ORTHO>(pview<T>(), fine<T>(), u, y, S, skip, pcfg<T>(), s); break;
     }
   }
 
@@ -1870,30 +1880,37 @@ int autotune_ku(FebHandle* h) {
 // bit c of l.  Read off the device element operator for the unit cube, checked to be those integers, laid
 // out as the kernel's B table: [face cz][node row b][output n][4a + c] in BF16 (exact).  Leaves tc_ok false
 // for other grids or models.
-// Row list of the paired-row operator (ids: material id of every regular cell) and its penalty diagonal.
-int setup_rows(FebHandle* h, const uint8_t* ids) {
+// The sparse part as a row list or through accumulators: a list is finished by the tiles' CTAs while their first planes are on
+// their way, 32 rows a CTA and pass and 8 entries of a node at a time, and saves a launch; with many rows, or much work a row,
+// those CTAs hold the tiles up, and k_fine_sparse has the whole chip for it.  List against accumulators, one FP64 V-cycle:
+//   24x18x16, 7 % of the nodes in the list 102 : 135 us, 25 % 119 : 135, 34 % 136 : 144, 52 % 153 : 149, 97 % 173 : 135;
+//   48x34x28, 3 % 176 : 211, 50 % 658 : 606, 97 % 440 : 311; FP32 V-cycles cross over at about 50 % too;
+//   24x18x16, 16 % with 16 entries a node of the grid 174 : 164; 48x34x28, all of an assembled matrix (160 a node) 1464 : 420;
+//   48x34x28, the rows of 475 entries of a rank-1 term on 475 nodes 460 : 423.
+bool rows_listed(int64_t rows, int64_t entries, int longest, int64_t nodes) {
+  return 5 * rows <= 2 * nodes && entries <= 8 * nodes && longest <= 64;
+}
+
+// Sparse part of the paired-row operator (ids: material id of every regular cell; entries, longest: its extra entries in all
+// and of a row): row list and penalty diagonal, or accumulators.
+int setup_rows(FebHandle* h, const uint8_t* ids, int64_t entries, int longest) {
   FebHandle& H = *h;
   const FineView<double>& F = H.F64;
   const int64_t ncell = (int64_t)H.nx * H.ny * H.nz;
   const size_t n3 = 3 * (size_t)H.ntotal;
   uint8_t* flag = nullptr;
-  double* kd64 = nullptr;
-  float* kd32 = nullptr;
   int *cmap = nullptr, *start = nullptr;
   FEB_TRY(H.pool.zeros(&flag, H.ntotal));
-  FEB_TRY(H.pool.zeros(&kd64, n3));
-  FEB_TRY(H.pool.alloc(&kd32, n3));
   FEB_TRY(H.pool.alloc(&cmap, ncell));
   FEB_TRY(H.pool.alloc(&start, H.ntotal));
   FEB_CUDA(cudaMemsetAsync(cmap, 0xff, ncell * sizeof(int), H.s));
   FEB_CUDA(cudaMemsetAsync(start, 0xff, H.ntotal * sizeof(int), H.s));
   launch_row_flags(F, flag, cmap, start, H.s);
-  launch_pen_diag(F.pen_node, F.pen_k, F.npen, kd64, H.s);
-  launch_convert<double, float>(kd64, kd32, (int64_t)n3, nullptr, H.s);
   FEB_CUDA(cudaGetLastError());
-  H.P64.kd = kd64; H.P32.kd = kd32;
   H.P64.rows = PairRows<double>{};
   H.P32.rows = PairRows<float>{};
+  H.P64.acc = nullptr;
+  H.P32.acc = nullptr;
   // room for every node that may be flagged
   const int64_t cap = std::min<int64_t>(H.ntotal, 8 * (int64_t)F.nirr + F.nrow + (H.ntotal - H.nnode));
   if (cap > 0) {
@@ -1910,15 +1927,31 @@ int setup_rows(FebHandle* h, const uint8_t* ids) {
     int n = 0;
     FEB_CUDA(cudaMemcpyAsync(&n, cnt, sizeof(int), cudaMemcpyDeviceToHost, H.s));
     FEB_CUDA(cudaStreamSynchronize(H.s));
-    FEB_TRY(H.pool.alloc(&cell, 8 * (size_t)n));
-    FEB_TRY(H.pool.alloc(&corner, 16 * (size_t)n));
-    FEB_TRY(H.pool.alloc(&ex, n));
-    launch_rows(F, node, n, H.orig_copy, cmap, start, ids, cell, corner, ex, H.s);
-    FEB_CUDA(cudaGetLastError());
-    H.P64.rows = PairRows<double>{n, node, cell, corner, F.irr_cell, F.irr_mat, ex, F.col, F.val};
-    H.P32.rows = PairRows<float>{n, node, cell, corner, F.irr_cell, H.F32.irr_mat, ex, H.F32.col, H.F32.val};
+    if (rows_listed(n, entries, longest, H.ntotal)) {
+      FEB_TRY(H.pool.alloc(&cell, 8 * (size_t)n));
+      FEB_TRY(H.pool.alloc(&corner, 16 * (size_t)n));
+      FEB_TRY(H.pool.alloc(&ex, n));
+      launch_rows(F, node, n, H.orig_copy, cmap, start, ids, cell, corner, ex, H.s);
+      FEB_CUDA(cudaGetLastError());
+      H.P64.rows = PairRows<double>{n, node, cell, corner, F.irr_cell, F.irr_mat, ex, F.col, F.val};
+      H.P32.rows = PairRows<float>{n, node, cell, corner, F.irr_cell, H.F32.irr_mat, ex, H.F32.col, H.F32.val};
+    } else {
+      FEB_TRY(H.pool.zeros(&H.P64.acc, n3));
+      FEB_TRY(H.pool.zeros(&H.P32.acc, n3));
+      H.pool.free(node);
+    }
     H.pool.free(tmp);
     H.pool.free(cnt);
+  }
+  if (!H.P64.acc) {
+    double* kd64 = nullptr;
+    float* kd32 = nullptr;
+    FEB_TRY(H.pool.zeros(&kd64, n3));
+    FEB_TRY(H.pool.alloc(&kd32, n3));
+    launch_pen_diag(F.pen_node, F.pen_k, F.npen, kd64, H.s);
+    launch_convert<double, float>(kd64, kd32, (int64_t)n3, nullptr, H.s);
+    FEB_CUDA(cudaGetLastError());
+    H.P64.kd = kd64; H.P32.kd = kd32;
   }
   H.pool.free(cmap);
   H.pool.free(start);
@@ -1928,11 +1961,11 @@ int setup_rows(FebHandle* h, const uint8_t* ids) {
 
 // Paired-row level-0 operator (fine_pair.cu): material ids of the regular cells (FEB_KU_PAIR=0 keeps the
 // per-cell kernels), flags of the grid nodes that receive sparse contributions, the cell-pair words, the
-// row list and the symmetric level-0 block-Jacobi inverse.  Leaves pair_ok false when more than
+// row list or accumulators and the symmetric level-0 block-Jacobi inverse.  Leaves pair_ok false when more than
 // kMaxMatIds - 1 distinct materials occur (or on a hash collision), and for connectivity whose corners are not the grid
 // node there or a copy of it.
 template <int W>
-int setup_pair(FebHandle* h, const double* mat_s64) {
+int setup_pair(FebHandle* h, const double* mat_s64, const Csr& extra) {
   FebHandle& H = *h;
   const char* env = std::getenv("FEB_KU_PAIR");
   if (env && env[0] == '0') return FEB_OK;
@@ -1966,7 +1999,7 @@ int setup_pair(FebHandle* h, const double* mat_s64) {
     H.pool.free(vals);
     return FEB_OK;
   }
-  FEB_TRY(setup_rows(h, ids));
+  FEB_TRY(setup_rows(h, ids, extra.nent, extra.longest));
   H.pool.free(ids);
   FEB_TRY(H.pool.alloc(&H.D6_32, 6 * (size_t)H.ntotal));
   FEB_TRY(H.pool.alloc(&H.D6_64, 6 * (size_t)H.ntotal));
@@ -2381,7 +2414,7 @@ int setup_level0(FebHandle* h, const FebOperator* op) {
   launch_block_inverse(D, H.ntotal, V.Dinv64, V.Dinv32, s);
   FEB_CUDA(cudaGetLastError());
   H.pool.free(D);
-  FEB_TRY(setup_pair<W>(h, mat_s64));
+  FEB_TRY(setup_pair<W>(h, mat_s64, c0));
   H.stage_mark();   // 3: used nodes, level-0 diagonal blocks, paired-row operator
   g_prof.mark("L0 local upload, diag blocks, pair operator", s);
   // the autotuner's timings must not share the GPU with the early level-1 stencil: wait for it first (the
@@ -2978,6 +3011,7 @@ int feb_set_rigid_groups(FebHandle* h, int32_t ngroups, const int64_t* offsets, 
   FEB_TRY(H.pool.alloc(&col, 3 * (size_t)H.ntotal));
   FEB_TRY(H.pool.alloc(&kcol, 3 * (size_t)H.ntotal));
   FEB_TRY(H.pool.alloc(&Ecd, (size_t)nc * nc));
+  FEB_TRY(H.wait_fine());
   if (!H.rs) {
     H.rs = g_streams.stream();
     if (!H.rs_fork) H.rs_fork = g_streams.event();
@@ -3221,6 +3255,7 @@ int feb_solve_batch(FebHandle* const* hs, int32_t n, const double* const* f, con
 int feb_apply(FebHandle* h, int32_t prec, const void* u, void* y) {
   if (!h || !u || !y) { set_last_error("feb_apply: null argument"); return FEB_ERR_ARG; }
   FEB_TRY(h->sync_in());
+  FEB_TRY(h->wait_fine());
   if (prec == 0) h->apply<double>(0, (const double*)u, (double*)y, nullptr);
   else h->apply<float>(0, (const float*)u, (float*)y, nullptr);
   FEB_CUDA(cudaGetLastError());
