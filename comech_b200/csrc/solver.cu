@@ -1242,8 +1242,7 @@ struct FebHandle {
       } else {
         ++late;
       }
-      // x: where a split step leaves K u (the last one replaces it by the result); a call in place keeps its b there
-      pair_run<T>(u, x == b ? nullptr : x, &A, skip);
+      pair_run<T>(u, x, &A, skip);               // x: where a split step leaves K u (the last one replaces it by the result)
     };
     launch_cheb_first6<T>(b, dinv6<T>(), lp, d, deg == 1 ? xs : nullptr, ntotal, skip, s);
     for (int k = 1; k < deg; ++k) {
@@ -1299,7 +1298,7 @@ struct FebHandle {
     smooth<T>(l, b, x, false, skip);
   }
 
-  // z = M r for the CG of precision T (FP64 CG with an FP64 or FP32 V-cycle, FP32 CG with FP32); rf_ready:
+  // z = M r, in other memory than r, for the CG of precision T (FP64 CG with an FP64 or FP32 V-cycle, FP32 CG with FP32); rf_ready:
   // the FP32 copy of r (rf) was written by the CG update already
   template <typename T>
   void precondition(const T* r_, T* z_, const int* skip, bool rf_ready = false) {
@@ -3277,6 +3276,13 @@ int feb_precondition(FebHandle* h, const double* r, double* z) {
   if (h->coarsest < 0) { set_last_error("feb_precondition: handle built with max_levels = 0 (operator only)"); return FEB_ERR_ARG; }
   FEB_TRY(h->settle());
   FEB_TRY(h->sync_in());
+  // A V-cycle writes z before it has read all of r, and the rigid modes' coefficients are formed from r on another stream
+  // meanwhile: where z overlaps r, the call works on a copy in q, which is free outside solves.
+  const size_t n = 3 * (size_t)h->ntotal;
+  if (r < z + n && z < r + n) {
+    FEB_CUDA(cudaMemcpyAsync(h->q, r, n * sizeof(double), cudaMemcpyDeviceToDevice, h->s));
+    r = h->q;
+  }
   h->precondition<double>(r, z, nullptr);
   FEB_CUDA(cudaGetLastError());
   return h->sync_out();

@@ -171,7 +171,7 @@ FEB_API int feb_solve_batch(FebHandle* const* hs, int32_t n, const double* const
 FEB_API int feb_apply(FebHandle* h, int32_t prec, const void* u, void* y);
 
 /* z = M r: one application of the solve's preconditioner (V-cycle in the handle's precision plus the rigid-mode
- * correction), FP64 full-layout r and z on the device.  Replaces the M LinearOperator of fe/gmg.py:125-135 for a
+ * correction), FP64 full-layout r and z on the device; z may be r.  Replaces the M LinearOperator of fe/gmg.py:125-135 for a
  * Krylov loop run by the caller (pcg_gmg with a separate A_op, fe/gmg.py:136). */
 FEB_API int feb_precondition(FebHandle* h, const double* r, double* z);
 
