@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(kConvThreads) k_conv(const FebConv P, int64_t 
 // 143 -> 12.3 us.
 constexpr int kC3Rows = 126;                     // outputs of 128 accumulator rows
 constexpr int kC3Row = kKS * 2;                  // bytes of a 32-channel operand row
-constexpr int kC3Tail = 8 * (4 + 4 + 2 + 2 + 1) + 24 + 2 * (2 * 2 * 4 + 4) * 32 * 4;   // barriers, TMEM slot, edge rows, bias
+constexpr int kC3Tail = 8 * (4 + 4 + 2 + 2 + 1) + 24 + 2 * (2 * 2 * 4 + 4) * 32 * 4;   // barriers, TMEM slot, drain, edge rows, bias
 
 struct Conv3Plan {
   int ndy, slots, boxes, box, stage;             // dy offsets a step, ring slots, A boxes a step and rows a box, slot bytes
@@ -355,6 +355,7 @@ k_conv3(const FebConv P, const __grid_constant__ CUtensorMap mapA, const __grid_
   uint64_t* wfull = tempty + 2;
   uint32_t* tslot = reinterpret_cast<uint32_t*>(wfull + 1);
   volatile uint32_t* dead = tslot + 1;
+  uint64_t* drain = wfull + 2;
   float (*edge)[2][2][4][32] = reinterpret_cast<float (*)[2][2][4][32]>(wfull + 4);   // [half][parity][direction][warp]
   float (*sbias)[4][32] = reinterpret_cast<float (*)[4][32]>(edge + 2);               // [half][warp][channel]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -363,6 +364,7 @@ k_conv3(const FebConv P, const __grid_constant__ CUtensorMap mapA, const __grid_
     for (int s = 0; s < 4; ++s) { tc::mbar_init(full + s, 1); tc::mbar_init(empty + s, 1); }
     for (int s = 0; s < 2; ++s) { tc::mbar_init(tfull + s, 1); tc::mbar_init(tempty + s, 4 * H); }
     tc::mbar_init(wfull, 1);
+    tc::mbar_init(drain, 1);
     tc::mbar_fence_init();
     *dead = 0;
   }
@@ -451,7 +453,11 @@ k_conv3(const FebConv P, const __grid_constant__ CUtensorMap mapA, const __grid_
         }
         if (ok) tc::commit(tfull + buf.slot);
       }
-      if (!ok) *dead = 1;
+      if (!ok) {                                 // the MMAs in flight end before the CTA frees its tensor memory
+        *dead = 1;
+        tc::commit(drain);
+        tc::mbar_wait(tc::smem_addr(drain), 0);
+      }
     }
     __syncwarp();
   } else {                                       // ---- epilogue of half h
