@@ -344,8 +344,9 @@ def ku_roofline(P, d, lib, engine, _lib, pk, pk_kind):
             del us, ys
     finally:
         pr.close()
-    # the solve's dominant kernel (its largest share of device time): the level-0 smoother step, the paired K.u
-    # with the fused Chebyshev update, as the V-cycle runs it (mixed precision handle with its hierarchy)
+    # the largest share of the solve's device time: the level-0 smoother step, the paired K.u with the Chebyshev update, in the
+    # form that the handle's plan has (mixed precision handle with its hierarchy); one that brings the iterate up to date, which
+    # two of a V-cycle's five do
     ps = engine.Problem(g, _lib.MAT_ISO_SRI, d["mat"], d["active"], cn=d["cn"], orig=d["orig"], pen_node=d["pen_node"],
                         pen_k=d["pen_k"], extra_coo=d["extra"], precision="mixed", tol=TOL)
     try:
@@ -357,21 +358,23 @@ def ku_roofline(P, d, lib, engine, _lib, pk, pk_kind):
         ptr = [(C.c_void_p * nbuf)(*[st[q].data_ptr() for st in sets]) for q in range(4)]
         ms = C.c_float()
         for nrep in (2 * nbuf, 20 * nbuf):
+            before = lib.feb_launch_count()
             _lib.check(lib.feb_benchmark_smooth_set(ps.h, nbuf, ptr[0], ptr[1], ptr[2], ptr[3], nrep, C.byref(ms)))
+            per_step = (lib.feb_launch_count() - before) // (nrep + 1)
         # d read; r and x read and written; d' written; the 6-value symmetric block-Jacobi inverse; the K.u's
-        # cell-pair words and sparse part as above
+        # cell-pair words and sparse part as above (a split step moves K d besides)
         sv = 4
         alg_s = 24 * ntotal * sv + 4 * npair + n_irr * (32 + 2 * sv) + n_pen * (4 + 3 * sv) + n_extra * (8 + sv)
-        sm = dict(ms=ms.value, bytes=alg_s, gbs=alg_s / (ms.value * 1e-3) / 1e9, nbuf=nbuf)
+        sm = dict(ms=ms.value, bytes=alg_s, gbs=alg_s / (ms.value * 1e-3) / 1e9, nbuf=nbuf,
+                  form="k_fine_pair with the Chebyshev update" if per_step == 1 else "k_fine_pair, then k_pair_update")
         del sets
     finally:
         ps.close()
     r32 = roof["fp32"]
     return {"bound": "hbm", "achieved": round(sm["gbs"], 1), "peak": pk, "unit": "GB/s",
             "frac": round(sm["gbs"] / pk, 4), "traffic": ku_traffic(SMOOTH_PROFILE),
-            "kernel": "level-0 smoother step FP32 (k_fine_pair with the Chebyshev update, fused or as k_pair_update), the "
-                      "solve's largest share of device time; operands rotated over "
-                      f"{sm['nbuf']} buffer sets (> L2)",
+            "kernel": f"level-0 smoother step FP32 that updates the iterate ({sm['form']}); such steps are the solve's largest "
+                      f"share of device time; operands rotated over {sm['nbuf']} buffer sets (> L2)",
             "peak_kind": pk_kind, "ms_per_launch": round(sm["ms"], 4), "algorithmic_bytes": sm["bytes"],
             "active_cells": nact,
             "ku_apply_fp32": {"achieved": round(r32["gbs"], 1), "frac": round(r32["gbs"] / pk, 4),

@@ -3322,6 +3322,8 @@ int feb_benchmark_smooth_set(FebHandle* h, int32_t nbuf, void* const* d, void* c
   FEB_TRY(h->settle());     // the Chebyshev coefficients come from the power iteration
   FEB_TRY(h->sync_in());
   FEB_TRY(h->tune_events());
+  float* ku = nullptr;      // K d of a step that the handle's plan splits in two launches
+  FEB_TRY(h->pool.alloc(&ku, 3 * (size_t)h->ntotal));
   auto step = [&](int i) {
     const int b = i % nbuf;
     SmoothArgs<float> A;
@@ -3329,13 +3331,14 @@ int feb_benchmark_smooth_set(FebHandle* h, int32_t nbuf, void* const* d, void* c
     A.x_in = (const float*)x[b]; A.x_out = (float*)x[b];
     A.d_out = (float*)e[b];
     A.lp = h->lp; A.k = 0;
-    h->pair_run<float>((const float*)d[b], nullptr, &A, nullptr);
+    h->pair_run<float>((const float*)d[b], ku, &A, nullptr);
   };
   step(0);
   FEB_CUDA(cudaEventRecord(h->tev0, h->s));
   for (int i = 0; i < nrep; ++i) step(i);
   FEB_CUDA(cudaEventRecord(h->tev1, h->s));
   FEB_CUDA(cudaEventSynchronize(h->tev1));
+  h->pool.free(ku);
   float t = 0.f;
   FEB_CUDA(cudaEventElapsedTime(&t, h->tev0, h->tev1));
   *ms = t / nrep;
