@@ -120,9 +120,9 @@ struct PairConfig {
 template <typename T, int MODE>
 int launch_fine_pair(const PairView<T>& F, const FineView<T>& G, const T* u, T* y, const SmoothArgs<T>* S, const int* skip,
                      PairConfig cfg, cudaStream_t s);
-// sets the shared-memory limits of every paired-kernel variant of this model on the current device (call
-// before any stream capture)
-int prepare_fine_pair(int mode, bool cube);
+// sets the shared-memory limits of every paired-kernel variant of this model, with a row list or with accumulators (acc), on the
+// current device (call before any stream capture)
+int prepare_fine_pair(int mode, bool cube, bool acc);
 // resident CTAs per SM of the paired kernel (smoothing variant) and its x-y tiles per node plane
 template <typename T>
 int fine_pair_blocks_per_sm(int mode, bool cube, int wy, bool smooth);

@@ -660,30 +660,30 @@ int launch_pair_kernel(const PairView<T>& F, const T* u, T* y, const SmoothArgs<
 }
 
 template <typename T, int MODE, bool CUBE, int WY, int EPI>
-int prepare_pair_kernel() {
+int prepare_pair_kernel(bool acc) {
   constexpr size_t smem = pair_smem_bytes<T, MODE, CUBE, WY>();
-  FEB_TRY(set_dyn_smem((const void*)k_fine_pair<T, MODE, CUBE, WY, EPI, false>, (int)smem));
-  return set_dyn_smem((const void*)k_fine_pair<T, MODE, CUBE, WY, EPI, true>, (int)smem);
+  return set_dyn_smem(acc ? (const void*)k_fine_pair<T, MODE, CUBE, WY, EPI, true>
+                          : (const void*)k_fine_pair<T, MODE, CUBE, WY, EPI, false>, (int)smem);
 }
 
 template <typename T, int MODE>
-int prepare_pair_precision(bool cube) {
+int prepare_pair_precision(bool cube, bool acc) {
   if constexpr (MODE == MAT_ISO_SRI && std::is_same<T, float>::value) {
     if (cube) {
-      FEB_TRY((prepare_pair_kernel<T, MODE, true, 16, kProduct>()));
-      FEB_TRY((prepare_pair_kernel<T, MODE, true, 16, kResidual>()));
+      FEB_TRY((prepare_pair_kernel<T, MODE, true, 16, kProduct>(acc)));
+      FEB_TRY((prepare_pair_kernel<T, MODE, true, 16, kResidual>(acc)));
     }
   }
   if constexpr (MODE == MAT_ISO_SRI) {
     if (cube) {
-      FEB_TRY((prepare_pair_kernel<T, MODE, true, 8, kProduct>()));
-      FEB_TRY((prepare_pair_kernel<T, MODE, true, 8, kResidual>()));
-      FEB_TRY((prepare_pair_kernel<T, MODE, true, 8, kStep>()));
+      FEB_TRY((prepare_pair_kernel<T, MODE, true, 8, kProduct>(acc)));
+      FEB_TRY((prepare_pair_kernel<T, MODE, true, 8, kResidual>(acc)));
+      FEB_TRY((prepare_pair_kernel<T, MODE, true, 8, kStep>(acc)));
     }
   }
-  FEB_TRY((prepare_pair_kernel<T, MODE, false, 8, kProduct>()));
-  FEB_TRY((prepare_pair_kernel<T, MODE, false, 8, kResidual>()));
-  FEB_TRY((prepare_pair_kernel<T, MODE, false, 8, kStep>()));
+  FEB_TRY((prepare_pair_kernel<T, MODE, false, 8, kProduct>(acc)));
+  FEB_TRY((prepare_pair_kernel<T, MODE, false, 8, kResidual>(acc)));
+  FEB_TRY((prepare_pair_kernel<T, MODE, false, 8, kStep>(acc)));
   return FEB_OK;
 }
 
@@ -961,17 +961,17 @@ template int fine_pair_blocks_per_sm<double>(int, bool, int, bool);
 
 int fine_pair_tiles_xy(int nxn, int nyn, int wy) { return div_up(nxn, kXOwn) * div_up(nyn, 2 * wy - 2); }
 
-int prepare_fine_pair(int mode, bool cube) {
+int prepare_fine_pair(int mode, bool cube, bool acc) {
   switch (mode) {
     case MAT_ISO_SRI:
-      FEB_TRY((prepare_pair_precision<float, MAT_ISO_SRI>(cube)));
-      return prepare_pair_precision<double, MAT_ISO_SRI>(cube);
+      FEB_TRY((prepare_pair_precision<float, MAT_ISO_SRI>(cube, acc)));
+      return prepare_pair_precision<double, MAT_ISO_SRI>(cube, acc);
     case MAT_ISO_FULL:
-      FEB_TRY((prepare_pair_precision<float, MAT_ISO_FULL>(cube)));
-      return prepare_pair_precision<double, MAT_ISO_FULL>(cube);
+      FEB_TRY((prepare_pair_precision<float, MAT_ISO_FULL>(cube, acc)));
+      return prepare_pair_precision<double, MAT_ISO_FULL>(cube, acc);
     default:
-      FEB_TRY((prepare_pair_precision<float, MAT_ORTHO>(cube)));
-      return prepare_pair_precision<double, MAT_ORTHO>(cube);
+      FEB_TRY((prepare_pair_precision<float, MAT_ORTHO>(cube, acc)));
+      return prepare_pair_precision<double, MAT_ORTHO>(cube, acc);
   }
 }
 

@@ -2032,7 +2032,7 @@ int setup_pair(FebHandle* h, const double* mat_s64, const Csr& extra) {
   };
   fill(H.P32, H.F32, H.D6_32);
   fill(H.P64, H.F64, H.D6_64);
-  FEB_TRY(prepare_fine_pair(H.mode, cube));
+  FEB_TRY(prepare_fine_pair(H.mode, cube, H.P64.acc != nullptr));
   H.pc32 = PairConfig{cube ? 16 : 8, 16};
   H.pc64 = PairConfig{8, 16};
   H.pair_ok = true;
