@@ -297,11 +297,11 @@ __global__ void __launch_bounds__(kConvThreads) k_conv(const FebConv P, int64_t 
 // When the window of three dy offsets would leave room for fewer than two slots (grids of some 500 cells along z), a step
 // takes one (x, y) offset instead (ndy = 1), with a window of the tile's rows alone.
 //
-// Loads bound the layers (an SM takes a row of an operand window about every three clocks, 64 or 128 bytes alike), so rows are
-// 64 channels long where the channel count allows it (SL), and the weights of a CTA's 32 output channels stay in shared
-// memory when they leave room for two A slots (a CTA then keeps to its channel tile).  64 -> 32 channels on 96x64x48, from
-// the caller's side: 171 us with gathered rows and a tap group a step, 41.5 us now (0.79 PFLOP/s); 256 -> 256 on 12x8x6:
-// 143 -> 12.3 us.
+// A slot's MMAs start when its whole window is there.  An SM takes a row of a window about every three clocks, 64 or 128 bytes
+// alike, so rows are 64 channels long where the channel count allows it (SL), and the weights of a CTA's 32 output channels
+// stay in shared memory when they leave room for two A slots (a CTA then keeps to its channel tile).  Neither side fills the
+// time: 64 -> 32 channels on 96x64x48 has the tensor pipe active for 47 % of its cycles and 5 TB/s from L2.  It takes 41.5 us
+// from the caller's side (0.79 PFLOP/s; 171 us with gathered rows and a tap group a step), 256 -> 256 on 12x8x6 12.3 us (143).
 constexpr int kC3Rows = 126;                     // outputs of 128 accumulator rows
 constexpr int kC3Row = kKS * 2;                  // bytes of a 32-channel operand row
 constexpr int kC3Tail = 8 * (4 + 4 + 2 + 2 + 1) + 24 + 2 * (2 * 2 * 4 + 4) * 32 * 4;   // barriers, TMEM slot, drain, edge rows, bias
@@ -658,7 +658,8 @@ __global__ void __launch_bounds__(128) k_wgrad(const FebWgrad W, int64_t R, int 
 // tensor memory and adds them with coalesced FP32 atomics at its end.
 //
 // The backward pass of 32 -> 32 on 96x64x48 (data, weight and bias gradients) takes 74 us, 31 of them here; with mma.sync weight
-// gradients and the former data gradient it took 365 us.  Bound by the windows' rows, as the convolutions are.
+// gradients and the former data gradient it took 365 us.  As with the convolutions, windows that arrive whole before their MMAs
+// start leave the tensor pipe active for 40 % of its cycles.
 //
 // FP32 rounding grows with the rows that one accumulator takes in sequence, so the accumulators are read every `per_sum` steps
 // (wgrad3_plan) and the sums added in registers: nine warps, dz = warp mod 4 and dx (for ndy = 1: dx, dy) = warp div 4.  Against

@@ -1884,11 +1884,6 @@ int autotune_ku(FebHandle* h) {
   return FEB_OK;
 }
 
-// Tensor-core operand of the FP32 level-0 K.u: on equal cubic cells of edge h the ISO element matrices are
-// h K(1) with 72 K_mu(1), 72 K_lambda(1) integer and the one-point 16 K_lambda(1) = s s^T, s[3l+c] = +-1 by
-// bit c of l.  Read off the device element operator for the unit cube, checked to be those integers, laid
-// out as the kernel's B table: [face cz][node row b][output n][4a + c] in BF16 (exact).  Leaves tc_ok false
-// for other grids or models.
 // The sparse part as a row list or through accumulators: a list is finished by the tiles' CTAs while their first planes are on
 // their way, 32 rows a CTA and pass and 8 entries of a node at a time, and saves a launch; with many rows, or much work a row,
 // those CTAs hold the tiles up, and k_fine_sparse has the whole chip for it.  List against accumulators, one FP64 V-cycle:
@@ -2039,6 +2034,11 @@ int setup_pair(FebHandle* h, const double* mat_s64, const Csr& extra) {
   return FEB_OK;
 }
 
+// Tensor-core operand of the FP32 level-0 K.u: on equal cubic cells of edge h the ISO element matrices are
+// h K(1) with 72 K_mu(1), 72 K_lambda(1) integer and the one-point 16 K_lambda(1) = s s^T, s[3l+c] = +-1 by
+// bit c of l.  Read off the device element operator for the unit cube, checked to be those integers, laid
+// out as the kernel's B table: [face cz][node row b][output n][4a + c] in BF16 (exact).  Leaves tc_ok false
+// for other grids or models.
 int setup_tc(FebHandle* h) {
   FebHandle& H = *h;
   if ((H.mode != MAT_ISO_SRI && H.mode != MAT_ISO_FULL) || env_tc() == 0) return FEB_OK;
