@@ -1298,8 +1298,8 @@ struct FebHandle {
     smooth<T>(l, b, x, false, skip);
   }
 
-  // z = M r, in other memory than r, for the CG of precision T (FP64 CG with an FP64 or FP32 V-cycle, FP32 CG with FP32); rf_ready:
-  // the FP32 copy of r (rf) was written by the CG update already
+  // z = M r, in other memory than r, for the CG of precision T (FP64 CG with an FP64 or FP32 V-cycle, FP32 CG with FP32);
+  // rf_ready: the FP32 copy of r (rf) was written by the CG update already
   template <typename T>
   void precondition(const T* r_, T* z_, const int* skip, bool rf_ready = false) {
     const int64_t n = 3 * ntotal;
@@ -1809,8 +1809,8 @@ int tune_pair(FebHandle* h, PairConfig* best, T* u, T* y, T* y2, T* y3) {
 }
 
 // Operators of one grid that share a plan: those without a sparse part, with a row list of up to an eighth of the nodes and with
-// a longer one, and with accumulators.  The tiles' CTAs finish the list, so the shape that suits one need not suit the other: a foot of
-// 48x34x28 cells on the plan of an operator that is all extra entries took 265 instead of 240 us a V-cycle.
+// a longer one, and with accumulators.  The tiles' CTAs finish the list, so the shape that suits one need not suit the other: a
+// foot of 48x34x28 cells on the plan of an operator that is all extra entries took 265 instead of 240 us a V-cycle.
 int sparse_class(const FebHandle& H) {
   if (!H.pair_ok) return 0;
   if (H.P64.acc) return 4;
